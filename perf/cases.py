@@ -29,31 +29,31 @@ VOCAB = 32768
 def listed():
     return [
         # A chat with one user, a small budget: two layers' update and attention and the eviction check.  Latency and launches.
-        dict(name="token, 1 request", kind="tokens", batch=1, heads=16, kv_heads=8, memory=512, buffer=128, new=1, layers=2,
+        dict(name="token 1 request", kind="tokens", batch=1, heads=16, kv_heads=8, memory=512, buffer=128, new=1, layers=2,
              dtype="bf16", budget="head"),
         # Serving 64 requests whose heads share each request's budget: lengths differ from head to head.
-        dict(name="token, 64 requests, shared", kind="tokens", batch=64, heads=32, kv_heads=8, memory=2048, buffer=128, new=1,
+        dict(name="token 64 requests shared", kind="tokens", batch=64, heads=32, kv_heads=8, memory=2048, buffer=128, new=1,
              layers=1, dtype="f16", budget="request"),
         # A long prompt fed in pieces of 512 tokens against a full cache; every piece evicts.
-        dict(name="piece of 512, 8 requests", kind="tokens", batch=8, heads=16, kv_heads=8, memory=4096, buffer=512, new=512,
+        dict(name="piece of 512 8 requests", kind="tokens", batch=8, heads=16, kv_heads=8, memory=4096, buffer=512, new=512,
              layers=1, dtype="bf16", budget="head"),
         # The end of a prompt pass: 8192 tokens of every head reduced to the budget.
-        dict(name="hand-off, 4 requests", kind="handoff", batch=4, kv_heads=8, tokens=8192, memory=4096, buffer=128, layers=2,
+        dict(name="hand-off 4 requests", kind="handoff", batch=4, kv_heads=8, tokens=8192, memory=4096, buffer=128, layers=2,
              dtype="bf16"),
         # Prompts through the mixers.  Many long ones, the largest case ...
-        dict(name="retention, 4 x 8192", kind="retention", width=2048, heads=16, lengths="8192,8192,8192,8192"),
+        dict(name="retention 4 x 8192", kind="retention", width=2048, heads=16, lengths="8192,8192,8192,8192"),
         # ... two of unequal length ...
-        dict(name="mamba2, 4096 + 2731", kind="mamba2", width=2048, heads=64, lengths="4096,2731"),
+        dict(name="mamba2 4096 + 2731", kind="mamba2", width=2048, heads=64, lengths="4096,2731"),
         # ... one that is twice the window ...
-        dict(name="differential, 8192", kind="differential", width=2048, heads=16, kv_heads=8, window=4096, lengths="8192"),
+        dict(name="differential 8192", kind="differential", width=2048, heads=16, kv_heads=8, window=4096, lengths="8192"),
         # ... one short prompt ...
-        dict(name="hgrn2, 1 x 1500", kind="hgrn2", width=2048, heads=16, lengths="1500"),
+        dict(name="hgrn2 1 x 1500", kind="hgrn2", width=2048, heads=16, lengths="1500"),
         # ... and a wide layer.
-        dict(name="latent, 2 x 4096 wide", kind="latent", width=4096, heads=32, window=4096, lengths="4096,4096"),
+        dict(name="latent 2 x 4096 wide", kind="latent", width=4096, heads=32, window=4096, lengths="4096,4096"),
         # Decoding with whole models (four layers of each).
-        dict(name="qwen3, 32 requests", kind="qwen3", width=2048, heads=16, kv_heads=8, ff=6144, memory=4096, buffer=128, batch=32),
-        dict(name="dafovik, 32 requests", kind="dafovik", width=2048, heads=16, kv_heads=8, ff=6144, window=4096, batch=32),
-        dict(name="lonulix, 8 requests", kind="lonulix", width=2048, heads=16, ff=6144, window=4096, batch=8),
+        dict(name="qwen3 32 requests", kind="qwen3", width=2048, heads=16, kv_heads=8, ff=6144, memory=4096, buffer=128, batch=32),
+        dict(name="dafovik 32 requests", kind="dafovik", width=2048, heads=16, kv_heads=8, ff=6144, window=4096, batch=32),
+        dict(name="lonulix 8 requests", kind="lonulix", width=2048, heads=16, ff=6144, window=4096, batch=8),
     ]
 
 
