@@ -439,6 +439,11 @@ int tkv_skinny_gemm_swiglu(const void* gate_up, const void* w, float* partial, i
  * vectors (norms, biases, convolution taps) are fp32 arrays.  No counterpart in the reference.
  */
 
+/* dst[i] = host_values[i], and dst[host_index[i]] = value, for i in [0, n).  The host arrays are read before the call returns and
+ * travel as launch arguments: no copy is queued and nothing is waited for. */
+int tkv_put_ints(int32_t* dst, const int32_t* host_values, int n, tkv_stream_t stream);
+int tkv_set_ints(int32_t* dst, const int32_t* host_index, int n, int value, tkv_stream_t stream);
+
 /* pos0[b] = lens[slots[b]]; lens[slots[b]] += tokens of request b in this step. */
 int tkv_batch_begin(int32_t* lens, const int32_t* slots, const int32_t* cu_tokens, int32_t* pos0, int batch,
                     tkv_stream_t stream);

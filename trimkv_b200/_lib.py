@@ -51,6 +51,8 @@ SIGNATURES = {
     "tkv_skinny_gemm_splits": (I, [I, I, I]),
     "tkv_skinny_gemm": (I, [P, P, P, I, I, I, I, P, P]),
     "tkv_skinny_gemm_swiglu": (I, [P, P, P, I, I, I, I, P, P]),
+    "tkv_put_ints": (I, [P, P, I, P]),
+    "tkv_set_ints": (I, [P, P, I, I, P]),
     "tkv_batch_begin": (I, [P, P, P, P, I, P]),
     "tkv_embed_stream": (I, [P, P, L, P, P, I, I, F, I, P, P]),
     "tkv_postnorm_add": (I, [P, P, P, P, I, I, F, F, F, I, P]),

@@ -214,7 +214,7 @@ class HybridForCausalLM(HybridPreTrainedModel, TrimKVForCausalLM):
         if want is not None:
             if len(want) == 0:
                 return stream.new_empty(0, self.config.vocab)
-            at = torch.tensor(list(want), dtype=torch.int32).to(ids.device, non_blocking=True)
+            at = ops.ints_on(ids.device, list(want))
         return self.head(self.model.final_norm(stream, at))
 
     def decode_step(self, ids: torch.Tensor, cache: HybridStateCache) -> torch.Tensor:

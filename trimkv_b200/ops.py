@@ -5,6 +5,7 @@ CUDA kernels of libtrimkv_b200.so.
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional
 
 import torch
@@ -424,6 +425,36 @@ update_flatten_view_triton = update_flatten_view  # the reference's name for the
 # --------------------------------------------------------------------------------------------------------------------
 # Decoders with recurrent layers, windowed attention and experts.  ``batch`` is a ``state_cache.StepBatch``: packed
 # tokens, ``cu`` (None in a one-token step), ``slots`` and ``pos0`` of the step's requests.
+
+def ints_on(device, values) -> torch.Tensor:
+    """A few host integers as an int32 tensor on ``device``: launch arguments of a small kernel instead of a copy, so that the
+    host neither stages nor waits."""
+    n = len(values)
+    if device.type != "cuda":
+        return torch.tensor(values, dtype=torch.int32)
+    if torch.cuda.is_current_stream_capturing():
+        raise RuntimeError("host integers would be baked into the CUDA graph being captured")
+    out = torch.empty(n, dtype=torch.int32, device=device)
+    with torch.cuda.device_of(out):
+        check(lib().tkv_put_ints(out.data_ptr(), (ctypes.c_int32 * n)(*values), n, _stream(out)), "tkv_put_ints")
+    _count(-(-n // 960))
+    return out
+
+
+def set_ints(dst: torch.Tensor, index, value: int) -> None:
+    """``dst[index] = value`` (int32) for a list of host integers, without a copy."""
+    n = len(index)
+    if not dst.is_cuda:
+        dst[list(index)] = value
+        return
+    if n and not 0 <= min(index) <= max(index) < dst.numel():
+        raise IndexError(f"index outside {dst.numel()} entries")
+    if torch.cuda.is_current_stream_capturing():
+        raise RuntimeError("host integers would be baked into the CUDA graph being captured")
+    with torch.cuda.device_of(dst):
+        check(lib().tkv_set_ints(dst.data_ptr(), (ctypes.c_int32 * n)(*index), n, value, _stream(dst)), "tkv_set_ints")
+    _count(-(-n // 960))
+
 
 def batch_begin(lens, slots, cu, pos0) -> None:
     check(lib().tkv_batch_begin(lens.data_ptr(), slots.data_ptr(), _ptr(cu), pos0.data_ptr(), slots.shape[0], _stream(lens)),

@@ -89,7 +89,7 @@ class StepBatch:
             if max(hist, default=0) == 0:
                 plan = (self.cu, at, 0)
             else:
-                plan = (torch.tensor(starts, dtype=torch.int32).to(self.slots.device, non_blocking=True), at, max(hist))
+                plan = (ops.ints_on(self.slots.device, starts), at, max(hist))
             self._plans[window] = plan
         return plan
 
@@ -135,7 +135,7 @@ class HybridStateCache:
         first = len(self._rows)
         self._rows += taken
         if taken:
-            self._lens[torch.tensor(taken, dtype=torch.int64, device=self.device)] = 0
+            ops.set_ints(self._lens, taken, 0)
         self._decode_key = None
         return list(range(first, first + count))
 
@@ -217,7 +217,7 @@ class HybridStateCache:
             if self._decode_key != tuple(slots):
                 if torch.cuda.is_current_stream_capturing():
                     raise RuntimeError("the batch changed while a one-token step was being recorded")
-                self._slots_dev = torch.tensor(slots, dtype=torch.int32).to(self.device)
+                self._slots_dev = ops.ints_on(self.device, slots)
                 self._pos0_dev = torch.empty_like(self._slots_dev)
                 self._decode_key = tuple(slots)
                 self._generation += 1
@@ -226,7 +226,7 @@ class HybridStateCache:
             bounds = [0]
             for n in counts:
                 bounds.append(bounds[-1] + n)
-            packed = torch.tensor(slots + bounds, dtype=torch.int32).to(self.device, non_blocking=True)
+            packed = ops.ints_on(self.device, slots + bounds)
             dev_slots, cu = packed[:len(slots)], packed[len(slots):]
             pos0 = torch.empty(len(slots), dtype=torch.int32, device=self.device)
         ops.batch_begin(self._lens, dev_slots, cu, pos0)
