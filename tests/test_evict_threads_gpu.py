@@ -1,0 +1,32 @@
+"""Eviction by CTAs of 1024, 512 and 256 threads: on both sides of the numbers of segments where the width changes."""
+import pytest
+import torch
+
+from trimkv_b200 import ops
+
+DEV = "cuda"
+
+
+# lengths with a remainder of a round of either width; 600 rows kept: several tiles of rows, the last one short
+@pytest.mark.gpu
+@pytest.mark.parametrize("nseg", [1, 148, 149, 296, 297])
+@pytest.mark.parametrize("n,m", [(1541, 600), (1025, 1024), (300, 7)])
+def test_widths_agree(nseg, n, m):
+    g = torch.Generator(device=DEV).manual_seed(nseg + n)
+    cap, d = n + 3, 64
+    k, v = (torch.randn(nseg * cap, d, generator=g, device=DEV).bfloat16() for _ in range(2))
+    beta = -torch.rand(nseg * cap, generator=g, device=DEV).mul(8).round().div(8)             # many equal scores ..
+    beta.view(nseg, cap)[:, ::3] -= torch.rand(nseg, -(-cap // 3), generator=g, device=DEV)   # .. among others
+    pos = torch.arange(cap, dtype=torch.int32, device=DEV).repeat(nseg)
+    score = beta.view(nseg, cap)[:, :n] * (n + 1 - pos[:n]).float()
+    keep = score.sort(dim=1, descending=True, stable=True).indices[:, :m].sort(dim=1).values
+    kept, count = torch.empty(nseg, m, dtype=torch.int32, device=DEV), torch.empty(nseg, dtype=torch.int32, device=DEV)
+    ops.evict_select(beta.view(nseg, cap), pos[:cap], None, n, nseg, n + 1, m, m, n, kept, count)
+    assert torch.equal(kept.long(), keep) and bool((count == m).all())
+    want = [t.view(nseg, cap, -1).gather(1, keep[:, :, None].expand(-1, -1, t.numel() // (nseg * cap))) for t in (k, v, beta, pos)]
+    ln = torch.full((nseg,), n, dtype=torch.int32, device=DEV)
+    status = ops.new_status(DEV)
+    ops.evict(k, v, beta, pos, ln, None, nseg, nseg, cap, n + 1, m, m, n, status=status)
+    assert ops.read_status(status) == 0 and bool((ln == m).all())
+    for t, w in zip((k, v, beta, pos), want):
+        assert torch.equal(t.view(nseg, cap, -1)[:, :m], w)

@@ -11,6 +11,7 @@
 //      a barrier, then stored at their destination.  dst <= src for every row and tiles are handled
 //      in ascending order, so a tile's stores can only land on rows whose content was already consumed.
 // Algorithmic bytes per segment: 8n (scan) + 2*M*row_pair_bytes (move K,V) + 8M (metadata).
+#include <type_traits>
 #include "tkv_common.cuh"
 
 namespace tkv {
@@ -23,7 +24,7 @@ constexpr int kMaxSelectLen = 57000;         // keys must fit in 227 KB of share
 constexpr int kEvictThreadsWide = 512;       // for long segments, whose key array allows fewer CTAs per SM
 constexpr int kMoveThreads = 256;            // evict_move_kernel: its staging area limits CTAs per SM, so each is wide
 constexpr int kMoveGridCtas = 148 * 4;       // evict_move_kernel: blocks in its grid (they loop over the evicting segments)
-constexpr int kEvictThreadsPlan = 1024;      // selection only (plan mode): few segments, so each gets a full CTA
+constexpr int kEvictThreadsPlan = 1024;      // selection only (plan mode), and few segments: each gets a full CTA
 struct SelectScratch {
   int hist[256];
   int warp_sums[kEvictThreadsPlan / 32 + 1];
@@ -491,7 +492,8 @@ struct SelectParams {
   int32_t* kept_idx; int32_t* kept_cnt; int32_t* status;
 };
 
-__global__ void __launch_bounds__(kEvictThreads) evict_select_kernel(SelectParams p) {
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads) evict_select_kernel(SelectParams p) {
   extern __shared__ __align__(16) uint32_t keys[];
   __shared__ SelectScratch sc;
   const int seg = blockIdx.x;
@@ -506,14 +508,14 @@ __global__ void __launch_bounds__(kEvictThreads) evict_select_kernel(SelectParam
   }
   const float* beta = p.beta + (int64_t)seg * p.beta_stride;
   const int32_t* pos = p.pos + (int64_t)seg * p.pos_stride;
-  for (int i = threadIdx.x; i < n; i += kEvictThreads)
+  for (int i = threadIdx.x; i < n; i += kThreads)
     keys[i] = score_key(retention_score(beta[i], pos[i], p.q_idx));
   __syncthreads();
   uint32_t thresh; int n_eq_keep;
-  radix_select_mth<kEvictThreads>(keys, n, p.m, &sc, &thresh, &n_eq_keep);
-  build_kept_list<kEvictThreads>(keys, n, thresh, n_eq_keep, &sc);
+  radix_select_mth<kThreads>(keys, n, p.m, &sc, &thresh, &n_eq_keep);
+  build_kept_list<kThreads>(keys, n, thresh, n_eq_keep, &sc);
   const int32_t* kept = reinterpret_cast<const int32_t*>(keys);
-  for (int j = threadIdx.x; j < p.m; j += kEvictThreads) p.kept_idx[(int64_t)seg * p.m + j] = kept[j];
+  for (int j = threadIdx.x; j < p.m; j += kThreads) p.kept_idx[(int64_t)seg * p.m + j] = kept[j];
   if (threadIdx.x == 0) p.kept_cnt[seg] = p.m;
 }
 
@@ -609,6 +611,17 @@ static int set_smem(K kernel, size_t bytes, const char* what) {
   return TKV_OK;
 }
 
+// Threads of a segment's CTA.  A segment is one CTA's, and its time is the latency of rounds over its keys (four selection passes
+// and the list) and of tiles of rows (load, barrier, store): the fewer threads, the more rounds and tiles.  So few segments get wide
+// CTAs, down to where the SMs' 1024 threads are shared by several of them; long segments, whose key array leaves room for at most
+// 3 CTAs per SM, get at least 512.  A piece of 512 tokens of 8 requests x 8 heads against 4096 rows (attention, append and this):
+// 315 us with 256 threads per segment, 279 us with 1024.
+template <typename F> static int with_evict_threads(int nseg, size_t smem, F launch) {
+  if (nseg <= 148) return launch(std::integral_constant<int, kEvictThreadsPlan>());
+  if (nseg <= 2 * 148 || smem > 56 * 1024) return launch(std::integral_constant<int, kEvictThreadsWide>());
+  return launch(std::integral_constant<int, kEvictThreads>());
+}
+
 }  // namespace tkv
 
 extern "C" int tkv_rebuild_cu_seqlens(const int32_t* seg_len, int32_t* cu_seqlens, int nseg, int group,
@@ -679,18 +692,18 @@ static int evict_impl(void* k_cache, void* v_cache, float* beta_cache, int32_t* 
     if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_evict_multi: memset: %s", cudaGetErrorString(e));
   }
   const size_t smem = (size_t)max_len * 4;
-  // Long segments: the key array leaves room for at most 3 CTAs per SM, so each CTA gets twice the threads (and
-  // twice the rows in flight per tile) to keep the memory system as busy as 4 narrow CTAs do.
-  const bool wide = smem > 56 * 1024;
-  int rc = wide ? set_smem(evict_inplace_kernel<kEvictThreadsWide>, smem, "tkv_evict")
-                : set_smem(evict_inplace_kernel<kEvictThreads>, smem, "tkv_evict");
-  if (rc != TKV_OK) return rc;
+  int rc;
   if (ctas > 1) {
     rc = set_smem(evict_inplace_kernel<kEvictThreadsPlan>, smem, "tkv_evict_multi");
-    if (rc != TKV_OK) return rc;
-    evict_inplace_kernel<kEvictThreadsPlan><<<nseg, kEvictThreadsPlan, smem, (cudaStream_t)stream>>>(p);
-  } else if (wide) evict_inplace_kernel<kEvictThreadsWide><<<nseg, kEvictThreadsWide, smem, (cudaStream_t)stream>>>(p);
-  else evict_inplace_kernel<kEvictThreads><<<nseg, kEvictThreads, smem, (cudaStream_t)stream>>>(p);
+    if (rc == TKV_OK) evict_inplace_kernel<kEvictThreadsPlan><<<nseg, kEvictThreadsPlan, smem, (cudaStream_t)stream>>>(p);
+  } else {
+    rc = with_evict_threads(nseg, smem, [&](auto threads) {
+      int r = set_smem(evict_inplace_kernel<threads.value>, smem, "tkv_evict");
+      if (r == TKV_OK) evict_inplace_kernel<threads.value><<<nseg, threads.value, smem, (cudaStream_t)stream>>>(p);
+      return r;
+    });
+  }
+  if (rc != TKV_OK) return rc;
   rc = check_launch("tkv_evict");
   if (rc != TKV_OK) return rc;
   if (ctas > 1) {
@@ -761,9 +774,12 @@ extern "C" int tkv_evict_select(const float* beta, int64_t beta_stride, const in
   p.m = memory_size; p.trigger_len = trigger_len; p.max_len = max_len;
   p.kept_idx = kept_idx; p.kept_cnt = kept_cnt; p.status = status;
   const size_t smem = (size_t)max_len * 4;
-  int rc = set_smem(evict_select_kernel, smem, "tkv_evict_select");
+  const int rc = with_evict_threads(nseg, smem, [&](auto threads) {
+    int r = set_smem(evict_select_kernel<threads.value>, smem, "tkv_evict_select");
+    if (r == TKV_OK) evict_select_kernel<threads.value><<<nseg, threads.value, smem, (cudaStream_t)stream>>>(p);
+    return r;
+  });
   if (rc != TKV_OK) return rc;
-  evict_select_kernel<<<nseg, kEvictThreads, smem, (cudaStream_t)stream>>>(p);
   return check_launch("tkv_evict_select");
 }
 
