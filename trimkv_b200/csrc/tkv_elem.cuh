@@ -57,6 +57,33 @@ template <int V> __device__ __forceinline__ void store_vec(__nv_bfloat16* p, con
   }
 }
 
+// V elements as they are in memory (V = 8: one or two 16-byte words), for loads that are requested well before they are used.
+template <typename T, int V> struct RawVec {
+  static_assert(V == 8, "vectors");
+  static constexpr int kWords = (int)sizeof(T) / 2;
+  uint4 w[kWords];
+  __device__ __forceinline__ void load(const T* p) {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) w[i] = ld16_stream(reinterpret_cast<const char*>(p) + 16 * i);
+  }
+  __device__ __forceinline__ void floats(float* v) const {
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
+      const uint32_t x[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if constexpr (sizeof(T) == 2) { v[2 * e] = __uint_as_float(x[e] << 16); v[2 * e + 1] = __uint_as_float(x[e] & 0xffff0000u); }
+        else v[4 * i + e] = __uint_as_float(x[e]);
+      }
+    }
+  }
+};
+template <typename T> struct RawVec<T, 1> {
+  T x;
+  __device__ __forceinline__ void load(const T* p) { x = *p; }
+  __device__ __forceinline__ void floats(float* v) const { v[0] = to_f32<T>(x); }
+};
+
 __device__ __forceinline__ float warp_add(float x) {
 #pragma unroll
   for (int o = 16; o >= 1; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
