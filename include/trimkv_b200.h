@@ -95,6 +95,11 @@ int tkv_evict_select(const float* beta, int64_t beta_stride, const int32_t* pos,
                      const int32_t* seg_len, int n_uniform, int nseg, int64_t q_idx,
                      int memory_size, int trigger_len, int max_len,
                      int32_t* kept_idx, int32_t* kept_cnt, int32_t* status, tkv_stream_t stream);
+/* The same from log betas of any of the three types (the score is taken of their fp32 value) and 32- or 64-bit positions. */
+int tkv_evict_select_as(const void* beta, int beta_dtype, int64_t beta_stride, const void* pos, int pos_bits, int64_t pos_stride,
+                        const int32_t* seg_len, int n_uniform, int nseg, int64_t q_idx,
+                        int memory_size, int trigger_len, int max_len,
+                        int32_t* kept_idx, int32_t* kept_cnt, int32_t* status, tkv_stream_t stream);
 
 /*
  * Gather kept rows from a source into a (different) capacity-strided cache:
@@ -113,6 +118,14 @@ int tkv_compact(void* k_dst, void* v_dst, float* beta_dst, int32_t* pos_dst, int
                 int32_t* seg_len, int32_t* cu_seqlens, int group,
                 int batch, int hkv, int n_src, int head_dim, int kv_dtype,
                 int32_t* status, tkv_stream_t stream);
+/* The same with the source's log betas of any of the three types and 32- or 64-bit positions. */
+int tkv_compact_as(void* k_dst, void* v_dst, float* beta_dst, int32_t* pos_dst, int64_t cap,
+                   const void* k_src, const void* v_src, int64_t k_sb, int64_t k_sh, int64_t k_ss,
+                   const void* beta_src, int beta_dtype, int64_t beta_stride, const void* pos_src, int pos_bits, int64_t pos_stride,
+                   const int32_t* kept_idx, int64_t kept_stride, const int32_t* kept_cnt,
+                   int32_t* seg_len, int32_t* cu_seqlens, int group,
+                   int batch, int hkv, int n_src, int head_dim, int kv_dtype,
+                   int32_t* status, tkv_stream_t stream);
 
 /*
  * Fused eviction, in place: select (as tkv_evict_select) then stable stream compaction of

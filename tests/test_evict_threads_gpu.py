@@ -30,3 +30,32 @@ def test_widths_agree(nseg, n, m):
     assert ops.read_status(status) == 0 and bool((ln == m).all())
     for t, w in zip((k, v, beta, pos), want):
         assert torch.equal(t.view(nseg, cap, -1)[:, :m], w)
+
+
+# log betas in every type, positions in 32 and 64 bits, shared by all segments and not; a prompt that is reduced and one that is not
+@pytest.mark.gpu
+@pytest.mark.parametrize("beta_type", [torch.float32, torch.bfloat16, torch.float16, torch.float64])
+@pytest.mark.parametrize("pos_type,shared", [(torch.int64, True), (torch.int32, True), (torch.int64, False), (torch.int32, False)])
+@pytest.mark.parametrize("n,transposed", [(333, False), (333, True), (120, False)])
+def test_prompts_in_the_callers_types(beta_type, pos_type, shared, n, transposed):
+    from trimkv_b200 import TrimKVCache
+    g = torch.Generator(device=DEV).manual_seed(n)
+    b, h, d, m, room = 2, 3, 64, 100, 30
+    k, v = (torch.randn(b, h, n, d, generator=g, device=DEV).bfloat16() for _ in range(2))
+    beta = -torch.rand(b, h, n, generator=g, device=DEV).to(beta_type)
+    if transposed:
+        beta = beta.transpose(1, 2).contiguous().transpose(1, 2)
+    pos = torch.arange(n, device=DEV, dtype=pos_type) + 5
+    if not shared:
+        pos = pos.expand(b, h, n) + torch.arange(b * h, device=DEV, dtype=pos_type).view(b, h, 1)
+    at = pos.expand(b, h, n)
+    cache = TrimKVCache(device=DEV)
+    cache.update(k, v, beta, pos, 0)
+    cache.compress(strategy="alpha", memory_size=m, buffer_size=room)
+    cache.check_status()
+    score = beta.float() * (n + 1 - at).float()
+    keep = score.sort(dim=-1, descending=True, stable=True).indices[..., :m].sort(dim=-1).values if n >= m + room else torch.arange(n, device=DEV).expand(b, h, n)
+    assert torch.equal(cache.kv_positions[0].long(), at.long().gather(2, keep))
+    assert torch.equal(cache.retention_weights[0], beta.float().gather(2, keep))
+    assert torch.equal(cache.key_cache[0], k.gather(2, keep[..., None].expand(-1, -1, -1, d)))
+    assert torch.equal(cache.value_cache[0], v.gather(2, keep[..., None].expand(-1, -1, -1, d)))

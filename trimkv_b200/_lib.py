@@ -22,6 +22,8 @@ SIGNATURES = {
     "tkv_last_error": (c_char_p, []),
     "tkv_append": (I, [P, P, P, P, P, P, P, P, L, L, L, P, I, L, L, L, P, L, L, L, I, I, I, I, L, I, P, P]),
     "tkv_evict_select": (I, [P, L, P, L, P, I, I, L, I, I, I, P, P, P, P]),
+    "tkv_evict_select_as": (I, [P, I, L, P, I, L, P, I, I, L, I, I, I, P, P, P, P]),
+    "tkv_compact_as": (I, [P, P, P, P, L, P, P, L, L, L, P, I, L, P, I, L, P, L, P, P, P, I, I, I, I, I, I, P, P]),
     "tkv_compact": (I, [P, P, P, P, L, P, P, L, L, L, P, L, P, L, P, L, P, P, P, I, I, I, I, I, I, P, P]),
     "tkv_evict": (I, [P, P, P, P, P, P, I, I, L, I, I, L, I, I, I, P, P, P]),
     "tkv_evict_ex": (I, [P, P, P, P, P, P, I, I, L, I, I, L, I, I, I, P, I, I, I, P, P, P, P]),

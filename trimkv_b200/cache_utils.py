@@ -336,8 +336,11 @@ class TrimKVCache:
                 continue
             k, v, beta, pos = p
             n = k.shape[2]
-            beta32 = beta.to(torch.float32).reshape(nseg, n).contiguous()
-            pos32 = pos.to(torch.int32).reshape(nseg, n).contiguous()
+            # In the caller's types where the kernels read them: two conversions fewer per layer.
+            held = ops.rows_as_held(beta, pos, nseg, n) if k.device.type == "cuda" else None
+            if held is None:
+                beta32 = beta.to(torch.float32).reshape(nseg, n).contiguous()
+                pos32 = pos.to(torch.int32).reshape(nseg, n).contiguous()
             kept_idx = kept_cnt = None
             if do_select and m is not None and bsz is not None and n >= m + bsz:
                 if n > MAX_ONE_PIECE_PROMPT:
@@ -347,13 +350,17 @@ class TrimKVCache:
                         "model.generate(..., prefill_chunk_size=N) or several forward calls of at most that many tokens")
                 kept_idx = torch.empty(nseg, m, dtype=torch.int32, device=dev)
                 kept_cnt = torch.empty(nseg, dtype=torch.int32, device=dev)
-                ops.evict_select(beta32, pos32, None, n, nseg, self.n_seen_tokens[l] + 1, m, m + bsz, n,
-                                 kept_idx, kept_cnt, self._status)
+                if held is not None:
+                    ops.evict_select_as(*held, n, nseg, self.n_seen_tokens[l] + 1, m, m + bsz, kept_idx, kept_cnt, self._status)
+                else:
+                    ops.evict_select(beta32, pos32, None, n, nseg, self.n_seen_tokens[l] + 1, m, m + bsz, n,
+                                     kept_idx, kept_cnt, self._status)
                 self._cache_len[l] = m
                 if self.record_kept:
                     kept_all.append(kept_idx.view(self._batch, self._hkv, m))
-            ops.compact(s["k"][l], s["v"][l], s["beta"][l], s["pos"][l], self._cap, k, v, beta32, pos32,
-                        kept_idx, kept_cnt, s["len"][l], s["cu"][l], nseg, self._status)
+            gather = ops.compact if held is None else ops.compact_as
+            gather(s["k"][l], s["v"][l], s["beta"][l], s["pos"][l], self._cap, k, v, *(held or (beta32, pos32)),
+                   kept_idx, kept_cnt, s["len"][l], s["cu"][l], nseg, self._status)
             self._pending[l] = None
         if kept_all:
             self.last_kept_idx = torch.stack(kept_all)  # [layers, B, Hkv, M]

@@ -485,8 +485,24 @@ __global__ void __launch_bounds__(kMoveThreads) evict_move_kernel(MoveParams p) 
   }
 }
 
+// Log beta and position of a row as the caller holds them: fp32, bf16 or f16; 32 or 64 bits (positions beyond 32 bits wrap, as a
+// cast does).
+struct RowMeta {
+  const void* beta; int beta_dtype; int64_t beta_stride;   // elements between segments
+  const void* pos; int pos_wide; int64_t pos_stride;
+  __device__ __forceinline__ float beta_at(int seg, int i) const {
+    const int64_t at = (int64_t)seg * beta_stride + i;
+    if (beta_dtype == TKV_F32) return reinterpret_cast<const float*>(beta)[at];
+    if (beta_dtype == TKV_BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(beta)[at]);
+    return __half2float(reinterpret_cast<const __half*>(beta)[at]);
+  }
+  __device__ __forceinline__ int32_t pos_at(int seg, int i) const {
+    const int64_t at = (int64_t)seg * pos_stride + i;
+    return pos_wide ? (int32_t)reinterpret_cast<const int64_t*>(pos)[at] : reinterpret_cast<const int32_t*>(pos)[at];
+  }
+};
 struct SelectParams {
-  const float* beta; int64_t beta_stride; const int32_t* pos; int64_t pos_stride;
+  RowMeta row;
   const int32_t* seg_len; int n_uniform; int nseg; int64_t q_idx;
   int m, trigger_len, max_len;
   int32_t* kept_idx; int32_t* kept_cnt; int32_t* status;
@@ -506,10 +522,8 @@ __global__ void __launch_bounds__(kThreads) evict_select_kernel(SelectParams p) 
     if (threadIdx.x == 0) { report(p.status, TKV_DEV_LEN_BOUND); p.kept_cnt[seg] = n; }
     return;
   }
-  const float* beta = p.beta + (int64_t)seg * p.beta_stride;
-  const int32_t* pos = p.pos + (int64_t)seg * p.pos_stride;
   for (int i = threadIdx.x; i < n; i += kThreads)
-    keys[i] = score_key(retention_score(beta[i], pos[i], p.q_idx));
+    keys[i] = score_key(retention_score(p.row.beta_at(seg, i), p.row.pos_at(seg, i), p.q_idx));
   __syncthreads();
   uint32_t thresh; int n_eq_keep;
   radix_select_mth<kThreads>(keys, n, p.m, &sc, &thresh, &n_eq_keep);
@@ -522,7 +536,7 @@ __global__ void __launch_bounds__(kThreads) evict_select_kernel(SelectParams p) 
 struct CompactParams {
   char* k_dst; char* v_dst; float* beta_dst; int32_t* pos_dst; int64_t cap;
   const char* k_src; const char* v_src; int64_t k_sb, k_sh, k_ss;  // byte strides
-  const float* beta_src; int64_t beta_stride; const int32_t* pos_src; int64_t pos_stride;
+  RowMeta row;
   const int32_t* kept_idx; int64_t kept_stride; const int32_t* kept_cnt;
   int32_t* seg_len; int hkv, n_src, row_vecs;
   int32_t* status;
@@ -562,8 +576,8 @@ __global__ void __launch_bounds__(256) compact_gather_kernel(CompactParams p) {
   for (int r = threadIdx.x; r < rows; r += blockDim.x) {
     const int src = identity ? jb + r : kept[jb + r];
     if ((unsigned)src >= (unsigned)p.n_src) continue;
-    p.beta_dst[dst_row0 + jb + r] = p.beta_src[(int64_t)seg * p.beta_stride + src];
-    p.pos_dst[dst_row0 + jb + r] = p.pos_src[(int64_t)seg * p.pos_stride + src];
+    p.beta_dst[dst_row0 + jb + r] = p.row.beta_at(seg, src);
+    p.pos_dst[dst_row0 + jb + r] = p.row.pos_at(seg, src);
   }
 }
 
@@ -755,12 +769,27 @@ extern "C" int tkv_evict_ex(void* k_cache, void* v_cache, float* beta_cache, int
                     keep_cnt, protect_last, strategy, kept_idx_out, status, stream, 1, nullptr, 0, scores);
 }
 
+static int check_row_meta(const char* what, int beta_dtype, int pos_bits) {
+  if (tkv::elem_size(beta_dtype) == 0 || (pos_bits != 32 && pos_bits != 64))
+    return tkv::fail(TKV_ERR_ARG, "%s: beta_dtype=%d, positions of %d bits", what, beta_dtype, pos_bits);
+  return TKV_OK;
+}
+
 extern "C" int tkv_evict_select(const float* beta, int64_t beta_stride, const int32_t* pos, int64_t pos_stride,
+                                const int32_t* seg_len, int n_uniform, int nseg, int64_t q_idx,
+                                int memory_size, int trigger_len, int max_len,
+                                int32_t* kept_idx, int32_t* kept_cnt, int32_t* status, tkv_stream_t stream) {
+  return tkv_evict_select_as(beta, TKV_F32, beta_stride, pos, 32, pos_stride, seg_len, n_uniform, nseg, q_idx, memory_size, trigger_len,
+                             max_len, kept_idx, kept_cnt, status, stream);
+}
+
+extern "C" int tkv_evict_select_as(const void* beta, int beta_dtype, int64_t beta_stride, const void* pos, int pos_bits, int64_t pos_stride,
                                 const int32_t* seg_len, int n_uniform, int nseg, int64_t q_idx,
                                 int memory_size, int trigger_len, int max_len,
                                 int32_t* kept_idx, int32_t* kept_cnt, int32_t* status, tkv_stream_t stream) {
   using namespace tkv;
   if (!beta || !pos || !kept_idx || !kept_cnt) return fail(TKV_ERR_ARG, "tkv_evict_select: NULL pointer argument");
+  if (const int rc = check_row_meta("tkv_evict_select", beta_dtype, pos_bits)) return rc;
   if (nseg < 0 || memory_size <= 0 || max_len <= 0 || (seg_len == nullptr && n_uniform < 0))
     return fail(TKV_ERR_ARG, "tkv_evict_select: bad sizes nseg=%d M=%d max_len=%d", nseg, memory_size, max_len);
   if (seg_len == nullptr && n_uniform > max_len)
@@ -769,7 +798,7 @@ extern "C" int tkv_evict_select(const float* beta, int64_t beta_stride, const in
     return fail(TKV_ERR_UNSUPPORTED, "tkv_evict_select: max_len=%d exceeds %d", max_len, kMaxSelectLen);
   if (nseg == 0) return TKV_OK;
   SelectParams p;
-  p.beta = beta; p.beta_stride = beta_stride; p.pos = pos; p.pos_stride = pos_stride;
+  p.row = {beta, beta_dtype, beta_stride, pos, pos_bits == 64, pos_stride};
   p.seg_len = seg_len; p.n_uniform = n_uniform; p.nseg = nseg; p.q_idx = q_idx;
   p.m = memory_size; p.trigger_len = trigger_len; p.max_len = max_len;
   p.kept_idx = kept_idx; p.kept_cnt = kept_cnt; p.status = status;
@@ -790,11 +819,24 @@ extern "C" int tkv_compact(void* k_dst, void* v_dst, float* beta_dst, int32_t* p
                            int32_t* seg_len, int32_t* cu_seqlens, int group,
                            int batch, int hkv, int n_src, int head_dim, int kv_dtype,
                            int32_t* status, tkv_stream_t stream) {
+  return tkv_compact_as(k_dst, v_dst, beta_dst, pos_dst, cap, k_src, v_src, k_sb, k_sh, k_ss, beta_src, TKV_F32, beta_stride, pos_src, 32,
+                        pos_stride, kept_idx, kept_stride, kept_cnt, seg_len, cu_seqlens, group, batch, hkv, n_src, head_dim, kv_dtype, status,
+                        stream);
+}
+
+extern "C" int tkv_compact_as(void* k_dst, void* v_dst, float* beta_dst, int32_t* pos_dst, int64_t cap,
+                              const void* k_src, const void* v_src, int64_t k_sb, int64_t k_sh, int64_t k_ss,
+                              const void* beta_src, int beta_dtype, int64_t beta_stride, const void* pos_src, int pos_bits, int64_t pos_stride,
+                              const int32_t* kept_idx, int64_t kept_stride, const int32_t* kept_cnt,
+                              int32_t* seg_len, int32_t* cu_seqlens, int group,
+                              int batch, int hkv, int n_src, int head_dim, int kv_dtype,
+                              int32_t* status, tkv_stream_t stream) {
   using namespace tkv;
   const int es = elem_size(kv_dtype);
   if (es == 0) return fail(TKV_ERR_ARG, "tkv_compact: unknown kv_dtype %d", kv_dtype);
   if (!k_dst || !v_dst || !beta_dst || !pos_dst || !k_src || !v_src || !beta_src || !pos_src || !seg_len)
     return fail(TKV_ERR_ARG, "tkv_compact: NULL pointer argument");
+  if (const int rc = check_row_meta("tkv_compact", beta_dtype, pos_bits)) return rc;
   if (batch < 0 || hkv <= 0 || n_src < 0 || head_dim <= 0 || cap <= 0)
     return fail(TKV_ERR_ARG, "tkv_compact: bad sizes");
   const int64_t row_bytes = (int64_t)head_dim * es;
@@ -810,7 +852,7 @@ extern "C" int tkv_compact(void* k_dst, void* v_dst, float* beta_dst, int32_t* p
   p.k_dst = (char*)k_dst; p.v_dst = (char*)v_dst; p.beta_dst = beta_dst; p.pos_dst = pos_dst; p.cap = cap;
   p.k_src = (const char*)k_src; p.v_src = (const char*)v_src;
   p.k_sb = k_sb * es; p.k_sh = k_sh * es; p.k_ss = k_ss * es;
-  p.beta_src = beta_src; p.beta_stride = beta_stride; p.pos_src = pos_src; p.pos_stride = pos_stride;
+  p.row = {beta_src, beta_dtype, beta_stride, pos_src, pos_bits == 64, pos_stride};
   p.kept_idx = kept_idx; p.kept_stride = kept_stride; p.kept_cnt = kept_cnt;
   p.seg_len = seg_len; p.hkv = hkv; p.n_src = n_src; p.row_vecs = (int)(row_bytes / 16); p.status = status;
   const int max_rows = (int)(n_src < cap ? n_src : cap);

@@ -121,6 +121,42 @@ def compact(k_dst, v_dst, beta_dst, pos_dst, cap: int, k_src, v_src, beta_src, p
     _count(1 if cu_seqlens is None else 2)
 
 
+_POS_BITS = {torch.int32: 32, torch.int64: 64}
+
+
+def rows_as_held(beta, pos, nseg: int, n: int):
+    """Log betas and positions ``[B,H,n]`` of a prompt as :func:`evict_select_as` and :func:`compact_as` read them: in their own types,
+    ``[nseg, n]``, positions that all segments share as ``[n]``; None for types those do not read."""
+    if beta.dtype not in _DTYPE or pos.dtype not in _POS_BITS:
+        return None
+    shared = all(size == 1 or step == 0 for size, step in zip(pos.shape[:2], pos.stride()[:2])) and pos.shape[2:] == (n,)
+    return beta.reshape(nseg, n).contiguous(), (pos[0, 0] if shared else pos.reshape(nseg, n)).contiguous()
+
+
+def evict_select_as(beta, pos, n: int, nseg: int, q_idx: int, memory_size: int, trigger_len: int, kept_idx, kept_cnt, status=None) -> None:
+    """:func:`evict_select` of ``nseg`` segments of ``n`` tokens from :func:`rows_as_held`."""
+    check(lib().tkv_evict_select_as(
+        beta.data_ptr(), dtype_code(beta.dtype), beta.stride(0), pos.data_ptr(), _POS_BITS[pos.dtype], 0 if pos.dim() == 1 else pos.stride(0),
+        None, n, nseg, q_idx, memory_size, trigger_len, n, kept_idx.data_ptr(), kept_cnt.data_ptr(), _ptr(status), _stream(beta)),
+        "tkv_evict_select_as")
+    _count(1)
+
+
+def compact_as(k_dst, v_dst, beta_dst, pos_dst, cap: int, k_src, v_src, beta_src, pos_src, kept_idx, kept_cnt,
+               seg_len, cu_seqlens, group: int, status=None) -> None:
+    """:func:`compact` with log betas and positions from :func:`rows_as_held`."""
+    b, h, n, d = k_src.shape
+    if v_src.stride() != k_src.stride() or k_src.stride(3) != 1:
+        k_src = k_src.contiguous(); v_src = v_src.contiguous()
+    check(lib().tkv_compact_as(
+        k_dst.data_ptr(), v_dst.data_ptr(), beta_dst.data_ptr(), pos_dst.data_ptr(), cap,
+        k_src.data_ptr(), v_src.data_ptr(), k_src.stride(0), k_src.stride(1), k_src.stride(2),
+        beta_src.data_ptr(), dtype_code(beta_src.dtype), beta_src.stride(0), pos_src.data_ptr(), _POS_BITS[pos_src.dtype],
+        0 if pos_src.dim() == 1 else pos_src.stride(0), _ptr(kept_idx), 0 if kept_idx is None else kept_idx.stride(0), _ptr(kept_cnt),
+        seg_len.data_ptr(), _ptr(cu_seqlens), group, b, h, n, d, dtype_code(k_dst.dtype), _ptr(status), _stream(k_dst)), "tkv_compact_as")
+    _count(1 if cu_seqlens is None else 2)
+
+
 def rebuild_cu_seqlens(seg_len, cu_seqlens, nseg: int, group: int) -> None:
     check(lib().tkv_rebuild_cu_seqlens(seg_len.data_ptr(), cu_seqlens.data_ptr(), nseg, group, _stream(seg_len)),
           "tkv_rebuild_cu_seqlens")
