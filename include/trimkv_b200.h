@@ -452,6 +452,11 @@ int tkv_skinny_gemm_swiglu(const void* gate_up, const void* w, float* partial, i
  * vectors (norms, biases, convolution taps) are fp32 arrays.  No counterpart in the reference.
  */
 
+/* out[m, n] = x[m, k] . w[n, k]^T of up to 16 rows (bf16; rows of x and w of whole 16-byte pieces on 16-byte boundaries), strides in
+ * elements.  The weights are not written by the kernel before this one in the stream. */
+int tkv_few_gemm(const void* x, int64_t x_stride, const void* w, void* out, int64_t out_stride, int m, int n, int k, int dtype,
+                 tkv_stream_t stream);
+
 /* dst[i] = host_values[i], and dst[host_index[i]] = value, for i in [0, n).  The host arrays are read before the call returns and
  * travel as launch arguments: no copy is queued and nothing is waited for. */
 int tkv_put_ints(int32_t* dst, const int32_t* host_values, int n, tkv_stream_t stream);
