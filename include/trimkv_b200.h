@@ -457,6 +457,11 @@ int tkv_skinny_gemm_swiglu(const void* gate_up, const void* w, float* partial, i
 int tkv_few_gemm(const void* x, int64_t x_stride, const void* w, void* out, int64_t out_stride, int m, int n, int k, int dtype,
                  tkv_stream_t stream);
 
+/* next[r] = ids[r] = index of the largest of the `vocab` logits (bf16 or fp32) of row r, the first of equals, a NaN above all;
+ * *pos += 1. */
+int tkv_greedy_next(const void* logits, int64_t stride, int rows, int vocab, int dtype, int64_t* next, int64_t* ids, int64_t* pos,
+                    tkv_stream_t stream);
+
 /* dst[i] = host_values[i], and dst[host_index[i]] = value, for i in [0, n).  The host arrays are read before the call returns and
  * travel as launch arguments: no copy is queued and nothing is waited for. */
 int tkv_put_ints(int32_t* dst, const int32_t* host_values, int n, tkv_stream_t stream);

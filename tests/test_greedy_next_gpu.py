@@ -1,0 +1,37 @@
+"""The next token of every row and the step's position in one kernel."""
+import pytest
+import torch
+
+from trimkv_b200 import ops
+
+DEV = "cuda"
+
+
+# whole vectors and single elements (odd sizes, rows that do not start on 16 bytes), less and more than a round of a CTA
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vocab,shift", [(1, 0), (7, 0), (8, 0), (1000, 0), (1000, 3), (32768, 0), (50257, 0), (8 * 4096 + 8, 0)])
+def test_same_as_argmax(vocab, shift, dtype):
+    g = torch.Generator(device=DEV).manual_seed(vocab)
+    rows = 6
+    z = torch.randn(rows, vocab + 16, generator=g, device=DEV).to(dtype)[:, shift:shift + vocab]
+    z[1] = z[1].clamp(max=0.0)                  # many equals: the first counts
+    z[2] = float("-inf")
+    z[3, vocab // 2:] = float("nan")
+    z[4] = -0.0
+    z[4, vocab // 3] = 0.0
+    z[5, vocab - 1] = float("inf")
+    nxt, ids, pos = torch.full((rows, 1), -1, device=DEV), torch.full((rows, 1), -1, device=DEV), torch.tensor([41], device=DEV)
+    assert ops.greedy_next(z, nxt, ids, pos)
+    want = z.float().cpu().argmax(-1, keepdim=True)
+    assert torch.equal(nxt.cpu(), want) and torch.equal(ids.cpu(), want) and pos.item() == 42
+
+
+@pytest.mark.gpu
+def test_logits_it_leaves_alone():
+    nxt = torch.zeros(2, 1, dtype=torch.int64, device=DEV)
+    pos = torch.zeros(1, dtype=torch.int64, device=DEV)
+    z = torch.zeros(2, 64, device=DEV)
+    for bad in (z.half(), z.double(), z[None], z.t()[:, :2], z[:0], z.cpu()):
+        assert not ops.greedy_next(bad, nxt, nxt, pos)
+    assert not ops.greedy_next(z, nxt.int(), nxt, pos) and pos.item() == 0

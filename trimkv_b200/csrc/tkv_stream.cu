@@ -8,6 +8,7 @@
 //   gated_norm_kernel    : group RMSNorm, a SiLU gate before or after it or none, optional weight;
 //   swiglu_kernel        : silu(gate) * up of one projection row;
 //   gelu_tanh_kernel     : the tanh form of GELU, in place;
+//   greedy_next_kernel   : largest logit of every row as the next token, and the step's position;
 //   batch_begin_kernel   : start positions of a step's requests, and the lengths after it;
 //   put_ints_kernel      : a few host integers into a device array, as launch arguments.
 // All statistics are fp32.  Every kernel runs for the 16-bit model type and for fp32.
@@ -443,6 +444,57 @@ __global__ void __launch_bounds__(kRowThreads) swiglu_kernel(const T* u, int64_t
   }
 }
 
+// next[r] = ids[r] = index of the largest of a row's logits (the first of equals, a NaN above all); *pos += 1.  One CTA per row, a
+// thread's vectors of a round requested together.  In the place of a reduction over few blocks, two copies and an addition
+// (10.8 us and three more launches for 8 rows of 32768).
+constexpr int kNextThreads = 1024;
+template <typename T, int V>
+__global__ void __launch_bounds__(kNextThreads) greedy_next_kernel(const T* logits, int64_t stride, int vocab, int64_t* next, int64_t* ids, int64_t* pos) {
+  constexpr int kAhead = 4;
+  __shared__ unsigned long long best_of[kNextThreads / 32];
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const T* row = logits + (int64_t)blockIdx.x * stride;
+  const int nvec = vocab / V;
+  unsigned long long best = 0ull;                          // order-preserving key, then the complement of the index
+  for (int64_t i0 = threadIdx.x; i0 < nvec; i0 += kAhead * kNextThreads) {
+    RawVec<T, V> x[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (i0 + u * kNextThreads < nvec) x[u].load(row + (i0 + u * kNextThreads) * V);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (i0 + u * kNextThreads >= nvec) break;
+      float v[V];
+      x[u].floats(v);
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const unsigned long long k = ((unsigned long long)score_key(v[e]) << 32) | (uint32_t)~(uint32_t)((i0 + u * kNextThreads) * V + e);
+        best = k > best ? k : best;
+      }
+    }
+  }
+  auto warp_best = [&]() {
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) {
+      const unsigned long long o = __shfl_xor_sync(0xffffffffu, best, d);
+      best = o > best ? o : best;
+    }
+  };
+  warp_best();
+  if ((threadIdx.x & 31) == 0) best_of[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  best = best_of[threadIdx.x];
+  warp_best();
+  if (threadIdx.x == 0) {
+    const int64_t at = (int64_t)(uint32_t)~(uint32_t)best;
+    next[blockIdx.x] = at;
+    ids[blockIdx.x] = at;
+    if (blockIdx.x == 0) *pos += 1;
+  }
+}
+
 __global__ void batch_begin_kernel(int32_t* lens, const int32_t* slots, const int32_t* cu, int32_t* pos0, int batch) {
   grid_dependency_wait();
   grid_launch_dependents();
@@ -638,6 +690,21 @@ extern "C" int tkv_batch_begin(int32_t* lens, const int32_t* slots, const int32_
                              pos0, batch);
   if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_batch_begin: %s", cudaGetErrorString(e));
   return check_launch("tkv_batch_begin");
+}
+
+extern "C" int tkv_greedy_next(const void* logits, int64_t stride, int rows, int vocab, int dtype, int64_t* next, int64_t* ids, int64_t* pos,
+                               tkv_stream_t stream) {
+  using namespace tkv;
+  if (!logits || !next || !ids || !pos) return fail(TKV_ERR_ARG, "tkv_greedy_next: NULL pointer argument");
+  if (!is_model_dtype(dtype)) return fail(TKV_ERR_UNSUPPORTED, "tkv_greedy_next: dtype %d", dtype);
+  if (rows <= 0 || vocab <= 0 || stride < vocab) return fail(TKV_ERR_ARG, "tkv_greedy_next: bad sizes rows=%d vocab=%d", rows, vocab);
+  const bool vec = vocab % 8 == 0 && (stride * elem_size(dtype)) % 16 == 0 && aligned16(logits);
+  TKV_WITH_TYPE(dtype, T, {
+    cudaError_t e = launch_pdl(vec ? greedy_next_kernel<T, 8> : greedy_next_kernel<T, 1>, dim3((unsigned)rows), dim3(kNextThreads), 0,
+                               (cudaStream_t)stream, (const T*)logits, stride, vocab, next, ids, pos);
+    if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_greedy_next: %s", cudaGetErrorString(e));
+  });
+  return check_launch("tkv_greedy_next");
 }
 
 extern "C" int tkv_put_ints(int32_t* dst, const int32_t* host_values, int n, tkv_stream_t stream) {

@@ -257,9 +257,10 @@ class GreedyDecoder:
             finally:
                 cfg.compress_memory, cfg.fused_decode_step = compress, auto
             self.logits = out.logits[:, -1]
-        self.next_ids.copy_(self.logits.argmax(-1, keepdim=True))
-        self.ids.copy_(self.next_ids)
-        self.pos.add_(1)
+        if not ops.greedy_next(self.logits, self.next_ids, self.ids, self.pos):
+            self.next_ids.copy_(self.logits.argmax(-1, keepdim=True))
+            self.ids.copy_(self.next_ids)
+            self.pos.add_(1)
 
     def capture(self):
         """Records one decode step.  Views handed to attention span the full capacity so the recorded

@@ -483,6 +483,19 @@ def linear(x, w) -> torch.Tensor:
     return F.linear(x, w)
 
 
+def greedy_next(logits, next_ids, ids, pos) -> bool:
+    """``next_ids = ids = logits.argmax(-1, keepdim=True)``, ``pos += 1`` in one kernel; False (and nothing done) for logits it does
+    not read."""
+    if (logits.dim() != 2 or logits.dtype not in (torch.bfloat16, torch.float32) or not logits.is_cuda or logits.stride(1) != 1
+            or logits.stride(0) < logits.shape[1] or logits.shape[0] == 0 or logits.device.index != torch.cuda.current_device()
+            or not all(t.dtype == torch.int64 and t.is_contiguous() and t.device == logits.device for t in (next_ids, ids, pos))):
+        return False
+    check(lib().tkv_greedy_next(logits.data_ptr(), logits.stride(0), logits.shape[0], logits.shape[1], dtype_code(logits.dtype),
+                                next_ids.data_ptr(), ids.data_ptr(), pos.data_ptr(), _stream(logits)), "tkv_greedy_next")
+    _count(1)
+    return True
+
+
 def ints_on(device, values) -> torch.Tensor:
     """A few host integers as an int32 tensor on ``device``: launch arguments of a small kernel instead of a copy, so that the
     host neither stages nor waits."""
