@@ -271,6 +271,11 @@ __device__ __forceinline__ bool pair_meet(PairSmem* sm, int phase) {
   return (bool)__all_sync(0xffffffffu, ok);
 }
 
+// Whether CTAs of two tiles of rows take less time than CTAs of one: a CTA per SM at a time, 2.6 us per key tile for a pair against
+// 1.64 us for a tile with the chain of its own (64 segments of 192 rows, 33 key tiles: 89 us as 64 pairs, 60 us as 128 tiles; 64
+// segments of 2048 rows: 329 us as 512 pairs, 394 us as 1024 tiles).  One tile only is never a pair.
+inline bool pair_is_faster(int64_t tiles, int64_t pairs) { return pairs < tiles && (pairs + 147) / 148 * 8 < (tiles + 147) / 148 * 5; }
+
 // TMEM is given back; an aborting CTA first waits for the copies it started.
 template <typename Shape>
 __device__ __forceinline__ void pair_finish(PairSmem* sm, uint32_t tmem, int nk, int nv) {
