@@ -3,7 +3,6 @@
 //   moe_route_kernel : softmax scores, choice among the experts of the best groups, weights, and each choice's rank among the
 //                      choices of its expert; with one CTA (few tokens) also the places;
 //   moe_place_kernel : first row of every expert, row of every choice, token of every row;
-//   moe_few_kernel   : grouped product of few rows per expert;
 //   moe_any_kernel   : grouped product on the CUDA cores.
 // The last `identity` experts return their input: they own no rows, their choices get place -1.
 #include "tkv_moe.cuh"
@@ -230,95 +229,6 @@ __global__ void __launch_bounds__(kPlaceThreads) moe_place_kernel(MoeRoute p) {
   }
 }
 
-// ------------------------------------------------------------------------------------------------ few rows per expert
-// A decoding step reads every weight of the experts it meets once for a handful of rows: HBM bounds it.  One CTA per (expert, 32
-// rows of its weights): four warps split k and add their parts in warp order.  A lane copies the 16-byte pieces of its own
-// fragments of m16n8k16 (a product does not mind in which order k is walked if both operands agree) into places of its own in
-// shared memory, eight steps ahead, so that no thread ever waits for another one; the 128 KB units are spread over the SMs by the
-// block scheduler, where tiles of 128 weight columns on tcgen05 left the SMs of a last, nearly empty round idle.
-// us for 32 experts of 2048 -> 1536 and 1536 -> 2048, T tokens with 6 of 36 choices each, against tcgen05: T = 1 8.8 / 17.1 and
-// 11.0 / 21.8, T = 4 21.9 / 37.2 and 23.5 / 24.6, T = 8 28.1 / 30.5 and 29.6 / 32.8 (4.4 TB/s), T = 21 37.9 / 41.2 and 40.3 / 41.5.
-constexpr int kFewWarps = 4, kFewTiles = 2, kFewRows = 16 * kFewTiles, kFewTokens = 8, kFewAhead = 8, kFewPieces = 2 * kFewTiles + 1;
-constexpr int kFewBytes = kFewWarps * kFewAhead * kFewPieces * 512;
-
-__device__ __forceinline__ void few_mma(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
-__global__ void __launch_bounds__(kFewWarps * 32, 2) moe_few_kernel(GroupedGemm p) {
-  extern __shared__ __align__(16) uint8_t ring[];         // [warp][step][piece][lane] of 16 bytes: rows of weights, one of A
-  constexpr int kPitch = kFewRows + 1;
-  float* part = reinterpret_cast<float*>(ring);           // [warp][token][kPitch], in the place of the pieces
-  static_assert(kFewWarps * kFewTokens * kPitch * 4 <= kFewBytes, "the parts take the place of the pieces");
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
-  const int e = blockIdx.y, row0 = blockIdx.x * kFewRows;
-  const int steps = (p.k + 31) / 32, s0 = (int)((int64_t)warp * steps / kFewWarps), s1 = (int)((int64_t)(warp + 1) * steps / kFewWarps);
-  const uint32_t start = (uint32_t)__cvta_generic_to_shared(ring), mine = (uint32_t)(warp * kFewAhead * kFewPieces * 512 + lane * 16);
-  auto place = [&](int s) { return mine + (uint32_t)((s - s0) % kFewAhead * kFewPieces * 512); };
-  // rows that do not exist repeat the last one: a row of either operand reaches only its own results, and those are not stored
-  const __nv_bfloat16* w[2 * kFewTiles];
-#pragma unroll
-  for (int r = 0; r < 2 * kFewTiles; ++r) w[r] = (const __nv_bfloat16*)p.w + ((int64_t)e * p.n + min(row0 + g + 8 * r, p.n - 1)) * p.k + c * 8;
-  grid_dependency_wait();
-  grid_launch_dependents();
-  const int hi = p.offsets[e + 1];
-  for (int r0 = p.offsets[e]; r0 < hi; r0 += kFewTokens) {
-    const int r = min(r0 + g, hi - 1);                    // this lane's row of A
-    const __nv_bfloat16* x = (const __nv_bfloat16*)p.a + (int64_t)(p.src != nullptr ? p.src[r] : r) * p.a_stride + c * 8;
-    auto copy = [](uint32_t dst, const __nv_bfloat16* src, int bytes) {
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-    };
-    auto fetch = [&](int s) {                             // a group per step, empty beyond the end
-      if (s < s1) {
-        const bool in = s * 32 + c * 8 < p.k;             // k is whole pieces of 8: its last step may lack some, zeros then
-        const int at = in ? s * 32 : -c * 8, bytes = in ? 16 : 0;
-#pragma unroll
-        for (int i = 0; i < 2 * kFewTiles; ++i) copy(start + place(s) + i * 512, w[i] + at, bytes);
-        copy(start + place(s) + kFewTiles * 1024, x + at, bytes);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-#pragma unroll
-    for (int u = 0; u < kFewAhead; ++u) fetch(s0 + u);
-    float acc[kFewTiles][4] = {};
-    for (int s = s0; s < s1; ++s) {
-      asm volatile("cp.async.wait_group %0;" ::"n"(kFewAhead - 1) : "memory");
-      const uint4* at = reinterpret_cast<const uint4*>(ring + place(s));
-      const uint4 b = at[64 * kFewTiles];
-#pragma unroll
-      for (int i = 0; i < kFewTiles; ++i) {
-        const uint4 a0 = at[64 * i], a1 = at[64 * i + 32];
-        few_mma(acc[i], a0.x, a1.x, a0.y, a1.y, b.x, b.y);
-        few_mma(acc[i], a0.z, a1.z, a0.w, a1.w, b.z, b.w);
-      }
-      fetch(s + kFewAhead);
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < kFewTiles; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) part[(warp * kFewTokens + 2 * c + (j & 1)) * kPitch + 16 * i + g + 8 * (j >> 1)] = acc[i][j];
-    __syncthreads();
-    for (int i = tid; i < kFewTokens * kFewRows; i += kFewWarps * 32) {
-      const int t = i / kFewRows, row = i - t * kFewRows;
-      float v = 0.f;
-#pragma unroll
-      for (int j = 0; j < kFewWarps; ++j) v += part[(j * kFewTokens + t) * kPitch + row];
-      if (r0 + t < hi && row0 + row < p.n)
-        ((__nv_bfloat16*)p.out)[(int64_t)(r0 + t) * p.n + row0 + row] = __float2bfloat16_rn(p.act == 1 ? gelu_erf(v) : v);
-    }
-    __syncthreads();
-  }
-}
-
-// Up to kFewMost rows per expert on average: an expert with more takes its weights from L2 again for every eight of them, and from
-// about six on the tensor cores' tiles are as fast.
-constexpr int kFewMost = 4;
-static bool moe_few_shape(const GroupedGemm& p) { return p.max_rows <= (int64_t)kFewMost * p.experts && p.experts <= 65535; }
-
 // ------------------------------------------------------------------------------------------------ any size, fp32 arithmetic
 constexpr int kAnyM = 32, kAnyN = 64, kAnyK = 16, kAnyThreads = 256;
 
@@ -431,18 +341,7 @@ extern "C" int tkv_moe_gemm(const void* a, int64_t a_stride, int64_t a_rows, con
   if (max_rows > INT32_MAX || a_rows > INT32_MAX) return fail(TKV_ERR_UNSUPPORTED, "tkv_moe_gemm: %lld rows", (long long)max_rows);
   GroupedGemm p = {a, a_stride, a_rows, src, w, offsets, out, experts, n, k, act, max_rows, status};
   cudaStream_t st = (cudaStream_t)stream;
-  if (moe_tc_shape(p, dtype)) {
-    if (!moe_few_shape(p)) return launch_moe_tc(p, st);
-    static bool configured = false;
-    if (!configured) {
-      cudaError_t e = cudaFuncSetAttribute(moe_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFewBytes);
-      if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_moe_gemm: %s", cudaGetErrorString(e));
-      configured = true;
-    }
-    cudaError_t e = launch_pdl(moe_few_kernel, dim3((n + kFewRows - 1) / kFewRows, experts), dim3(kFewWarps * 32), (size_t)kFewBytes, st, p);
-    if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_moe_gemm: %s", cudaGetErrorString(e));
-    return check_launch("tkv_moe_gemm");
-  }
+  if (moe_tc_shape(p, dtype)) return launch_moe_tc(p, st);
   const int64_t tiles = max_rows / kAnyM + (experts < max_rows ? experts : max_rows);
   if (tiles > 65535) return fail(TKV_ERR_UNSUPPORTED, "tkv_moe_gemm: %lld row tiles", (long long)tiles);
   const dim3 grid((n + kAnyN - 1) / kAnyN, (unsigned)tiles);
