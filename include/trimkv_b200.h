@@ -452,11 +452,6 @@ int tkv_skinny_gemm_swiglu(const void* gate_up, const void* w, float* partial, i
  * vectors (norms, biases, convolution taps) are fp32 arrays.  No counterpart in the reference.
  */
 
-/* out[m, n] = x[m, k] . w[n, k]^T of up to 16 rows (bf16; rows of x and w of whole 16-byte pieces on 16-byte boundaries), strides in
- * elements.  The weights are not written by the kernel before this one in the stream. */
-int tkv_few_gemm(const void* x, int64_t x_stride, const void* w, void* out, int64_t out_stride, int m, int n, int k, int dtype,
-                 tkv_stream_t stream);
-
 /* next[r] = ids[r] = index of the largest of the `vocab` logits (bf16 or fp32) of row r, the first of equals, a NaN above all;
  * *pos += 1. */
 int tkv_greedy_next(const void* logits, int64_t stride, int rows, int vocab, int dtype, int64_t* next, int64_t* ids, int64_t* pos,

@@ -53,7 +53,6 @@ SIGNATURES = {
     "tkv_skinny_gemm_splits": (I, [I, I, I]),
     "tkv_skinny_gemm": (I, [P, P, P, I, I, I, I, P, P]),
     "tkv_skinny_gemm_swiglu": (I, [P, P, P, I, I, I, I, P, P]),
-    "tkv_few_gemm": (I, [P, L, P, P, L, I, I, I, I, P]),
     "tkv_greedy_next": (I, [P, L, I, I, I, P, P, P, P]),
     "tkv_put_ints": (I, [P, P, I, P]),
     "tkv_set_ints": (I, [P, P, I, I, P]),

@@ -62,7 +62,7 @@ class SwiGLU(FeedForward):
         u = self.proj(x)
         act = torch.empty(x.shape[0], self.ff, dtype=x.dtype, device=x.device)
         ops.swiglu(u, act)
-        y = ops.linear(act, self.down)
+        y = F.linear(act, self.down)
         return (y, self._gate(u)) if self.gate_rows else y
 
 

@@ -12,6 +12,7 @@ import math
 from typing import Dict, Optional
 
 import torch
+import torch.nn.functional as F
 from torch import nn
 
 from . import ops
@@ -60,7 +61,7 @@ class FusedProjection(nn.Module):
             self.weight[self.used:].zero_()
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return ops.linear(x, self.weight)
+        return F.linear(x, self.weight)
 
 
 def rotary_frequencies(base: float, dims: int) -> torch.Tensor:
@@ -146,14 +147,14 @@ class RetentionMixer(Mixer):
         freq = self._freq(x.device)
         if batch.cu is None:
             ops.retention_step(u, data["state"], batch, self._decay(x.device, False), freq, out, d, self.rot_dims, d ** -0.5, self.eps)
-            return ops.linear(out, self.o)
+            return F.linear(out, self.o)
         qk = torch.empty(x.shape[0], 2 * h * d, dtype=x.dtype, device=x.device)
         ops.rotate_qk(u, qk, batch, h, d, self.rot_dims, freq, d ** -0.5)
         y = torch.empty_like(out)
         ops.linrec(qk[:, :h * d], qk[:, h * d:], u[:, 2 * h * d:2 * h * d + h * p], data["state"], batch, y, h,
                    head_decay=self._decay(x.device, False), head_log_decay=self._decay(x.device, True))
         ops.gated_norm(y, u[:, 2 * h * d + h * p:2 * h * (d + p)], None, out, h, self.eps, gate_first=False)
-        return ops.linear(out, self.o)
+        return F.linear(out, self.o)
 
 
 class SSDMixer(Mixer):
@@ -212,7 +213,7 @@ class SSDMixer(Mixer):
                        log_decay=log_decay, v_scale=dt, skip=skip)
         out = torch.empty_like(y)
         ops.gated_norm(y, u[:, :inner], as_f32(self, "norm"), out, self.norm_groups, self.eps, gate_first=True)
-        return ops.linear(out, self.o)
+        return F.linear(out, self.o)
 
 
 class DifferentialAttentionMixer(Mixer):
@@ -263,7 +264,7 @@ class DifferentialAttentionMixer(Mixer):
         g0, g1 = self.proj.offsets["g"]
         ops.diff_attention(u, u[:, g0:g1], as_f32(self, "q_norm"), as_f32(self, "k_norm"), data["k"], data["v"], batch,
                            self._lambda(), self.diff, self.scale, self.eps, out, self.heads, self.dim, self.vdim, self.window)
-        return ops.linear(out, self.o)
+        return F.linear(out, self.o)
 
 
 class HGRN2Mixer(Mixer):
@@ -304,7 +305,7 @@ class HGRN2Mixer(Mixer):
             y = torch.empty_like(out)
             ops.chanrec(q, f, v, bias, lower, data["state"], batch, y)
             ops.gated_norm(y, None, norm, out, h, self.eps)
-        y = ops.linear(out, self.o)
+        y = F.linear(out, self.o)
         return (y, self._gate(u)) if self.gate_rows else y
 
 
@@ -352,7 +353,7 @@ class LatentAttentionMixer(Mixer):
         u, freq = self.proj(x), self._freq(x.device)
         cq, lin = ops.latent_prep(u, as_f32(self, "q_norm"), as_f32(self, "kv_norm"), self.eps, r, self.rot_dims, freq, data["latent"],
                                   batch, self.window)
-        q = ops.linear(cq, self.uq)
+        q = F.linear(cq, self.uq)
         out = torch.empty(T, h * p, dtype=x.dtype, device=x.device)
         if batch.cu is None:
             q3 = q.view(T, h, d + r)
@@ -364,7 +365,7 @@ class LatentAttentionMixer(Mixer):
             ops.rotate_pairs(q, batch, h, d + r, d, self.rot_dims, freq)
             kv = self.ukv(lin[:, :rank])
             ops.latent_prefill(q, kv, lin, batch, self.scale, out, h, d, r, p, rank, self.window)
-        y = ops.linear(out, self.o)
+        y = F.linear(out, self.o)
         return (y, self._gate(u)) if self.gate_rows else y
 
 
@@ -384,9 +385,9 @@ class GeluMLP(nn.Module):
         nn.init.normal_(self.down, mean=0.0, std=std)
 
     def forward(self, x):
-        u = ops.linear(x, self.up)
+        u = F.linear(x, self.up)
         ops.gelu_tanh(u)
-        return ops.linear(u, self.down)
+        return F.linear(u, self.down)
 
 
 __all__ = ["DifferentialAttentionMixer", "FusedProjection", "GeluMLP", "HGRN2Mixer", "LatentAttentionMixer", "Mixer",

@@ -9,7 +9,6 @@ import ctypes
 from typing import Optional
 
 import torch
-import torch.nn.functional as F
 
 from . import _lib
 from ._lib import TKV_BF16, TKV_F16, TKV_F32, check, lib
@@ -462,26 +461,6 @@ update_flatten_view_triton = update_flatten_view  # the reference's name for the
 # --------------------------------------------------------------------------------------------------------------------
 # Decoders with recurrent layers, windowed attention and experts.  ``batch`` is a ``state_cache.StepBatch``: packed
 # tokens, ``cu`` (None in a one-token step), ``slots`` and ``pos0`` of the step's requests.
-
-# Rows and columns up to which the kernel for few rows takes a projection: its CTAs are all on the SMs at once then.  With 14336
-# columns it is no faster than the library for 8 rows and slower for 16; with 32 rows what a product of 2048 columns gains is lost
-# again in a whole step.
-FEW_ROWS, FEW_COLUMNS = 16, 2 * 148 * 32
-
-
-def linear(x, w) -> torch.Tensor:
-    """``F.linear(x, w)`` for a projection's weight; a few 16-bit rows go to a kernel of their own."""
-    if (0 < x.shape[0] <= FEW_ROWS and 0 < w.shape[0] <= FEW_COLUMNS and x.dim() == 2 and x.is_cuda and x.dtype == torch.bfloat16 == w.dtype
-            and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.stride(0) >= x.shape[1] and w.is_contiguous()
-            and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and x.device.index == torch.cuda.current_device()
-            and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))):
-        out = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
-        check(lib().tkv_few_gemm(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), w.shape[0], x.shape[0], w.shape[0], x.shape[1],
-                                 dtype_code(x.dtype), _stream(x)), "tkv_few_gemm")
-        _count(1)
-        return out
-    return F.linear(x, w)
-
 
 def greedy_next(logits, next_ids, ids, pos) -> bool:
     """``next_ids = ids = logits.argmax(-1, keepdim=True)``, ``pos += 1`` in one kernel; False (and nothing done) for logits it does
