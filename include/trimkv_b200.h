@@ -639,9 +639,6 @@ int tkv_latent_decode(const void* q_abs, int64_t qa_token, int64_t qa_head, cons
  * row of every expert.  counts [experts]: zeros on entry (may be NULL for at most 128 tokens).  top <= 64, experts <= 1024.
  * tkv_moe_gemm: out[r, :] = act(a[src ? src[r] : r, :] . w[e]^T), r in expert e's rows; w [experts, n, k]; act 0 none, 1 GELU
  * (erf); max_rows: host bound on the number of rows; a_rows: rows of a; experts here: those that own rows. */
-/* logits[t, e] = x[t, :] . w[e, :] in fp32 (bf16, width and x_stride multiples of 8, rows on 16-byte boundaries). */
-int tkv_moe_logits(const void* x, int64_t x_stride, const void* w, float* logits, int tokens, int experts, int width, int dtype,
-                   tkv_stream_t stream);
 int tkv_moe_route(const float* logits, int64_t logit_stride, const float* correction, int tokens, int experts, int identity, int top,
                   int groups, int keep, float scale, float* weight, int32_t* choice, int32_t* place, int32_t* src, int32_t* counts,
                   int32_t* offsets, tkv_stream_t stream);

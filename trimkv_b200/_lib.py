@@ -85,7 +85,6 @@ SIGNATURES = {
     "tkv_latent_prefill": (I, [P, L, P, L, P, P, L, P, P, F, P, I, I, I, I, I, I, I, I, I, I, P, P]),
     "tkv_latent_decode_workspace_bytes": (L, [I, I, I, I, I, I]),
     "tkv_latent_decode": (I, [P, L, L, P, L, L, P, P, I, P, P, F, P, L, L, P, L, I, I, I, I, I, I, P]),
-    "tkv_moe_logits": (I, [P, L, P, P, I, I, I, I, P]),
     "tkv_moe_route": (I, [P, L, P, I, I, I, I, I, I, F, P, P, P, P, P, P, P]),
     "tkv_moe_gemm": (I, [P, L, L, P, P, P, P, L, I, I, I, I, I, P, P]),
     "tkv_read_status": (I, [P, P]),

@@ -1,5 +1,4 @@
 // Routing of a mixture of experts, and the grouped product for every size and type:
-//   moe_logits_kernel: router logits of few tokens;
 //   moe_route_kernel : softmax scores, choice among the experts of the best groups, weights, and each choice's rank among the
 //                      choices of its expert; with one CTA (few tokens) also the places;
 //   moe_place_kernel : first row of every expert, row of every choice, token of every row;
@@ -25,34 +24,6 @@ struct MoeRoute {
   int32_t* counts;                                        // [experts], zero on entry (multi-CTA only)
   int32_t* offsets;                                       // [experts - identity + 1]
 };
-
-// logits[t, e] = x[t, :] . w[e, :] in fp32, for few tokens: a CTA per expert and eight tokens, a warp per token, every 16-byte piece
-// of four rounds requested before the first is used.  Latency bounds it: the rows come from L2 once the first token has read them.
-// A GEMM of 8 x 36 x 2048 is one nearly empty tile walking k alone: 24 us, here 5.6.
-constexpr int kLogitWarps = 8;
-__global__ void __launch_bounds__(kLogitWarps * 32) moe_logits_kernel(const __nv_bfloat16* x, int64_t x_stride, const __nv_bfloat16* w, float* logits,
-                                                                    int tokens, int experts, int width) {
-  constexpr int kAhead = 4;
-  const int lane = threadIdx.x & 31, t = blockIdx.y * kLogitWarps + (threadIdx.x >> 5), e = blockIdx.x;
-  grid_dependency_wait();
-  grid_launch_dependents();
-  if (t >= tokens) return;
-  const __nv_bfloat16 *xr = x + (int64_t)t * x_stride, *wr = w + (int64_t)e * width;
-  float sum[2] = {0.f, 0.f};
-  for (int c = lane * 8; c < width; c += kAhead * 256) {
-    float a[kAhead][8], b[kAhead][8];
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i)
-      if (c + i * 256 < width) { load_vec<8>(xr + c + i * 256, a[i]); load_vec<8>(wr + c + i * 256, b[i]); }
-#pragma unroll
-    for (int i = 0; i < kAhead; ++i)
-      if (c + i * 256 < width)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) sum[j & 1] = fmaf(a[i][j], b[i][j], sum[j & 1]);
-  }
-  const float z = warp_add(sum[0] + sum[1]);
-  if (lane == 0) logits[(int64_t)t * experts + e] = z;
-}
 
 // Exclusive sums of the counts of the experts that own rows, by one warp; off[n] = total.
 __device__ __forceinline__ void warp_offsets(const int32_t* counts, int n, int32_t* off) {
@@ -286,21 +257,6 @@ __global__ void __launch_bounds__(kAnyThreads) moe_any_kernel(GroupedGemm p) {
 }  // namespace tkv
 
 using namespace tkv;
-
-extern "C" int tkv_moe_logits(const void* x, int64_t x_stride, const void* w, float* logits, int tokens, int experts, int width, int dtype,
-                              tkv_stream_t stream) {
-  if (!x || !w || !logits) return fail(TKV_ERR_ARG, "tkv_moe_logits: NULL pointer argument");
-  if (tokens < 0 || experts <= 0 || width <= 0 || x_stride < width) return fail(TKV_ERR_ARG, "tkv_moe_logits: bad sizes experts=%d width=%d", experts, width);
-  if (dtype != TKV_BF16 || width % 8 || x_stride % 8 || !aligned16(x) || !aligned16(w))
-    return fail(TKV_ERR_UNSUPPORTED, "tkv_moe_logits: bf16 rows of whole 16-byte pieces only");
-  const int64_t blocks = ((int64_t)tokens + kLogitWarps - 1) / kLogitWarps;
-  if (blocks > 65535) return fail(TKV_ERR_UNSUPPORTED, "tkv_moe_logits: %d tokens", tokens);
-  if (tokens == 0) return TKV_OK;
-  cudaError_t e = launch_pdl(moe_logits_kernel, dim3(experts, (unsigned)blocks), dim3(kLogitWarps * 32), 0, (cudaStream_t)stream,
-                             (const __nv_bfloat16*)x, x_stride, (const __nv_bfloat16*)w, logits, tokens, experts, width);
-  if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_moe_logits: %s", cudaGetErrorString(e));
-  return check_launch("tkv_moe_logits");
-}
 
 extern "C" int tkv_moe_route(const float* logits, int64_t logit_stride, const float* correction, int tokens, int experts,
                              int identity, int top, int groups, int keep, float scale, float* weight, int32_t* choice,

@@ -99,7 +99,7 @@ class SparseMLP(FeedForward):
 
     def route(self, x):
         """Router logits in fp32, then ``(place, weight, src, offsets)``."""
-        z = F.linear(x, self.router) if x.dtype == torch.float32 else ops.moe_logits(x, self.router)
+        z = F.linear(x, self.router) if x.dtype == torch.float32 else torch.mm(x, self.router.t(), out_dtype=torch.float32)
         return ops.moe_route(z, as_f32(self, "correction"), self.identity, self.top, self.groups, self.keep, self.scale)
 
     def forward(self, x, status: Optional[torch.Tensor] = None):

@@ -748,24 +748,6 @@ def latent_decode(q_abs, q, rot_dim: int, freq, ring, batch, scale: float, out, 
 
 
 # ---- mixture of experts
-# Products of tokens and experts up to which the warp-per-logit kernel is the faster one.
-MOE_LOGITS_MOST = 8192
-
-
-def moe_logits(x, w) -> torch.Tensor:
-    """Router logits ``x @ w.T`` in fp32 of 16-bit rows."""
-    T, E = x.shape[0], w.shape[0]
-    if (x.dtype == torch.bfloat16 == w.dtype and 0 < T * E <= MOE_LOGITS_MOST and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
-            and x.stride(0) >= x.shape[1] and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0 and x.is_cuda
-            and x.device.index == torch.cuda.current_device() and not (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad))):
-        out = torch.empty(T, E, dtype=torch.float32, device=x.device)
-        check(lib().tkv_moe_logits(x.data_ptr(), x.stride(0), w.data_ptr(), out.data_ptr(), T, E, x.shape[1], dtype_code(x.dtype), _stream(x)),
-              "tkv_moe_logits")
-        _count(1)
-        return out
-    return torch.mm(x, w.t(), out_dtype=torch.float32)
-
-
 def moe_route(logits, correction, identity: int, top: int, groups: int, keep: int, scale: float):
     """``(place [T, top], weight [T, top], src [T * top], offsets)`` of fp32 router logits (see tkv_moe_route in the header)."""
     T, E = logits.shape
