@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(kLdThreads * HG, 2 / HG) latent_decode_kernel(
 // weight, then holds four columns and adds the chunks up, many rows requested before the first is used.  (With every thread
 // working out every weight for itself, a step of 8 requests against 4096 rows spent 15 us here on chains of dependent loads, now about 6.)
 __global__ void __launch_bounds__(kLpThreads) latent_merge_kernel(LatentDecode p, int nchunks) {
-  __shared__ float weight[kLpThreads], red[kLpThreads / 32];
+  __shared__ float weight[kLpThreads], part[kLpThreads], red[kLpThreads / 32];
   grid_dependency_wait();
   grid_launch_dependents();
   const int tid = threadIdx.x;
@@ -438,9 +438,10 @@ __global__ void __launch_bounds__(kLpThreads) latent_merge_kernel(LatentDecode p
     if (tid < n) {
       const float2 x = ml[(int64_t)(k0 + tid) * kLdHeads];
       weight[tid] = exp2_weight(x.x - top);
-      sum = fmaf(weight[tid], x.y, sum);
+      part[tid] = x.y;
     }
     __syncthreads();
+    for (int k = 0; k < n; ++k) sum = fmaf(weight[k], part[k], sum);   // by every thread, in the order of the chunks
     if (c < p.cpad) {
 #pragma unroll 8
       for (int k = 0; k < n; ++k) {
@@ -450,7 +451,6 @@ __global__ void __launch_bounds__(kLpThreads) latent_merge_kernel(LatentDecode p
       }
     }
   }
-  sum = block_add<kLpThreads>(sum, red);
   __nv_bfloat16* dst = (__nv_bfloat16*)p.out + (int64_t)b * p.out_token + (int64_t)h * p.out_head + c;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
