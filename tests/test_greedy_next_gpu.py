@@ -35,3 +35,17 @@ def test_logits_it_leaves_alone():
     for bad in (z.half(), z.double(), z[None], z.t()[:, :2], z[:0], z.cpu()):
         assert not ops.greedy_next(bad, nxt, nxt, pos)
     assert not ops.greedy_next(z, nxt.int(), nxt, pos) and pos.item() == 0
+
+
+@pytest.mark.gpu
+def test_buffers_of_another_size_are_left_alone():
+    """The kernel writes an id per row and one position: fewer or more are for the general path, which raises or broadcasts."""
+    z = torch.zeros(3, 64, device=DEV)
+
+    def ints(*shape):
+        return torch.full(shape, 9, dtype=torch.int64, device=DEV)
+    for sizes in ((2, 3, 1), (3, 2, 1), (4, 3, 1), (3, 4, 1), (0, 3, 1), (3, 3, 2), (3, 3, 0)):
+        held = [ints(n) for n in sizes]
+        assert not ops.greedy_next(z, *held) and all(bool((t == 9).all()) for t in held)
+    held = ints(3, 1), ints(3), ints()
+    assert ops.greedy_next(z, *held) and held[0].flatten().tolist() == held[1].tolist() == [0, 0, 0] and held[2].item() == 10

@@ -467,7 +467,8 @@ def greedy_next(logits, next_ids, ids, pos) -> bool:
     not read."""
     if (logits.dim() != 2 or logits.dtype not in (torch.bfloat16, torch.float32) or not logits.is_cuda or logits.stride(1) != 1
             or logits.stride(0) < logits.shape[1] or logits.shape[0] == 0 or logits.device.index != torch.cuda.current_device()
-            or not all(t.dtype == torch.int64 and t.is_contiguous() and t.device == logits.device for t in (next_ids, ids, pos))):
+            or not all(t.dtype == torch.int64 and t.is_contiguous() and t.device == logits.device for t in (next_ids, ids, pos))
+            or not next_ids.numel() == ids.numel() == logits.shape[0] or pos.numel() != 1):
         return False
     check(lib().tkv_greedy_next(logits.data_ptr(), logits.stride(0), logits.shape[0], logits.shape[1], dtype_code(logits.dtype),
                                 next_ids.data_ptr(), ids.data_ptr(), pos.data_ptr(), _stream(logits)), "tkv_greedy_next")
