@@ -56,3 +56,34 @@ def test_refused_while_capturing():
         with pytest.raises(RuntimeError, match="captured"):
             ops.ints_on(dev, [1])
     graph.reset()
+
+
+def test_takes_what_a_tensor_takes():
+    """``want`` of a packed forward pass may hold whatever an int32 tensor is made of; beyond 32 bits is an error, not another row."""
+    np = pytest.importorskip("numpy")
+    cpu = torch.device("cpu")
+    assert ops.ints_on(cpu, [torch.tensor(5), np.int64(7), True, 2.0]).tolist() == [5, 7, 1, 2]
+    t = torch.zeros(4, dtype=torch.int32)
+    for far in (2 ** 31, -2 ** 31 - 1, 2 ** 32 + 1):
+        with pytest.raises(RuntimeError, match="overflow"):
+            ops.ints_on(cpu, [0, far])
+        with pytest.raises(RuntimeError, match="overflow"):
+            ops.set_ints(t, [1], far)
+        with pytest.raises(IndexError):
+            ops.set_ints(t, [far], 0)
+    with pytest.raises(IndexError):
+        ops.set_ints(t, [4], 0)
+    with torch.device("meta"):                   # a default device of another kind changes nothing
+        assert ops.ints_on(cpu, [1]).device == cpu
+
+
+@pytest.mark.gpu
+def test_takes_what_a_tensor_takes_on_the_gpu():
+    np = pytest.importorskip("numpy")
+    dev = torch.device("cuda", 0)
+    mixed = [torch.tensor(5), torch.tensor(6, device=dev), np.int64(7), True, 2.0]
+    assert ops.ints_on(dev, mixed).tolist() == [5, 6, 7, 1, 2]
+    with pytest.raises(RuntimeError, match="overflow"):
+        ops.ints_on(dev, [2 ** 32 + 1])
+    with pytest.raises(RuntimeError, match="overflow"):
+        ops.set_ints(torch.zeros(4, dtype=torch.int32, device=dev), [1], 2 ** 32 + 1)

@@ -5,7 +5,6 @@ CUDA kernels of libtrimkv_b200.so.
 """
 from __future__ import annotations
 
-import ctypes
 from typing import Optional
 
 import torch
@@ -476,33 +475,41 @@ def greedy_next(logits, next_ids, ids, pos) -> bool:
     return True
 
 
+def _host_ints(values) -> torch.Tensor:
+    """Integers as an int32 host tensor: what ``torch.tensor`` takes as such is taken, what it refuses (beyond 32 bits) is refused."""
+    return torch.tensor(values, dtype=torch.int32, device="cpu")
+
+
 def ints_on(device, values) -> torch.Tensor:
     """A few host integers as an int32 tensor on ``device``: launch arguments of a small kernel instead of a copy, so that the
     host neither stages nor waits."""
-    n = len(values)
+    host = _host_ints(values)
     if device.type != "cuda":
-        return torch.tensor(values, dtype=torch.int32)
-    if torch.cuda.is_current_stream_capturing():
-        raise RuntimeError("host integers would be baked into the CUDA graph being captured")
-    out = torch.empty(n, dtype=torch.int32, device=device)
-    with torch.cuda.device_of(out):
-        check(lib().tkv_put_ints(out.data_ptr(), (ctypes.c_int32 * n)(*values), n, _stream(out)), "tkv_put_ints")
-    _count(-(-n // 960))
+        return host.to(device)
+    with torch.cuda.device(device):
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("host integers would be baked into the CUDA graph being captured")
+        out = torch.empty(host.shape, dtype=torch.int32, device=device)
+        check(lib().tkv_put_ints(out.data_ptr(), host.data_ptr(), host.numel(), _stream(out)), "tkv_put_ints")
+    _count(-(-host.numel() // 960))
     return out
 
 
 def set_ints(dst: torch.Tensor, index, value: int) -> None:
     """``dst[index] = value`` (int32) for a list of host integers, without a copy."""
-    n = len(index)
-    if not dst.is_cuda:
-        dst[list(index)] = value
-        return
-    if n and not 0 <= min(index) <= max(index) < dst.numel():
+    if len(index) and not 0 <= min(index) <= max(index) < dst.numel():
         raise IndexError(f"index outside {dst.numel()} entries")
-    if torch.cuda.is_current_stream_capturing():
-        raise RuntimeError("host integers would be baked into the CUDA graph being captured")
+    if not -2 ** 31 <= value < 2 ** 31:
+        raise RuntimeError(f"overflow: {value} is not a 32-bit integer")
+    host = _host_ints(index)
+    n = host.numel()
+    if not dst.is_cuda:
+        dst[host.long()] = value
+        return
     with torch.cuda.device_of(dst):
-        check(lib().tkv_set_ints(dst.data_ptr(), (ctypes.c_int32 * n)(*index), n, value, _stream(dst)), "tkv_set_ints")
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("host integers would be baked into the CUDA graph being captured")
+        check(lib().tkv_set_ints(dst.data_ptr(), host.data_ptr(), n, value, _stream(dst)), "tkv_set_ints")
     _count(-(-n // 960))
 
 
