@@ -128,7 +128,9 @@ def rows_as_held(beta, pos, nseg: int, n: int):
     ``[nseg, n]``, positions that all segments share as ``[n]``; None for types those do not read."""
     if beta.dtype not in _DTYPE or pos.dtype not in _POS_BITS:
         return None
-    shared = all(size == 1 or step == 0 for size, step in zip(pos.shape[:2], pos.stride()[:2])) and pos.shape[2:] == (n,)
+    # Anything but one entry per segment and token goes on to the reshape, which refuses it.
+    shared = (pos.dim() == 3 and pos.shape[0] * pos.shape[1] == nseg and pos.shape[2] == n and nseg > 0
+              and all(size == 1 or step == 0 for size, step in zip(pos.shape[:2], pos.stride()[:2])))
     return beta.reshape(nseg, n).contiguous(), (pos[0, 0] if shared else pos.reshape(nseg, n)).contiguous()
 
 
