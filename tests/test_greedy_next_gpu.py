@@ -49,3 +49,14 @@ def test_buffers_of_another_size_are_left_alone():
         assert not ops.greedy_next(z, *held) and all(bool((t == 9).all()) for t in held)
     held = ints(3, 1), ints(3), ints()
     assert ops.greedy_next(z, *held) and held[0].flatten().tolist() == held[1].tolist() == [0, 0, 0] and held[2].item() == 10
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,vocab,taken", [(1, 151936, True), (1, 154000, True), (1, 154001, False), (8, 256000, False), (32, 256000, True)])
+def test_large_vocabularies_of_few_rows_are_left_alone(rows, vocab, taken):
+    z = torch.randn(rows, vocab, generator=torch.Generator(device=DEV).manual_seed(rows), device=DEV).bfloat16()
+    nxt, ids, pos = (torch.zeros(*shape, dtype=torch.int64, device=DEV) for shape in ((rows, 1), (rows, 1), (1,)))
+    assert ops.greedy_next(z, nxt, ids, pos) == taken
+    if taken:
+        want = z.float().cpu().argmax(-1, keepdim=True)
+        assert torch.equal(nxt.cpu(), want) and torch.equal(ids.cpu(), want) and pos.item() == 1

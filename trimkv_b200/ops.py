@@ -465,11 +465,14 @@ update_flatten_view_triton = update_flatten_view  # the reference's name for the
 
 def greedy_next(logits, next_ids, ids, pos) -> bool:
     """``next_ids = ids = logits.argmax(-1, keepdim=True)``, ``pos += 1`` in one kernel; False (and nothing done) for logits it does
-    not read."""
+    not read, and for few rows of a vocabulary so large that one CTA per row takes longer than a reduction of a row by many and its
+    three launches more.  us by (rows, vocabulary), kernel and reduction: (1, 151936) 14.9, 15.9; (1, 200064) 18.7, 15.4; (8, 256000)
+    23.1, 17.1; (32, 256000) 23.3, 25.6; (32, 400000) 34.9, 30.0; (64, 400000) 38.0, 48.1."""
     if (logits.dim() != 2 or logits.dtype not in (torch.bfloat16, torch.float32) or not logits.is_cuda or logits.stride(1) != 1
             or logits.stride(0) < logits.shape[1] or logits.shape[0] == 0 or logits.device.index != torch.cuda.current_device()
             or not all(t.dtype == torch.int64 and t.is_contiguous() and t.device == logits.device for t in (next_ids, ids, pos))
-            or not next_ids.numel() == ids.numel() == logits.shape[0] or pos.numel() != 1):
+            or not next_ids.numel() == ids.numel() == logits.shape[0] or pos.numel() != 1
+            or logits.shape[1] > 150_000 + 4_000 * logits.shape[0]):
         return False
     check(lib().tkv_greedy_next(logits.data_ptr(), logits.stride(0), logits.shape[0], logits.shape[1], dtype_code(logits.dtype),
                                 next_ids.data_ptr(), ids.data_ptr(), pos.data_ptr(), _stream(logits)), "tkv_greedy_next")
