@@ -64,7 +64,8 @@ template <typename T, int V> struct RawVec {
   uint4 w[kWords];
   __device__ __forceinline__ void load(const T* p) {
 #pragma unroll
-    for (int i = 0; i < kWords; ++i) w[i] = ld16_stream(reinterpret_cast<const char*>(p) + 16 * i);
+    for (int i = 0; i < kWords; ++i)                       // the words of an fp32 vector share a sector: L1 holds it for the second
+      w[i] = kWords == 1 ? ld16_stream(p) : ld16(reinterpret_cast<const char*>(p) + 16 * i);
   }
   __device__ __forceinline__ void floats(float* v) const {
 #pragma unroll

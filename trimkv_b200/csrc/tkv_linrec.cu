@@ -63,9 +63,11 @@ __global__ void __launch_bounds__(kRotThreads) rotate_qk_kernel(const T* proj, i
 
 constexpr int kConvThreads = 128, kConvStrip = 32, kConvAhead = 8;
 
-// grid: (channel blocks, strips of kConvStrip tokens, requests).  kTaps = 0: any number of taps, inputs re-read per tap.
+// grid: (channel blocks, strips of kConvStrip tokens, requests).  kTaps = 0: any number of taps, inputs re-read per tap.  Four CTAs per
+// SM where rows requested ahead fill the registers of 16-bit vectors; the other forms are left to the compiler (with the same bound
+// the form for any number of taps took 72 registers instead of 64: 1500 tokens, 3 taps, 35.2 -> 38.8 us).
 template <typename T, int V, int kTaps>
-__global__ void __launch_bounds__(kConvThreads, sizeof(T) == 2 ? 4 : 1) conv_silu_kernel(const T* proj, int64_t row_stride, const T* ring, const float* w,
+__global__ void __launch_bounds__(kConvThreads, sizeof(T) == 2 && V > 1 && kTaps > 0 ? 4 : 0) conv_silu_kernel(const T* proj, int64_t row_stride, const T* ring, const float* w,
                                                                 const float* bias, T* out, const int32_t* cu, const int32_t* slots,
                                                                 const int32_t* pos0, int channels, int taps_rt) {
   const int taps = kTaps > 0 ? kTaps : taps_rt;
@@ -97,7 +99,8 @@ __global__ void __launch_bounds__(kConvThreads, sizeof(T) == 2 ? 4 : 1) conv_sil
 #pragma unroll
     for (int k = 1; k < kT; ++k) input(i0 - k, win[k - 1]);
     // Latency would bound a token after the other: kConvAhead rows are requested at a time.  6827 tokens of 6144 channels: 48 us
-    // one at a time, 40 us so.
+    // one at a time, 40 us so.  In fp32, with the copy into the ring, 118 and 110 us (163 registers; 144 us when the two words of a vector
+    // both went past L1).
     for (int ib = i0; ib < i1; ib += kConvAhead) {
       RawVec<T, V> ahead[kConvAhead];
 #pragma unroll
