@@ -345,71 +345,64 @@ __global__ void __launch_bounds__(kRowThreads) gated_norm_kernel(const T* y, int
   }
 }
 
-// The same for groups of up to two 16-byte-aligned vectors per lane, kLanes lanes per group, kItems groups per lane in turn.  Memory
-// bounds it: every vector of all its groups is requested, as it is, before the first is used, and the rows are found by 32-bit
-// divisions.  32768 rows of 16 groups of 128: 107 us with one group at a time, held as fp32 behind a 64-bit division; now 76 us,
-// 5.3 TB/s.
+// The same for groups of up to two 16-byte-aligned vectors per lane, kLanes lanes per group.  Memory bounds it: both vectors of y and z
+// are requested, as they are, before the first is used, and the row is found by a 32-bit division.  32768 rows of 16 groups of 128 with
+// a gate: 117 us behind a 64-bit division and loads that leave y and z in L1, 80 us so, 5.0 TB/s; 84 us with two groups per lane in
+// turn, which a small call only waits for (32 rows: 2.5, 2.3 and 3.3 us; without a gate 2.2, 2.1 and 2.8 us).
 template <typename T, int kLanes>
 __global__ void __launch_bounds__(kRowThreads) gated_norm_vec_kernel(const T* y, int64_t y_stride, const T* z, int64_t z_stride,
                                                                     const float* w, int w_shared, T* out, int rows, int groups,
                                                                     int len, float eps, int gate_first) {
-  constexpr int kKeep = 2, kItems = sizeof(T) == 2 ? 2 : 1, kPer = kRowThreads / kLanes;
+  constexpr int kKeep = 2;
   const int lane = threadIdx.x & (kLanes - 1);
   const uint32_t items = (uint32_t)rows * (uint32_t)groups;          // below 2^31 (checked on the host)
-  const uint32_t item0 = blockIdx.x * (kPer * kItems) + threadIdx.x / kLanes;
+  const uint32_t item_rt = blockIdx.x * (kRowThreads / kLanes) + threadIdx.x / kLanes;
+  const uint32_t item = min(item_rt, items - 1), row = item / (uint32_t)groups;   // a warp's spare lanes take part in its shuffles
+  const uint32_t grp = item - row * groups;
   const int nvec = len / 8;
   const bool has_gate = z != nullptr;
   grid_dependency_wait();
   grid_launch_dependents();
-  RawVec<T, 8> a[kItems][kKeep], g[kItems][kKeep];
-  uint32_t grp[kItems];
+  RawVec<T, 8> a[kKeep], g[kKeep];
 #pragma unroll
-  for (int k = 0; k < kItems; ++k) {
-    const uint32_t item = min(item0 + k * kPer, items - 1), row = item / (uint32_t)groups;   // a warp's spare lanes take part in its shuffles
-    grp[k] = item - row * groups;
+  for (int j = 0; j < kKeep; ++j)
+    if (lane + kLanes * j < nvec) {
+      const int64_t c = (int64_t)grp * len + (lane + kLanes * j) * 8;
+      a[j].load(y + row * y_stride + c);
+      if (has_gate) g[j].load(z + row * z_stride + c);
+    }
+  float av[kKeep][8], gv[kKeep][8], ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < kKeep; ++j)
-      if (lane + kLanes * j < nvec) {
-        const int64_t c = (int64_t)grp[k] * len + (lane + kLanes * j) * 8;
-        a[k][j].load(y + row * y_stride + c);
-        if (has_gate) g[k][j].load(z + row * z_stride + c);
+  for (int j = 0; j < kKeep; ++j)
+    if (lane + kLanes * j < nvec) {
+      a[j].floats(av[j]);
+      if (has_gate) g[j].floats(gv[j]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        gv[j][e] = has_gate ? silu_act<T>(gv[j][e]) : 1.0f;
+        if (gate_first) av[j][e] *= gv[j][e];
+        ss += av[j][e] * av[j][e];
       }
-  }
+    }
 #pragma unroll
-  for (int k = 0; k < kItems; ++k) {
-    float av[kKeep][8], gv[kKeep][8], ss = 0.f;
+  for (int d = kLanes / 2; d >= 1; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+  const float rstd = 1.0f / sqrtf(ss / (float)len + eps);
+  if (item_rt >= items) return;
+  T* o = out + (int64_t)item * len;
 #pragma unroll
-    for (int j = 0; j < kKeep; ++j)
-      if (lane + kLanes * j < nvec) {
-        a[k][j].floats(av[j]);
-        if (has_gate) g[k][j].floats(gv[j]);
+  for (int j = 0; j < kKeep; ++j)
+    if (lane + kLanes * j < nvec) {
+      const int c = (lane + kLanes * j) * 8;
+      float wv[8];
+      if (w != nullptr) load_vec<8>(w + (w_shared ? 0 : (int64_t)grp * len) + c, wv);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          gv[j][e] = has_gate ? silu_act<T>(gv[j][e]) : 1.0f;
-          if (gate_first) av[j][e] *= gv[j][e];
-          ss += av[j][e] * av[j][e];
-        }
+      for (int e = 0; e < 8; ++e) {
+        av[j][e] *= rstd;
+        if (w != nullptr) av[j][e] *= wv[e];
+        if (!gate_first) av[j][e] *= gv[j][e];
       }
-#pragma unroll
-    for (int d = kLanes / 2; d >= 1; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-    const float rstd = 1.0f / sqrtf(ss / (float)len + eps);
-    if (item0 + k * kPer >= items) continue;
-    T* o = out + (int64_t)(item0 + k * kPer) * len;
-#pragma unroll
-    for (int j = 0; j < kKeep; ++j)
-      if (lane + kLanes * j < nvec) {
-        const int c = (lane + kLanes * j) * 8;
-        float wv[8];
-        if (w != nullptr) load_vec<8>(w + (w_shared ? 0 : (int64_t)grp[k] * len) + c, wv);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          av[j][e] *= rstd;
-          if (w != nullptr) av[j][e] *= wv[e];
-          if (!gate_first) av[j][e] *= gv[j][e];
-        }
-        store_vec<8>(o + c, av[j]);
-      }
-  }
+      store_vec<8>(o + c, av[j]);
+    }
 }
 
 template <typename T, int V>
@@ -641,7 +634,7 @@ extern "C" int tkv_gated_norm(const void* y, int64_t y_stride, const void* z, in
   // two vectors per lane: 8, 16 or 32 lanes; longer groups, other alignments and numbers of groups beyond 32 bits: a warp, in turn
   const bool kept = vec && group_len <= 512 && (int64_t)rows * groups <= INT32_MAX;
   const int lanes = !kept || group_len > 256 ? 32 : group_len > 128 ? 16 : 8;
-  const int64_t per = kRowThreads / lanes * (kept && dtype == TKV_BF16 ? 2 : 1), grid = ((int64_t)rows * groups + per - 1) / per;
+  const int64_t per = kRowThreads / lanes, grid = ((int64_t)rows * groups + per - 1) / per;
   int rc = rows_grid("tkv_gated_norm", grid);
   if (rc != TKV_OK) return rc;
   TKV_WITH_TYPE(dtype, T, {
