@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from trimkv_b200 import ops
+from trimkv_b200 import _lib, ops
 
 DEV = "cuda"
 
@@ -24,14 +24,15 @@ def _reference(q, k, v, lens, hkv, scale):
 
 
 # rows of a segment = q_tokens * hq / hkv: one tile, its edge, one row into the second, both, one row into the next CTA; segments
-# that end at, before and behind the edge of a key tile, and (40 of 130 tokens) ones of which the first rows see nothing.  Alone the
+# that end at, before and behind the edge of a key tile, and (40 of 130 tokens) ones of which the first rows see nothing.  Of 257 rows
+# the last CTA's second tile has none, of 400 rows against 200 keys a CTA's first tile sees nothing and its second does.  Alone the
 # segments are few: one tile per CTA; `copies` times over they are many: two.
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("hq,hkv,ql,lens,copies", [
     (1, 1, 1, (1, 128, 129), 1), (2, 2, 128, (128, 256, 383, 200), 1), (3, 1, 43, (300, 43), 40), (2, 1, 128, (128, 129, 640), 27),
-    (1, 1, 257, (257, 258, 512), 25), (1, 1, 130, (40, 130, 131), 27), (4, 2, 64, (64, 127, 500, 65), 1), (4, 2, 65, (65, 127, 500, 66), 20),
-    (3, 3, 385, (385, 512, 700), 14),
+    (1, 1, 257, (257, 258, 512), 24), (1, 1, 130, (40, 130, 131), 27), (4, 2, 64, (64, 127, 500, 65), 1), (4, 2, 65, (65, 127, 500, 66), 20),
+    (3, 3, 385, (385, 512, 700), 14), (1, 1, 400, (200, 400), 37), (1, 1, 300, (20, 170, 172), 24),
 ])
 def test_tile_edges(dtype, hq, hkv, ql, lens, copies):
     g = torch.Generator(device=DEV).manual_seed(hq + 10 * ql)
@@ -48,6 +49,7 @@ def test_tile_edges(dtype, hq, hkv, ql, lens, copies):
     unit = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
     outs = []
     for times in sorted({1, copies}):
+        assert _lib.lib().tkv_prefill_attn_rows_per_cta(len(lens) * times, ql * hq // hkv) == (128 if times == 1 else 256)
         out = torch.full((b * times, ql, hq, d), float("nan"), dtype=dtype, device=DEV)
         status = ops.new_status(DEV)
         ops.prefill_attn(q.repeat(times, 1, 1, 1), k.repeat(times, 1, 1), v.repeat(times, 1, 1),
@@ -73,6 +75,7 @@ def test_two_part_keys(n, copies, window, dim, vdim):
     lin = torch.randn(n, rank + rot, generator=g, device=DEV).bfloat16()
     outs = []
     for times in (1, copies):
+        assert _lib.lib().tkv_latent_prefill_rows_per_cta(times, heads, n * times, n) == (128 if times == 1 else 256)
         cache = cache_of(LatentState(rank + rot, window), dtype=torch.bfloat16)
         cache.open(times)
         b = cache.begin([n] * times)

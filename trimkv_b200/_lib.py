@@ -82,6 +82,8 @@ SIGNATURES = {
     "tkv_chanrec_chunk": (I, [P, P, P, L, P, P, P, P, P, P, P, P, L, I, I, I, I, I, I, P, P]),
     "tkv_rotate_pairs": (I, [P, L, P, P, I, I, I, I, I, I, P, I, P]),
     "tkv_latent_prep": (I, [P, L, P, P, F, I, I, I, I, P, P, P, I, P, P, P, P, P, I, I, I, I, I, P]),
+    "tkv_prefill_attn_rows_per_cta": (I, [I, L]),
+    "tkv_latent_prefill_rows_per_cta": (I, [I, I, I, I]),
     "tkv_latent_prefill": (I, [P, L, P, L, P, P, L, P, P, F, P, I, I, I, I, I, I, I, I, I, I, P, P]),
     "tkv_latent_decode_workspace_bytes": (L, [I, I, I, I, I, I]),
     "tkv_latent_decode": (I, [P, L, L, P, L, L, P, P, I, P, P, F, P, L, L, P, L, I, I, I, I, I, I, P]),

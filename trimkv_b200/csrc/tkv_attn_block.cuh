@@ -1,5 +1,5 @@
-// Shared by the query-resident attention kernels on tcgen05 whose blocks are 128 query rows against tiles of 128 keys: two
-// softmax threads per row (eight warps) and one warp that issues copies and products.
+// Shared by the query-resident attention kernels on tcgen05 whose tiles are 128 query rows against 128 keys: eight softmax warps, two
+// threads per row of one tile or one per row of two tiles, and a warp (kDaThreads) or two that issue copies and products.
 #pragma once
 #include "tkv_tc.cuh"
 
@@ -10,9 +10,6 @@ constexpr int kDaTile = 128, kDaHalf = 16384;             // 128 rows x 64 eleme
 constexpr int kDaTmemCols = 512;
 constexpr float kDaRescaleGap = 8.0f;
 
-__device__ __forceinline__ uint32_t da_idesc(int n, int b_mn_major) {   // kind::f16, bf16 operands, fp32 D, M = 128
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)b_mn_major << 16) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
-}
 __device__ __forceinline__ uint32_t da_swz(int r, int c) {              // 16-byte chunk c of row r, 64-element halves
   return (uint32_t)((c >> 3) * kDaHalf + r * 128 + (((c & 7) ^ (r & 7)) << 4));
 }

@@ -463,16 +463,23 @@ static int launch_prefill(K kernel, int threads, int bytes, bool* configured, co
   if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_prefill_attn: %s", cudaGetErrorString(e));
   return check_launch("tkv_prefill_attn");
 }
+static bool prefill_in_pairs(int nseg, int64_t rows) {
+  return pair_is_faster(nseg * ((rows + kPfTile - 1) / kPfTile), nseg * ((rows + kPfRows - 1) / kPfRows));
+}
 template <int kDtype>
 static int launch_prefill(const CUtensorMap& mk, const CUtensorMap& mv, const AttnParams& p, int nseg, cudaStream_t st) {
   static bool one_configured = false, pair_configured = false;
   const int64_t tiles = ((int64_t)p.rows + kPfTile - 1) / kPfTile, pairs = ((int64_t)p.rows + kPfRows - 1) / kPfRows;
-  if (pair_is_faster(nseg * tiles, nseg * pairs))
+  if (prefill_in_pairs(nseg, p.rows))
     return launch_prefill(prefill_attn_kernel<kDtype>, kPairThreads, PfShape::kBytes, &pair_configured, mk, mv, p, nseg, (int)pairs, st);
   return launch_prefill(prefill_attn_one_kernel<kDtype>, kDaThreads, kPfOneBytes, &one_configured, mk, mv, p, nseg, (int)tiles, st);
 }
 
 }  // namespace tkv
+
+extern "C" int tkv_prefill_attn_rows_per_cta(int nseg, int64_t rows) {
+  return tkv::prefill_in_pairs(nseg, rows) ? tkv::kPfRows : tkv::kPfTile;
+}
 
 extern "C" int tkv_prefill_attn(const void* q, int64_t q_sb, int64_t q_st, int64_t q_sh,
                                 const void* k_cache, const void* v_cache, const int32_t* seg_len, int64_t cap,

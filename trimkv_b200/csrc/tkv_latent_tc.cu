@@ -225,7 +225,7 @@ two_part_one_kernel(const __grid_constant__ CUtensorMap map_k1, const __grid_con
 
   if (is_ctrl) {
     if (tid == kDaSoftmaxThreads) {
-      const uint32_t idesc_s = da_idesc(128, 0), idesc_pv = da_idesc(VH * 64, 1);
+      const uint32_t idesc_s = pair_idesc<true>(128, 0), idesc_pv = pair_idesc<true>(VH * 64, 1);
       const uint32_t p_addr = smem_u32(p_s), q_addr = smem_u32(q_s), v_addr = smem_u32(v_s);
       auto issue_s = [&](int s) -> bool {
         if (!mbar_wait_or_abort(&sm->bar_k[s & 1], (s >> 1) & 1, abort_flag)) return false;
@@ -422,6 +422,13 @@ bool two_part_tc_shape(const TwoPartAttn& p, int dtype) {
   return aligned16(p.q1) && aligned16(p.q2) && aligned16(p.k1) && aligned16(p.k2) && aligned16(p.v) && aligned16(p.out);
 }
 
+// Counts the tiles and pairs that have rows at most: prompts shorter than the longest leave blocks without any.
+static bool two_part_in_pairs(int batch, int heads, int tokens, int max_tokens) {
+  const int64_t tiles = ((int64_t)max_tokens + kDaTile - 1) / kDaTile, pairs = ((int64_t)max_tokens + kTpRows - 1) / kTpRows;
+  const int64_t held = ((int64_t)tokens + kDaTile - 1) / kDaTile + batch - 1, held_pairs = held / 2 + batch;
+  return pair_is_faster(heads * (held < batch * tiles ? held : batch * tiles), heads * (held_pairs < batch * pairs ? held_pairs : batch * pairs));
+}
+
 template <typename K>
 static int launch_tp(K kernel, int threads, int bytes, bool* configured, const CUtensorMap& m1, const CUtensorMap& m2, const CUtensorMap& mv,
                      const TwoPartAttn& p, int64_t grid, int nblocks, cudaStream_t st) {
@@ -439,9 +446,8 @@ static int launch_tp(const CUtensorMap& m1, const CUtensorMap& m2, const CUtenso
   static bool one_configured = false, pair_configured = false;
   static_assert(tp_smem_bytes<K1 + 1, VH>() <= 232448, "shared memory of the kernel");
   const int64_t tiles = ((int64_t)max_tokens + kDaTile - 1) / kDaTile, pairs = ((int64_t)max_tokens + kTpRows - 1) / kTpRows;
-  const int64_t each = (int64_t)p.batch * p.heads, held = ((int64_t)p.tokens + kDaTile - 1) / kDaTile + p.batch - 1;
-  // tiles and pairs that have rows at most: prompts shorter than the longest leave blocks without any
-  if (pair_is_faster(p.heads * (held < p.batch * tiles ? held : p.batch * tiles), p.heads * (held / 2 + p.batch < p.batch * pairs ? held / 2 + p.batch : p.batch * pairs)))
+  const int64_t each = (int64_t)p.batch * p.heads;
+  if (two_part_in_pairs(p.batch, p.heads, p.tokens, max_tokens))
     return launch_tp(two_part_prefill_kernel<K1, 1, VH>, kPairThreads, PairShape<K1 + 1, VH, false>::kBytes, &pair_configured, m1, m2, mv, p, each * pairs,
                      (int)pairs, st);
   return launch_tp(two_part_one_kernel<K1, 1, VH>, kDaThreads, tp_smem_bytes<K1 + 1, VH>(), &one_configured, m1, m2, mv, p, each * tiles, (int)tiles, st);
@@ -461,3 +467,7 @@ int launch_two_part_tc(const TwoPartAttn& p, int64_t kv_rows, int max_tokens, cu
 }
 
 }  // namespace tkv
+
+extern "C" int tkv_latent_prefill_rows_per_cta(int batch, int heads, int tokens, int max_tokens) {
+  return tkv::two_part_in_pairs(batch, heads, tokens, max_tokens) ? tkv::kTpRows : tkv::kDaTile;
+}
