@@ -59,3 +59,14 @@ def test_prompts_in_the_callers_types(beta_type, pos_type, shared, n, transposed
     assert torch.equal(cache.retention_weights[0], beta.float().gather(2, keep))
     assert torch.equal(cache.key_cache[0], k.gather(2, keep[..., None].expand(-1, -1, -1, d)))
     assert torch.equal(cache.value_cache[0], v.gather(2, keep[..., None].expand(-1, -1, -1, d)))
+
+
+# on both sides of the lengths where the width changes, in place and in the selection; kept rows that outweigh the keys and that do not
+@pytest.mark.gpu
+@pytest.mark.parametrize("nseg,n,m", [
+    (148, 256, 200), (148, 257, 200), (148, 1024, 900), (148, 1025, 900), (148, 2047, 1500), (148, 2048, 2000), (2, 8191, 4096), (2, 8192, 4096),
+    (149, 256, 99), (149, 257, 256), (193, 512, 500), (193, 513, 512), (149, 1024, 1000), (192, 1025, 1024), (193, 1025, 1024), (193, 1025, 300), (296, 1535, 700), (296, 1536, 700),
+    (297, 1536, 700), (3, 14337, 5000),
+])
+def test_widths_agree_where_the_length_decides(nseg, n, m):
+    test_widths_agree(nseg, n, m)

@@ -626,13 +626,28 @@ static int set_smem(K kernel, size_t bytes, const char* what) {
 }
 
 // Threads of a segment's CTA.  A segment is one CTA's, and its time is the latency of rounds over its keys (four selection passes
-// and the list) and of tiles of rows (load, barrier, store): the fewer threads, the more rounds and tiles.  So few segments get wide
-// CTAs, down to where the SMs' 1024 threads are shared by several of them; long segments, whose key array leaves room for at most
-// 3 CTAs per SM, get at least 512.  A piece of 512 tokens of 8 requests x 8 heads against 4096 rows (attention, append and this):
-// 315 us with 256 threads per segment, 279 us with 1024.
-template <typename F> static int with_evict_threads(int nseg, size_t smem, F launch) {
-  if (nseg <= 148) return launch(std::integral_constant<int, kEvictThreadsPlan>());
-  if (nseg <= 2 * 148 || smem > 56 * 1024) return launch(std::integral_constant<int, kEvictThreadsWide>());
+// and the list) and of tiles of rows (load, barrier, store): the fewer threads, the more rounds and tiles; the more threads, the dearer
+// each of the barriers, and the fewer CTAs on an SM.  So few segments get wide CTAs, short ones narrow CTAs, and beyond two CTAs of
+// 512 per SM only segments whose key array leaves room for at most 3 CTAs get 512.  us with 256, 512 and 1024 threads:
+//   in place, 64 segments of     144 -> 128 rows   9.0   9.9  13.1      16 of  640 ->  512  17.6  17.1  17.1
+//                               1152 -> 1024      35.9  28.7  30.0            4608 -> 4096 109.7  84.8  78.2
+//   in place, 224 segments of    640 -> 512       30.9  32.2  40.1            1536 -> 1024  57.4  55.8  65.4
+//                               4608 -> 4096     197.0 205.2 192.5            2048 ->  256  34.0  29.0  38.5
+//   selection, 64 segments of    640 -> 512        8.5   9.4   9.9            4224 -> 4096  25.8  24.6  26.1    8192 -> 1024  43.0  39.4  35.7
+//   selection, 224 segments of  1152 -> 1024      15.0  16.2  22.2            4608 -> 4096  42.5  38.9  44.9
+// `moved`: bytes of K of a segment's kept rows; where they outweigh the keys, memory and not latency bounds 193 segments and more.
+enum class EvictWork { kInPlace, kSelect };
+template <typename F> static int with_evict_threads(EvictWork work, int nseg, int n, int64_t moved, F launch) {
+  int threads = n > 14336 ? kEvictThreadsWide : kEvictThreads;
+  if (work == EvictWork::kInPlace) {
+    if (nseg <= 148) threads = n >= 2048 ? kEvictThreadsPlan : n > 256 ? kEvictThreadsWide : kEvictThreads;
+    else if (nseg <= 2 * 148 && n > 256 && !(n > 512 && moved > 200 * (int64_t)n && (nseg > 192 || n <= 1024))) threads = kEvictThreadsWide;
+  } else {
+    if (nseg <= 148) threads = n >= 8192 ? kEvictThreadsPlan : n > 1024 ? kEvictThreadsWide : kEvictThreads;
+    else if (nseg <= 2 * 148 && n >= 1536) threads = kEvictThreadsWide;
+  }
+  if (threads == kEvictThreadsPlan) return launch(std::integral_constant<int, kEvictThreadsPlan>());
+  if (threads == kEvictThreadsWide) return launch(std::integral_constant<int, kEvictThreadsWide>());
   return launch(std::integral_constant<int, kEvictThreads>());
 }
 
@@ -711,7 +726,8 @@ static int evict_impl(void* k_cache, void* v_cache, float* beta_cache, int32_t* 
     rc = set_smem(evict_inplace_kernel<kEvictThreadsPlan>, smem, "tkv_evict_multi");
     if (rc == TKV_OK) evict_inplace_kernel<kEvictThreadsPlan><<<nseg, kEvictThreadsPlan, smem, (cudaStream_t)stream>>>(p);
   } else {
-    rc = with_evict_threads(nseg, smem, [&](auto threads) {
+    // a keep count of each segment's own is not known here: as if all rows stayed
+    rc = with_evict_threads(EvictWork::kInPlace, nseg, max_len, (int64_t)(keep_cnt ? max_len : memory_size) * head_dim * es, [&](auto threads) {
       int r = set_smem(evict_inplace_kernel<threads.value>, smem, "tkv_evict");
       if (r == TKV_OK) evict_inplace_kernel<threads.value><<<nseg, threads.value, smem, (cudaStream_t)stream>>>(p);
       return r;
@@ -803,7 +819,7 @@ extern "C" int tkv_evict_select_as(const void* beta, int beta_dtype, int64_t bet
   p.m = memory_size; p.trigger_len = trigger_len; p.max_len = max_len;
   p.kept_idx = kept_idx; p.kept_cnt = kept_cnt; p.status = status;
   const size_t smem = (size_t)max_len * 4;
-  const int rc = with_evict_threads(nseg, smem, [&](auto threads) {
+  const int rc = with_evict_threads(EvictWork::kSelect, nseg, max_len, 0, [&](auto threads) {
     int r = set_smem(evict_select_kernel<threads.value>, smem, "tkv_evict_select");
     if (r == TKV_OK) evict_select_kernel<threads.value><<<nseg, threads.value, smem, (cudaStream_t)stream>>>(p);
     return r;
