@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kRowThreads) gated_norm_vec_kernel(const T* y,
   for (int d = kLanes / 2; d >= 1; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
   const float rstd = 1.0f / sqrtf(ss / (float)len + eps);
   if (item_rt >= items) return;
-  T* o = out + (int64_t)item * len;
+  T* o = out + (int64_t)item_rt * len;
 #pragma unroll
   for (int j = 0; j < kKeep; ++j)
     if (lane + kLanes * j < nvec) {
