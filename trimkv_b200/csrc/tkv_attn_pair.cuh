@@ -9,8 +9,8 @@
 // of 128 dims) and, in a chain product - softmax - product, the length of the chain: two independent chains share the units.
 // One tile with two threads per row, S of the next key tile computed ahead and P through shared memory took 3800 cycles a tile:
 // every step crossed four barriers of 256 arrivals and waited for P . V of the step before.  Now 2500 cycles.  512 queries of 8 x 16
-// heads against 4608 keys 233 -> 192 us; differential with its preparation, 8192 tokens, 16 heads, window 4096, 652 -> 486 us; two-part,
-// 2 x 4096 tokens, 32 heads, 591 -> 435 us.  Sums are taken in the order of those kernels: the results are the same bit for bit.
+// heads against 4608 keys 233 -> 187 us; differential with its preparation, 8192 tokens, 16 heads, window 4096, 652 -> 464 us; two-part,
+// 2 x 4096 tokens, 32 heads, 591 -> 441 us.  Sums are taken in the order of those kernels: the results are the same bit for bit.
 //
 // P . V of a step reads the TMEM columns that S of the next one writes.  PTX promises an order of two products only where they have
 // one accumulator and shape, so S is issued when P . V is complete; behind S of a step O may therefore be rescaled.  O is rescaled
@@ -126,49 +126,58 @@ __device__ __forceinline__ bool pair_copies(PairSmem* sm, int nt, LoadK load_k, 
 
 // The products, in the order  P.V of tile 0 - S of tile 0 for the next keys - P.V of tile 1 - S of tile 1 for the next keys.  S waits
 // until the P.V before it is complete, since it is written over the weights which that reads.  That costs the two kernels with keys of
-// 128 dims 4 to 7 % (a warp of its own for each tile's products: 25 %, as its polling takes issue slots from the softmax; S in two halves,
+// 128 dims 3 % (a warp of its own for each tile's products: 25 %, as its polling takes issue slots from the softmax; S in two halves,
 // the one beside the weights first: 20 %, as products of 64 columns take as long as of 128).  Stages are given back where a copy will
-// wait for them, a single stage of V before S of tile 1: its copy is then ready in time (two-part 490 -> 435 us).
+// wait for them, a single stage of V before S of tile 1: its copy is then ready in time (two-part 490 -> 441 us).
 template <typename Shape, bool kBf16>
 __device__ __forceinline__ bool pair_products(PairSmem* sm, uint8_t* base, uint32_t tmem, int nt, const PairRange* range) {
   volatile int* abort_flag = &sm->abort_flag;
   const uint32_t idesc_s = pair_idesc<kBf16>(128, 0), idesc_pv = pair_idesc<kBf16>(Shape::VH * 64, 1);
+  auto weighted = [&](int t, int j, int k0, int k1) {      // 16 keys per product: 8 columns of P, 2048 bytes down the V tile
+    const uint32_t v_addr = smem_u32(Shape::v(base, j));
+#pragma unroll
+    for (int k = k0; k < k1; ++k)
+      umma_ts(tmem + 256 + 128 * t, tmem + 128 * t + 8 * k, make_desc(v_addr + k * 2048, kDaHalf, 1024, 2), idesc_pv, (j > range[t].j0 || k > 0));
+  };
+  auto scores = [&](int t, int j) {                        // 16 dims per product
+    const uint32_t q_addr = smem_u32(Shape::q(base, t)), k_addr = smem_u32(Shape::k(base, j)) + (Shape::kTwoKeys ? t * Shape::kTileK : 0);
+#pragma unroll
+    for (int k = 0; k < Shape::KH * 4; ++k) {
+      const uint32_t off = (k >> 2) * kDaHalf + (k & 3) * 32;
+      umma(tmem + 128 * t, make_desc(q_addr + off, 16, 1024, 2), make_desc(k_addr + off, 16, 1024, 2), idesc_s, k > 0);
+    }
+  };
+  auto wait_for = [&](uint64_t* bar, int t, int j) {
+    if (!mbar_wait_or_abort(bar, (j - range[t].j0) & 1, abort_flag)) return false;
+    tc_fence_after();
+    return true;
+  };
+  auto in = [&](int t, int j) { return j >= range[t].j0 && j < range[t].j1; };
   for (int j = -1; j < nt; ++j) {
     const int jn = j + 1;
-    if (jn < nt && !mbar_wait_or_abort(&sm->full_k[jn % Shape::kNK], (jn / Shape::kNK) & 1, abort_flag)) return false;
     if (j >= 0 && !mbar_wait_or_abort(&sm->full_v[j % Shape::kNV], (j / Shape::kNV) & 1, abort_flag)) return false;
-    const bool give_v = j >= 0 && j + Shape::kNV < nt, give_k = jn + Shape::kNK < nt;
+    if (jn < nt && !mbar_wait_or_abort(&sm->full_k[jn % Shape::kNK], (jn / Shape::kNK) & 1, abort_flag)) return false;
+    tc_fence_after();
+    const bool give_v = j >= 0 && j + Shape::kNV < nt;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
-      const bool now = j >= range[t].j0 && j < range[t].j1, next = jn >= range[t].j0 && jn < range[t].j1;
-      if (now) {
-        const uint32_t v_addr = smem_u32(Shape::v(base, j));
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {                      // 16 keys per product: 8 columns of P, 2048 bytes down the V tile
-          if (k % 4 == 0) {                                // the first half of P runs under the exponentials of the second
-            if (!mbar_wait_or_abort(k == 0 ? &sm->p_half[t] : &sm->p_ready[t], (j - range[t].j0) & 1, abort_flag)) return false;
-            tc_fence_after();
-          }
-          umma_ts(tmem + 256 + 128 * t, tmem + 128 * t + 8 * k, make_desc(v_addr + k * 2048, kDaHalf, 1024, 2), idesc_pv,
-                  (j > range[t].j0 || k > 0));
-        }
+      if (in(t, j)) {
+        if (!wait_for(&sm->p_half[t], t, j)) return false; // the first half of P runs under the exponentials of the second
+        weighted(t, j, 0, 4);
+        if (!wait_for(&sm->p_ready[t], t, j)) return false;
+        weighted(t, j, 4, 8);
         umma_commit(&sm->o_ready[t]);
       }
-      if (Shape::kNV == 1 && t == 1 && give_v) umma_commit(&sm->empty_v[j % Shape::kNV]);
-      if (next) {
-        if (now && !mbar_wait_or_abort(&sm->o_ready[t], (j - range[t].j0) & 1, abort_flag)) return false;
+      if (Shape::kNV == 1 && t == 1 && give_v) umma_commit(&sm->empty_v[0]);
+      if (in(t, jn)) {
+        if (in(t, j) && !wait_for(&sm->o_ready[t], t, j)) return false;
         tc_fence_after();
-        const uint32_t q_addr = smem_u32(Shape::q(base, t)), k_addr = smem_u32(Shape::k(base, jn)) + (Shape::kTwoKeys ? t * Shape::kTileK : 0);
-#pragma unroll
-        for (int k = 0; k < Shape::KH * 4; ++k) {          // 16 dims per product
-          const uint32_t off = (k >> 2) * kDaHalf + (k & 3) * 32;
-          umma(tmem + 128 * t, make_desc(q_addr + off, 16, 1024, 2), make_desc(k_addr + off, 16, 1024, 2), idesc_s, k > 0);
-        }
+        scores(t, jn);
         umma_commit(&sm->s_ready[t]);
       }
     }
     if (Shape::kNV > 1 && give_v) umma_commit(&sm->empty_v[j % Shape::kNV]);
-    if (give_k) umma_commit(&sm->empty_k[jn % Shape::kNK]);
+    if (jn + Shape::kNK < nt) umma_commit(&sm->empty_k[jn % Shape::kNK]);
   }
   return true;
 }
@@ -281,8 +290,8 @@ __device__ __forceinline__ bool pair_meet(PairSmem* sm, int phase) {
 
 // Whether CTAs of two tiles of rows take less time than CTAs of one: a CTA per SM at a time, 2.6 us per key tile for a pair against
 // 1.64 us for a tile with the chain of its own (64 segments of 192 rows, 33 key tiles: 96 us as 64 pairs, 62 us as 128 tiles; 64
-// segments of 2048 rows: 383 us as 512 pairs, 430 us as 1024 tiles).  Two-part keys of 192 dims: 3.7 and 2.6 us (2 x 4096 tokens, 32
-// heads: 435 and 591 us; 1500 tokens, 16 heads: 48 and 52 us); of 128 dims the ratio is lower, and 6000 tokens of 8 heads, 192 pairs or
+// segments of 2048 rows: 373 us as 512 pairs, 430 us as 1024 tiles).  Two-part keys of 192 dims: 3.7 and 2.6 us (2 x 4096 tokens, 32
+// heads: 441 and 591 us; 1500 tokens, 16 heads: 48 and 52 us); of 128 dims the ratio is lower, and 6000 tokens of 8 heads, 192 pairs or
 // 376 tiles, would take 118 us instead of 148.  CTAs count as equally long, which those of a prompt without a past are not: 16 segments of
 // 1536 rows take 41 us as 96 pairs, 37 us as 192 tiles.  One tile only is never a pair.
 inline bool pair_is_faster(int64_t tiles, int64_t pairs) { return pairs < tiles && (pairs + 147) / 148 * 8 < (tiles + 147) / 148 * 5; }
