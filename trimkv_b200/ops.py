@@ -5,6 +5,7 @@ CUDA kernels of libtrimkv_b200.so.
 """
 from __future__ import annotations
 
+from array import array
 from typing import Optional
 
 import torch
@@ -480,23 +481,29 @@ def greedy_next(logits, next_ids, ids, pos) -> bool:
     return True
 
 
-def _host_ints(values) -> torch.Tensor:
-    """Integers as an int32 host tensor: what ``torch.tensor`` takes as such is taken, what it refuses (beyond 32 bits) is refused."""
-    return torch.tensor(values, dtype=torch.int32, device="cpu")
+def _host_ints(values):
+    """``(address, count, shape, owner)`` of integers as int32 in host memory: what ``torch.tensor`` takes as such is taken, what it
+    refuses (beyond 32 bits) is refused.  Plain lists of integers need no tensor."""
+    try:
+        held = array("i", values)
+        return (*held.buffer_info(), (len(held),), held)
+    except (TypeError, OverflowError):
+        held = torch.tensor(values, dtype=torch.int32, device="cpu")
+        return held.data_ptr(), held.numel(), held.shape, held
 
 
 def ints_on(device, values) -> torch.Tensor:
     """A few host integers as an int32 tensor on ``device``: launch arguments of a small kernel instead of a copy, so that the
     host neither stages nor waits."""
-    host = _host_ints(values)
     if device.type != "cuda":
-        return host.to(device)
+        return torch.tensor(values, dtype=torch.int32, device=device)
+    address, n, shape, _held = _host_ints(values)
     with torch.cuda.device(device):
         if torch.cuda.is_current_stream_capturing():
             raise RuntimeError("host integers would be baked into the CUDA graph being captured")
-        out = torch.empty(host.shape, dtype=torch.int32, device=device)
-        check(lib().tkv_put_ints(out.data_ptr(), host.data_ptr(), host.numel(), _stream(out)), "tkv_put_ints")
-    _count(-(-host.numel() // 960))
+        out = torch.empty(shape, dtype=torch.int32, device=device)
+        check(lib().tkv_put_ints(out.data_ptr(), address, n, _stream(out)), "tkv_put_ints")
+    _count(-(-n // 960))
     return out
 
 
@@ -506,15 +513,14 @@ def set_ints(dst: torch.Tensor, index, value: int) -> None:
         raise IndexError(f"index outside {dst.numel()} entries")
     if not -2 ** 31 <= value < 2 ** 31:
         raise RuntimeError(f"overflow: {value} is not a 32-bit integer")
-    host = _host_ints(index)
-    n = host.numel()
     if not dst.is_cuda:
-        dst[host.long()] = value
+        dst[list(index)] = value
         return
+    address, n, _, _held = _host_ints(index)
     with torch.cuda.device_of(dst):
         if torch.cuda.is_current_stream_capturing():
             raise RuntimeError("host integers would be baked into the CUDA graph being captured")
-        check(lib().tkv_set_ints(dst.data_ptr(), host.data_ptr(), n, value, _stream(dst)), "tkv_set_ints")
+        check(lib().tkv_set_ints(dst.data_ptr(), address, n, value, _stream(dst)), "tkv_set_ints")
     _count(-(-n // 960))
 
 
