@@ -70,3 +70,29 @@ def test_prompts_in_the_callers_types(beta_type, pos_type, shared, n, transposed
 ])
 def test_widths_agree_where_the_length_decides(nseg, n, m):
     test_widths_agree(nseg, n, m)
+
+
+# the selection's digits start where the keys first differ and end where a digit's keys all stay: scores that differ in the sign, in one
+# bit, nowhere, in a few values, in everything; the fewest and the most kept; the longest segment
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [33, 1030, 57000])
+@pytest.mark.parametrize("kind", ["equal", "low_bit", "sign", "few", "wide", "narrow", "infinite"])
+def test_selection_of_any_scores(n, kind):
+    g = torch.Generator(device=DEV).manual_seed(n)
+    nseg = 3
+    draw = torch.randint(0, 2, (nseg, n), generator=g, device=DEV)
+    score = {"equal": lambda: torch.full((nseg, n), -1.5, device=DEV),
+             "low_bit": lambda: (draw + 0x3F800000).int().view(torch.float32),
+             "sign": lambda: draw * 2.0 - 1.0,
+             "few": lambda: -torch.randint(0, 5, (nseg, n), generator=g, device=DEV).float(),
+             "wide": lambda: torch.randn(nseg, n, generator=g, device=DEV) * 10.0 ** torch.randint(-30, 30, (nseg, n), generator=g, device=DEV),
+             "narrow": lambda: (torch.randint(0, 5000, (nseg, n), generator=g, device=DEV) + 0x3F800000).int().view(torch.float32),
+             "infinite": lambda: torch.where(draw == 1, float("-inf"), torch.randn(nseg, n, generator=g, device=DEV))}[kind]()
+    pos = torch.full((n,), 6, dtype=torch.int32, device=DEV)                         # q_idx - pos = 1: the score is log beta itself
+    for m in sorted({1, 2, n // 2, n - n // 8, n - 1}):
+        keep = score.sort(dim=1, descending=True, stable=True).indices[:, :m].sort(dim=1).values
+        kept, count = torch.empty(nseg, m, dtype=torch.int32, device=DEV), torch.empty(nseg, dtype=torch.int32, device=DEV)
+        status = ops.new_status(DEV)
+        ops.evict_select(score, pos, None, n, nseg, 7, m, m, n, kept, count, status)
+        assert ops.read_status(status) == 0 and bool((count == m).all())
+        assert torch.equal(kept.long(), keep)

@@ -4,7 +4,7 @@
 // torch.topk, torch.sort and four gathers into fresh allocations.  Here one CTA owns one segment:
 //   1. keys: score = f32(log beta) * f32(q_idx - pos) mapped to an order-preserving uint32, kept in
 //      shared memory (4 bytes per live token);
-//   2. 4-pass, 8-bit radix select of the M-th largest key, warp-aggregated histogram updates;
+//   2. radix select of the M-th largest key, 10 bits a pass from the first bit in which keys differ (two passes as a rule);
 //   3. one ordered block scan turns "key > T, or key == T and among the first r equal keys" into the
 //      ascending list of kept indices (written over the keys);
 //   4. in-place stable compaction: tiles of kept rows are loaded into registers (16-byte vectors),
@@ -25,47 +25,68 @@ constexpr int kEvictThreadsWide = 512;       // for long segments, whose key arr
 constexpr int kMoveThreads = 256;            // evict_move_kernel: its staging area limits CTAs per SM, so each is wide
 constexpr int kMoveGridCtas = 148 * 4;       // evict_move_kernel: blocks in its grid (they loop over the evicting segments)
 constexpr int kEvictThreadsPlan = 1024;      // selection only (plan mode), and few segments: each gets a full CTA
+constexpr int kSelectBits = 10;              // of a key per pass; the bins and the keys of kMaxSelectLen tokens fill shared memory
 struct SelectScratch {
-  int hist[256];
+  int hist[1 << kSelectBits];
   int warp_sums[kEvictThreadsPlan / 32 + 1];
+  uint32_t differ;
   int sel_digit;
   int sel_k;
+  int sel_count;
   int first_evicted;
 };
+static_assert(kMaxSelectLen * 4 + sizeof(SelectScratch) <= 232448, "shared memory of the selection");
 
-// Finds T = key of the m-th largest element and r = how many elements equal to T are kept.
-// All threads of the block call this; keys[0..n) are in shared memory.
+// Finds T and r such that the m < n largest of keys[0..n) (shared memory; the lower index first among equals) are the keys above T and
+// the first r that equal T.  All threads of the block call this.  Digits start at the highest bit in which the keys differ: scores share
+// sign and much of the exponent, and a digit that few values take would serialise the counting and decide little.  A pass ends the
+// search when its bin is kept whole, which for scores without many ties is the second one.  Fixed digits of 8 bits from the top,
+// counted by one elected lane per digit, took four passes of 2300 to 4100 cycles each for 4608 keys and 1024 threads.
 template <int kThreads>
 __device__ __forceinline__ void radix_select_mth(const uint32_t* keys, int n, int m, SelectScratch* sc,
                                                  uint32_t* thresh, int* n_eq_keep) {
-  const int lane = threadIdx.x & 31;
-  uint32_t prefix = 0, decided = 0;
-  int k = m;
-  const int n_round = (n + kThreads - 1) / kThreads * kThreads;
+  constexpr int kBins = 1 << kSelectBits, kPer = kBins / kThreads;
+  if (threadIdx.x == 0) sc->differ = 0;
+  __syncthreads();
+  const uint32_t any = keys[0];
+  uint32_t diff = 0;
+  for (int i = threadIdx.x; i < n; i += kThreads) diff |= keys[i] ^ any;
+  diff = __reduce_or_sync(0xffffffffu, diff);
+  if ((threadIdx.x & 31) == 0 && diff != 0) atomicOr(&sc->differ, diff);
+  __syncthreads();
+  int rest = 32 - __clz(sc->differ), k = m;                // bits still open
+  uint32_t prefix = rest == 32 ? 0u : any & (0xffffffffu << rest);
 #pragma unroll 1
-  for (int shift = 24; shift >= 0; shift -= 8) {
-    if (threadIdx.x < 256) sc->hist[threadIdx.x] = 0;
+  while (rest > 0) {
+    const int bits = min(kSelectBits, rest), shift = rest - bits;
+    const uint32_t decided = rest == 32 ? 0u : 0xffffffffu << rest, mask = (1u << bits) - 1u;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) sc->hist[threadIdx.x + u * kThreads] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < n_round; i += kThreads) {
-      uint32_t key = i < n ? keys[i] : 0u;
-      const bool valid = i < n && (key & decided) == prefix;
-      const int digit = valid ? (int)((key >> shift) & 255u) : 256 + lane;
-      // Lanes with the same digit elect one leader that adds their count: the high digits of the
-      // scores are nearly constant, which would serialise plain shared-memory atomics.
-      const unsigned peers = __match_any_sync(0xffffffffu, digit);
-      if (valid && lane == __ffs(peers) - 1) atomicAdd(&sc->hist[digit], __popc(peers));
+    for (int i = threadIdx.x; i < n; i += kThreads) {
+      const uint32_t key = keys[i];
+      if ((key & decided) == prefix) atomicAdd(&sc->hist[(key >> shift) & mask], 1);
     }
     __syncthreads();
-    // Thread t looks at bin 255 - t: an exclusive scan in this order is the count of strictly larger digits.
-    const int bin = 255 - (int)threadIdx.x;
-    const int c = threadIdx.x < 256 ? sc->hist[bin] : 0;
+    // Thread t looks at kPer bins from kBins - 1 - kPer * t down: an exclusive scan in this order counts the strictly larger digits.
+    int c[kPer], sum = 0;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) { c[u] = sc->hist[kBins - 1 - (kPer * (int)threadIdx.x + u)]; sum += c[u]; }
     int total;
-    const int above = block_exclusive_scan<kThreads>(c, sc->warp_sums, &total);
-    if (threadIdx.x < 256 && above < k && k <= above + c) { sc->sel_digit = bin; sc->sel_k = k - above; }
+    int above = block_exclusive_scan<kThreads>(sum, sc->warp_sums, &total);
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      if (above < k && k <= above + c[u]) { sc->sel_digit = kBins - 1 - (kPer * (int)threadIdx.x + u); sc->sel_k = k - above; sc->sel_count = c[u]; }
+      above += c[u];
+    }
     __syncthreads();
     prefix |= (uint32_t)sc->sel_digit << shift;
-    decided |= 255u << shift;
     k = sc->sel_k;
+    rest = shift;
+    if (sc->sel_count == k && rest > 0) {                  // all of them stay; not the lowest prefix, as m < n
+      *thresh = prefix - 1; *n_eq_keep = 0;
+      return;
+    }
     __syncthreads();
   }
   *thresh = prefix;
@@ -625,26 +646,30 @@ static int set_smem(K kernel, size_t bytes, const char* what) {
   return TKV_OK;
 }
 
-// Threads of a segment's CTA.  A segment is one CTA's, and its time is the latency of rounds over its keys (four selection passes
-// and the list) and of tiles of rows (load, barrier, store): the fewer threads, the more rounds and tiles; the more threads, the dearer
-// each of the barriers, and the fewer CTAs on an SM.  So few segments get wide CTAs, short ones narrow CTAs, and beyond two CTAs of
-// 512 per SM only segments whose key array leaves room for at most 3 CTAs get 512.  us with 256, 512 and 1024 threads:
-//   in place, 64 segments of     144 -> 128 rows   9.0   9.9  13.1      16 of  640 ->  512  17.6  17.1  17.1
-//                               1152 -> 1024      35.9  28.7  30.0            4608 -> 4096 109.7  84.8  78.2
-//   in place, 224 segments of    640 -> 512       30.9  32.2  40.1            1536 -> 1024  57.4  55.8  65.4
-//                               4608 -> 4096     197.0 205.2 192.5            2048 ->  256  34.0  29.0  38.5
-//   selection, 64 segments of    640 -> 512        8.5   9.4   9.9            4224 -> 4096  25.8  24.6  26.1    8192 -> 1024  43.0  39.4  35.7
-//   selection, 224 segments of  1152 -> 1024      15.0  16.2  22.2            4608 -> 4096  42.5  38.9  44.9
-// `moved`: bytes of K of a segment's kept rows; where they outweigh the keys, memory and not latency bounds 193 segments and more.
+// Threads of a segment's CTA.  A segment is one CTA's, and its time is the latency of rounds over its keys (two selection passes and
+// the list) and of tiles of rows (load, barrier, store): the fewer threads, the more rounds and tiles; the more threads, the dearer
+// each of the barriers, and the fewer CTAs on an SM.  So few and long segments get wide CTAs, many and short ones narrow CTAs.  us with
+// 256, 512 and 1024 threads:
+//   in place, 148 segments of  144 ->  128 rows   9.0   8.4   9.2     1152 -> 1024   39.4  34.3  34.8      4224 -> 4096  141   121   120
+//             224              400 ->  256       16.9  16.1  21.8     1152 -> 1024   47.9  49.4  52.4      4608 -> 4096  175   186   169
+//             296             1152 ->  1024      60.2  60.7  64.8     4224 -> 4096   229   225   229       8192 -> 1024   80    70    76
+//            2048              144 ->  128       51.7  61.1   104     1152 -> 1024   358   354   378       4224 -> 4096 1421  1408  1446
+//   selection, 148 segments   1152 -> 1024        7.9   7.2   7.4     4224 -> 4096   13.6  10.2   9.2      8192 -> 1024   22.0  14.1  11.3
+//              296            1152 -> 1024        8.2   8.2   9.7     4224 -> 4096   14.6  12.0  12.6     16512 -> 16384  41.0  28.4  26.6
+//             2048            1152 -> 1024       20.5  27.4  45.6     4224 -> 4096   52.2  58.6  76.8      8192 -> 1024  102.1  83.7  97.8
+// `moved`: bytes of K of a segment's kept rows.  Where they outweigh the keys and 512 threads would leave one CTA on some SMs and two on
+// others, up to about 1.75 a SM, CTAs of a whole SM in two rounds share the memory better (224 segments above).
 enum class EvictWork { kInPlace, kSelect };
 template <typename F> static int with_evict_threads(EvictWork work, int nseg, int n, int64_t moved, F launch) {
-  int threads = n > 14336 ? kEvictThreadsWide : kEvictThreads;
+  int threads = kEvictThreadsWide;
   if (work == EvictWork::kInPlace) {
-    if (nseg <= 148) threads = n >= 2048 ? kEvictThreadsPlan : n > 256 ? kEvictThreadsWide : kEvictThreads;
-    else if (nseg <= 2 * 148 && n > 256 && !(n > 512 && moved > 200 * (int64_t)n && (nseg > 192 || n <= 1024))) threads = kEvictThreadsWide;
+    if (nseg <= 148) threads = n >= 2048 ? kEvictThreadsPlan : kEvictThreadsWide;
+    else if (nseg <= 2 * 148) threads = nseg > 192 && nseg <= 259 && n >= 2048 && moved > 200 * (int64_t)n ? kEvictThreadsPlan : kEvictThreadsWide;
+    else threads = n > 512 ? kEvictThreadsWide : kEvictThreads;
   } else {
-    if (nseg <= 148) threads = n >= 8192 ? kEvictThreadsPlan : n > 1024 ? kEvictThreadsWide : kEvictThreads;
-    else if (nseg <= 2 * 148 && n >= 1536) threads = kEvictThreadsWide;
+    if (nseg <= 148) threads = n >= 4096 ? kEvictThreadsPlan : n > 256 ? kEvictThreadsWide : kEvictThreads;
+    else if (nseg <= 2 * 148) threads = n >= 16384 ? kEvictThreadsPlan : n > 1024 ? kEvictThreadsWide : kEvictThreads;
+    else threads = n >= 6144 ? kEvictThreadsWide : kEvictThreads;
   }
   if (threads == kEvictThreadsPlan) return launch(std::integral_constant<int, kEvictThreadsPlan>());
   if (threads == kEvictThreadsWide) return launch(std::integral_constant<int, kEvictThreadsWide>());
@@ -893,6 +918,7 @@ extern "C" int tkv_compact_as(void* k_dst, void* v_dst, float* beta_dst, int32_t
 namespace tkv {
 
 constexpr int kBudgetThreads = 1024;
+constexpr int kBudgetBits = 11;              // of a key per pass
 constexpr int kBudgetMaxSegs = 2048;
 
 struct BudgetParams {
@@ -911,7 +937,7 @@ __global__ void __launch_bounds__(kBudgetThreads) group_budget_kernel(BudgetPara
   __shared__ int s_len[kBudgetMaxSegs];
   __shared__ int s_gt[kBudgetMaxSegs];
   __shared__ int s_eq[kBudgetMaxSegs];
-  __shared__ int hist[256];
+  __shared__ int hist[1 << kBudgetBits];
   __shared__ int warp_sums[kBudgetThreads / 32 + 1];
   __shared__ int sel_digit, sel_k;
   __shared__ long long s_total;
@@ -938,39 +964,40 @@ __global__ void __launch_bounds__(kBudgetThreads) group_budget_kernel(BudgetPara
   } else if (p.k_total <= 0) {
     thresh = 0xFFFFFFFFu; n_eq_keep = 0;
   } else {
-    // 4-pass radix select of the k_total-th largest key over all rows of the group.
+    // Radix select of the k_total-th largest key over all rows of the group, in three passes.  Plain shared-memory counters: one elected
+    // lane per digit (__match_any_sync) made a pass over the 8 x 4096 rows of each of 64 groups take 24 us (4 x 8 bits, 160 us in all;
+    // 76 without it).
     uint32_t prefix = 0, decided = 0;
     long long k = p.k_total;
 #pragma unroll 1
-    for (int shift = 24; shift >= 0; shift -= 8) {
-      if (tid < 256) hist[tid] = 0;
+    for (int rest = 32; rest > 0;) {
+      const int bits = min(kBudgetBits, rest), shift = rest - bits;
+      for (int u = tid; u < 1 << kBudgetBits; u += kBudgetThreads) hist[u] = 0;
       __syncthreads();
       for (int j = 0; j < nsegs; ++j) {
         const int n = s_len[j];
         const int64_t row0 = seg_of(j) * p.cap;
-        const int n_round = (n + kBudgetThreads - 1) / kBudgetThreads * kBudgetThreads;
-        for (int i = tid; i < n_round; i += kBudgetThreads) {
-          bool valid = i < n;
-          uint32_t key = 0;
-          if (valid) {
-            key = score_key(p.scores != nullptr ? p.scores[row0 + i] : retention_score_as(p.beta[row0 + i], p.pos[row0 + i], p.q_idx, p.score_dtype));
-            valid = (key & decided) == prefix;
-          }
-          const int digit = valid ? (int)((key >> shift) & 255u) : 256 + lane;
-          const unsigned peers = __match_any_sync(0xffffffffu, digit);
-          if (valid && lane == __ffs(peers) - 1) atomicAdd(&hist[digit], __popc(peers));
+        for (int i = tid; i < n; i += kBudgetThreads) {
+          const uint32_t key = score_key(p.scores != nullptr ? p.scores[row0 + i] : retention_score_as(p.beta[row0 + i], p.pos[row0 + i], p.q_idx, p.score_dtype));
+          if ((key & decided) == prefix) atomicAdd(&hist[(key >> shift) & ((1u << bits) - 1u)], 1);
         }
       }
       __syncthreads();
-      // bins from the top: thread t (< 256) looks at bin 255 - t
-      const int bin = 255 - tid;
-      const int c = tid < 256 ? hist[bin] : 0;
-      int tot;
-      const int above = block_exclusive_scan<kBudgetThreads>(c, warp_sums, &tot);
-      if (tid < 256 && above < k && k <= (long long)above + c) { sel_digit = bin; sel_k = (int)(k - above); }
+      // bins from the top: thread t looks at two of them
+      constexpr int kPer = (1 << kBudgetBits) / kBudgetThreads;
+      int c[kPer], sum = 0, tot;
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) { c[u] = hist[(1 << kBudgetBits) - 1 - (kPer * tid + u)]; sum += c[u]; }
+      int above = block_exclusive_scan<kBudgetThreads>(sum, warp_sums, &tot);
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        if (above < k && k <= (long long)above + c[u]) { sel_digit = (1 << kBudgetBits) - 1 - (kPer * tid + u); sel_k = (int)(k - above); }
+        above += c[u];
+      }
       __syncthreads();
       prefix |= (uint32_t)sel_digit << shift;
-      decided |= 255u << shift;
+      decided = shift == 0 ? 0xffffffffu : 0xffffffffu << shift;
+      rest = shift;
       k = sel_k;
       __syncthreads();
     }
