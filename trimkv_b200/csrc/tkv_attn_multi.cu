@@ -68,7 +68,7 @@ multi_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   const int seg = blockIdx.x / p.nchunks, chunk = blockIdx.x - seg * p.nchunks;
   const int len = min(p.seg_len[seg], p.max_len);
   const int t0 = chunk * kMtChunk;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int b = seg / p.hkv, h = seg - b * p.hkv;
   const int G = p.hq / p.hkv;
   const int row_base = blockIdx.y * kMtRows;
@@ -140,25 +140,26 @@ multi_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   volatile int* abort_flag = &sm->abort_flag;
   bool v1_issued = false;
 
-  // ---- thread 0: S = K . Q^T for both tiles
-  if (tid == 0) {
+  // ---- warp 0: S = K . Q^T for both tiles
+  const uint32_t tm = warp_uniform(tmem);
+  if (warp == 0) {
+    const uint64_t a_desc = make_desc(smem_u32(stage), 16, 1024, 2), b_desc = make_desc(smem_u32(q_s), 128, 2048, 0);
     bool ok = true;
     for (int i = 0; i < ntiles && ok; ++i) {
-      ok = mbar_wait(&sm->bar_k[i], 0);
+      ok = (bool)__all_sync(0xffffffffu, mbar_wait(&sm->bar_k[i], 0));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t a0 = smem_u32(stage + i * kMtStageBytes);
+      if (elect_one()) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint64_t ad = make_desc(a0 + (k >> 2) * kMtHalfBytes + (k & 3) * 32, 16, 1024, 2);
-        const uint64_t bd = make_desc(smem_u32(q_s) + k * 256, 128, 2048, 0);
-        umma(tmem + kMtRows * i, ad, bd, idesc_qk, k > 0);
+        for (int k = 0; k < 8; ++k)
+          umma(tm + kMtRows * i, a_desc + i * (kMtStageBytes >> 4) + (uint32_t)((k >> 2) * kMtHalfBytes + (k & 3) * 32) / 16, b_desc + k * 16, idesc_qk, k > 0);
+        if (i == ntiles - 1) umma_commit(&sm->bar_s);
       }
+      __syncwarp();
     }
-    if (ok) umma_commit(&sm->bar_s);
-    else { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+    if (!ok && lane == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+    __syncwarp();
   }
-  __syncwarp();
   if (!mbar_wait_or_abort(&sm->bar_s, 0, abort_flag)) {
     if (*abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
   }
@@ -236,25 +237,25 @@ multi_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // ---- thread 0: O^T += V^T . P for both tiles
-  if (tid == 0 && *abort_flag == 0) {
+  // ---- warp 0: O^T += V^T . P for both tiles
+  if (warp == 0 && __all_sync(0xffffffffu, *abort_flag == 0)) {
+    const uint64_t a_desc = make_desc(smem_u32(stage), kMtHalfBytes, 1024, 2), b_desc = make_desc(smem_u32(p_s), 128, 2048, 0);
     bool ok = true;
     for (int i = 0; i < ntiles && ok; ++i) {
-      ok = mbar_wait(&sm->bar_v[i], 0);
+      ok = (bool)__all_sync(0xffffffffu, mbar_wait(&sm->bar_v[i], 0));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t a0 = smem_u32(stage + (i == 0 ? 2 : 0) * kMtStageBytes);
+      if (elect_one()) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint64_t ad = make_desc(a0 + k * 2048, kMtHalfBytes, 1024, 2);
-        const uint64_t bd = make_desc(smem_u32(p_s + i * kMtPBytes) + k * 256, 128, 2048, 0);
-        umma(tmem + 2 * kMtRows, ad, bd, idesc_pv, (i > 0 || k > 0));
+        for (int k = 0; k < 8; ++k)
+          umma(tm + 2 * kMtRows, a_desc + (i == 0 ? 2 : 0) * (kMtStageBytes >> 4) + k * 128, b_desc + i * (kMtPBytes >> 4) + k * 16, idesc_pv, (i > 0 || k > 0));
+        if (i == ntiles - 1) umma_commit(&sm->bar_o);
       }
+      __syncwarp();
     }
-    if (ok) umma_commit(&sm->bar_o);
-    else { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+    if (!ok && lane == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+    __syncwarp();
   }
-  __syncwarp();
   bool have_o = *abort_flag == 0 && mbar_wait_or_abort(&sm->bar_o, 0, abort_flag);
   if (!have_o && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
   tc_fence_after();

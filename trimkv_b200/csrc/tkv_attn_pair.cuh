@@ -129,55 +129,74 @@ __device__ __forceinline__ bool pair_copies(PairSmem* sm, int nt, LoadK load_k, 
 // 128 dims 3 % (a warp of its own for each tile's products: 25 %, as its polling takes issue slots from the softmax; S in two halves,
 // the one beside the weights first: 20 %, as products of 64 columns take as long as of 128).  Stages are given back where a copy will
 // wait for them, a single stage of V before S of tile 1: its copy is then ready in time (two-part 490 -> 441 us).
+// Run by a whole warp.
 template <typename Shape, bool kBf16>
-__device__ __forceinline__ bool pair_products(PairSmem* sm, uint8_t* base, uint32_t tmem, int nt, const PairRange* range) {
+__device__ __forceinline__ bool pair_products(PairSmem* sm, uint8_t* base, uint32_t tmem_, int nt_, const PairRange* range_) {
   volatile int* abort_flag = &sm->abort_flag;
   const uint32_t idesc_s = pair_idesc<kBf16>(128, 0), idesc_pv = pair_idesc<kBf16>(Shape::VH * 64, 1);
+  const uint32_t tmem = warp_uniform(tmem_);
+  const int nt = warp_uniform(nt_);
+  const PairRange range[2] = {{warp_uniform(range_[0].j0), warp_uniform(range_[0].j1)}, {warp_uniform(range_[1].j0), warp_uniform(range_[1].j1)}};
+  const uint64_t q_desc = make_desc(smem_u32(Shape::q(base, 0)), 16, 1024, 2), k_desc = make_desc(smem_u32(Shape::k(base, 0)), 16, 1024, 2),
+                 v_desc = make_desc(smem_u32(Shape::v(base, 0)), kDaHalf, 1024, 2);   // in units of 16 bytes
   auto weighted = [&](int t, int j, int k0, int k1) {      // 16 keys per product: 8 columns of P, 2048 bytes down the V tile
-    const uint32_t v_addr = smem_u32(Shape::v(base, j));
+    const uint64_t v = v_desc + (uint32_t)(j % Shape::kNV) * (Shape::kStageV >> 4);
 #pragma unroll
-    for (int k = k0; k < k1; ++k)
-      umma_ts(tmem + 256 + 128 * t, tmem + 128 * t + 8 * k, make_desc(v_addr + k * 2048, kDaHalf, 1024, 2), idesc_pv, (j > range[t].j0 || k > 0));
+    for (int k = k0; k < k1; ++k) umma_ts(tmem + 256 + 128 * t, tmem + 128 * t + 8 * k, v + k * 128, idesc_pv, (j > range[t].j0 || k > 0));
   };
   auto scores = [&](int t, int j) {                        // 16 dims per product
-    const uint32_t q_addr = smem_u32(Shape::q(base, t)), k_addr = smem_u32(Shape::k(base, j)) + (Shape::kTwoKeys ? t * Shape::kTileK : 0);
+    const uint64_t q = q_desc + t * (Shape::kTileQ >> 4);
+    const uint64_t k_ = k_desc + (uint32_t)(j % Shape::kNK) * (Shape::kStageK >> 4) + (Shape::kTwoKeys ? t * (Shape::kTileK >> 4) : 0);
 #pragma unroll
     for (int k = 0; k < Shape::KH * 4; ++k) {
-      const uint32_t off = (k >> 2) * kDaHalf + (k & 3) * 32;
-      umma(tmem + 128 * t, make_desc(q_addr + off, 16, 1024, 2), make_desc(k_addr + off, 16, 1024, 2), idesc_s, k > 0);
+      const uint32_t off = (k >> 2) * (kDaHalf >> 4) + (k & 3) * 2;
+      umma(tmem + 128 * t, q + off, k_ + off, idesc_s, k > 0);
     }
   };
   auto wait_for = [&](uint64_t* bar, int t, int j) {
-    if (!mbar_wait_or_abort(bar, (j - range[t].j0) & 1, abort_flag)) return false;
+    if (!warp_wait(bar, (j - range[t].j0) & 1, abort_flag)) return false;
     tc_fence_after();
     return true;
   };
   auto in = [&](int t, int j) { return j >= range[t].j0 && j < range[t].j1; };
   for (int j = -1; j < nt; ++j) {
     const int jn = j + 1;
-    if (j >= 0 && !mbar_wait_or_abort(&sm->full_v[j % Shape::kNV], (j / Shape::kNV) & 1, abort_flag)) return false;
-    if (jn < nt && !mbar_wait_or_abort(&sm->full_k[jn % Shape::kNK], (jn / Shape::kNK) & 1, abort_flag)) return false;
+    if (j >= 0 && !warp_wait(&sm->full_v[j % Shape::kNV], (j / Shape::kNV) & 1, abort_flag)) return false;
+    if (jn < nt && !warp_wait(&sm->full_k[jn % Shape::kNK], (jn / Shape::kNK) & 1, abort_flag)) return false;
     tc_fence_after();
     const bool give_v = j >= 0 && j + Shape::kNV < nt;
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       if (in(t, j)) {
         if (!wait_for(&sm->p_half[t], t, j)) return false; // the first half of P runs under the exponentials of the second
-        weighted(t, j, 0, 4);
+        if (elect_one()) weighted(t, j, 0, 4);
+        __syncwarp();
         if (!wait_for(&sm->p_ready[t], t, j)) return false;
-        weighted(t, j, 4, 8);
-        umma_commit(&sm->o_ready[t]);
+        if (elect_one()) {
+          weighted(t, j, 4, 8);
+          umma_commit(&sm->o_ready[t]);
+        }
+        __syncwarp();
       }
-      if (Shape::kNV == 1 && t == 1 && give_v) umma_commit(&sm->empty_v[0]);
+      if (Shape::kNV == 1 && t == 1 && give_v) {
+        if (elect_one()) umma_commit(&sm->empty_v[0]);
+        __syncwarp();
+      }
       if (in(t, jn)) {
         if (in(t, j) && !wait_for(&sm->o_ready[t], t, j)) return false;
         tc_fence_after();
-        scores(t, jn);
-        umma_commit(&sm->s_ready[t]);
+        if (elect_one()) {
+          scores(t, jn);
+          umma_commit(&sm->s_ready[t]);
+        }
+        __syncwarp();
       }
     }
-    if (Shape::kNV > 1 && give_v) umma_commit(&sm->empty_v[j % Shape::kNV]);
-    if (jn + Shape::kNK < nt) umma_commit(&sm->empty_k[jn % Shape::kNK]);
+    if (elect_one()) {
+      if (Shape::kNV > 1 && give_v) umma_commit(&sm->empty_v[j % Shape::kNV]);
+      if (jn + Shape::kNK < nt) umma_commit(&sm->empty_k[jn % Shape::kNK]);
+    }
+    __syncwarp();
   }
   return true;
 }

@@ -35,7 +35,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   grid_launch_dependents();
   const int seg = (int)(blockIdx.x / (unsigned)nblocks);
   const int blk = nblocks - 1 - (int)(blockIdx.x % (unsigned)nblocks);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
   const bool is_row = warp < 8;
   const int t = (tid >> 7) & 1, row = tid & (kPfTile - 1);
   const int G = p.hq / p.hkv;
@@ -91,7 +91,7 @@ prefill_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   int k_issued = 0, v_issued = 0;                          // copying lane: tiles whose copies have been started
   bool ok = true;
   if (warp == 8) {
-    if ((tid & 31) == 0) ok = pair_products<PfShape, kBf16>(sm, base, tmem, ntiles, range);
+    ok = pair_products<PfShape, kBf16>(sm, base, tmem, ntiles, range);
     __syncwarp();
   } else if (warp == 9) {
     if ((tid & 31) == 0) {
@@ -159,7 +159,7 @@ prefill_attn_one_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   grid_launch_dependents();
   const int seg = (int)(blockIdx.x / (unsigned)nblocks);
   const int blk = nblocks - 1 - (int)(blockIdx.x % (unsigned)nblocks);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
   const bool is_ctrl = warp == 8;
   const int row = tid & (kPfTile - 1), half = (tid >> 7) & 1;
   const int G = p.hq / p.hkv;
@@ -196,20 +196,18 @@ prefill_attn_one_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   volatile int* abort_flag = &sm->abort_flag;
   const int64_t row0 = (int64_t)seg * p.cap;
 
-  int k_issued = 0, v_issued = 0;                          // control lane: tiles whose copies have been started
+  int k_issued = 0, v_issued = 0;                          // control warp: tiles whose copies have been started
   auto load_k = [&](int j) {
     const int st = j & 1;
     mbar_expect_tx(&sm->bar_k[st], kPfTileBytes);
     tma_load_2d(k_s + st * kPfTileBytes, &map_k, &sm->bar_k[st], 0, (int)(row0 + j * kPfTile));
     tma_load_2d(k_s + st * kPfTileBytes + kDaHalf, &map_k, &sm->bar_k[st], 64, (int)(row0 + j * kPfTile));
-    ++k_issued;
   };
   auto load_v = [&](int j) {
     const int st = j & 1;
     mbar_expect_tx(&sm->bar_v[st], kPfTileBytes);
     tma_load_2d(v_s + st * kPfTileBytes, &map_v, &sm->bar_v[st], 0, (int)(row0 + j * kPfTile));
     tma_load_2d(v_s + st * kPfTileBytes + kDaHalf, &map_v, &sm->bar_v[st], 64, (int)(row0 + j * kPfTile));
-    ++v_issued;
   };
   if (tid == kDaSoftmaxThreads) {
     for (int i = 0; i < 2; ++i) { mbar_init(&sm->bar_k[i], 1); mbar_init(&sm->bar_v[i], 1); mbar_init(&sm->bar_s[i], 1); }
@@ -220,6 +218,8 @@ prefill_attn_one_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     for (int i = 0; i < 2 && i < ntiles; ++i) load_k(i);
     load_v(0);
+    k_issued = min(2, ntiles);
+    v_issued = 1;
   }
   __syncwarp();
   if (is_ctrl) {
@@ -240,53 +240,65 @@ prefill_attn_one_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
   const uint32_t tmem = sm->tmem_base;
 
   if (is_ctrl) {
-    // ------------------------------------------------------------------------------------ TMA + MMA issue (one lane)
-    if (tid == kDaSoftmaxThreads) {
+    // ------------------------------------------------------------------------------------ TMA + MMA issue (whole warp, elected lane)
+    {
+      const uint32_t tm = warp_uniform(tmem);
+      const int nt = warp_uniform(ntiles);
       const uint32_t idesc_s = pair_idesc<kDtype == TKV_BF16>(128, 0);
       const uint32_t idesc_pv = pair_idesc<kDtype == TKV_BF16>(128, 1);
-      const uint32_t q_addr = smem_u32(q_s), p_addr = smem_u32(p_s);
+      const uint64_t q_desc = make_desc(smem_u32(q_s), 16, 1024, 2), p_desc = make_desc(smem_u32(p_s), 16, 1024, 2),
+                     k_desc = make_desc(smem_u32(k_s), 16, 1024, 2), v_desc = make_desc(smem_u32(v_s), kDaHalf, 1024, 2);
       auto issue_s = [&](int j) -> bool {       // S of tile j into S buffer j & 1
-        if (!mbar_wait_or_abort(&sm->bar_k[j & 1], (j >> 1) & 1, abort_flag)) return false;
+        if (!warp_wait(&sm->bar_k[j & 1], (j >> 1) & 1, abort_flag)) return false;
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(k_s + (j & 1) * kPfTileBytes);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {   // 16 dims per MMA: 4 steps inside a 128-byte swizzle atom, then the other half
-          const uint32_t off = (k >> 2) * kDaHalf + (k & 3) * 32;
-          umma(tmem + 128 * (j & 1), make_desc(q_addr + off, 16, 1024, 2), make_desc(k_addr + off, 16, 1024, 2), idesc_s, k > 0);
+          for (int k = 0; k < 8; ++k) { // 16 dims per MMA: 4 steps inside a 128-byte swizzle atom, then the other half
+            const uint32_t off = (k >> 2) * (kDaHalf >> 4) + (k & 3) * 2;
+            umma(tm + 128 * (j & 1), q_desc + off, k_desc + (j & 1) * (kPfTileBytes >> 4) + off, idesc_s, k > 0);
+          }
+          umma_commit(&sm->bar_s[j & 1]);
         }
-        umma_commit(&sm->bar_s[j & 1]);
+        __syncwarp();
         return true;
       };
       bool ok = issue_s(0);
-      for (int j = 0; j < ntiles && ok; ++j) {
+      for (int j = 0; j < nt && ok; ++j) {
         // S of the next tile: its buffer was read for tile j-1, whose P has been waited for below (bar_p) already
-        if (j + 1 < ntiles) ok = issue_s(j + 1);
+        if (j + 1 < nt) ok = issue_s(j + 1);
         // V of the next tile goes where V of tile j-1 was: free once P.V of tile j-1 has completed
-        if (ok && j + 1 < ntiles) {
-          if (j > 0) ok = mbar_wait_or_abort(&sm->bar_o, (j - 1) & 1, abort_flag);
-          if (ok) load_v(j + 1);
+        if (ok && j + 1 < nt) {
+          if (j > 0) ok = warp_wait(&sm->bar_o, (j - 1) & 1, abort_flag);
+          if (ok) {
+            if (elect_one()) load_v(j + 1);
+            __syncwarp();
+            ++v_issued;
+          }
         }
         // K two tiles ahead goes where K of this tile is: free once S of this tile has completed
-        if (ok && j + 2 < ntiles) {
-          ok = mbar_wait_or_abort(&sm->bar_s[j & 1], (j >> 1) & 1, abort_flag);
-          if (ok) load_k(j + 2);
+        if (ok && j + 2 < nt) {
+          ok = warp_wait(&sm->bar_s[j & 1], (j >> 1) & 1, abort_flag);
+          if (ok) {
+            if (elect_one()) load_k(j + 2);
+            __syncwarp();
+            ++k_issued;
+          }
         }
         // O += P . V once the softmax warps have written all of P (and rescaled O if they had to)
-        if (ok) ok = mbar_wait_or_abort(&sm->bar_p, j & 1, abort_flag);
-        if (ok) ok = mbar_wait_or_abort(&sm->bar_v[j & 1], (j >> 1) & 1, abort_flag);
+        if (ok) ok = warp_wait(&sm->bar_p, j & 1, abort_flag);
+        if (ok) ok = warp_wait(&sm->bar_v[j & 1], (j >> 1) & 1, abort_flag);
         if (ok) {
           tc_fence_after();
-          const uint32_t v_addr = smem_u32(v_s + (j & 1) * kPfTileBytes);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {   // 16 tokens per MMA: along K of P inside the swizzle atom, 2048 B down the V tile
-            const uint64_t ad = make_desc(p_addr + (k >> 2) * kDaHalf + (k & 3) * 32, 16, 1024, 2);
-            const uint64_t bd = make_desc(v_addr + k * 2048, kDaHalf, 1024, 2);
-            umma(tmem + 256, ad, bd, idesc_pv, (j > 0 || k > 0));
+            for (int k = 0; k < 8; ++k)   // 16 tokens per MMA: along K of P inside the swizzle atom, 2048 B down the V tile
+              umma(tm + 256, p_desc + (k >> 2) * (kDaHalf >> 4) + (k & 3) * 2, v_desc + (j & 1) * (kPfTileBytes >> 4) + k * 128, idesc_pv, (j > 0 || k > 0));
+            umma_commit(&sm->bar_o);
           }
-          umma_commit(&sm->bar_o);
+          __syncwarp();
         }
       }
-      if (!ok && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+      if (!ok && tid == kDaSoftmaxThreads && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
     }
     __syncwarp();
   } else {

@@ -78,7 +78,7 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   if (chunk == 0 && threadIdx.x == 0 && p.seg_len[seg] > p.max_len) report(p.status, TKV_DEV_LEN_BOUND);
   const int n_valid = min(kTcChunk, len - t0);
   const int ntiles = (n_valid + kTileTokens - 1) / kTileTokens;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int b = seg / p.hkv, h = seg - b * p.hkv;
 
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -132,25 +132,26 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   volatile int* abort_flag = &sm->abort_flag;
   bool v1_issued = false;
 
-  // ---- thread 0: S = K . Q^T for both tiles
-  if (tid == 0) {
+  // ---- warp 0: S = K . Q^T for both tiles
+  const uint32_t tm = warp_uniform(tmem);
+  if (warp == 0) {
+    const uint64_t a_desc = make_desc(smem_u32(stage), 16, 1024, 2), b_desc = make_desc(smem_u32(q_s), 128, 2048, 0);
     bool ok = true;
     for (int i = 0; i < ntiles && ok; ++i) {
-      ok = mbar_wait(&sm->bar_k[i], 0);
+      ok = (bool)__all_sync(0xffffffffu, mbar_wait(&sm->bar_k[i], 0));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t a0 = smem_u32(stage + i * kStageBytes);
+      if (elect_one()) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {  // 16 dims per MMA; 4 steps inside a 128-byte swizzle atom, then the next half
-        const uint64_t ad = make_desc(a0 + (k >> 2) * kHalfBytes + (k & 3) * 32, 16, 1024, 2);
-        const uint64_t bd = make_desc(smem_u32(q_s) + k * 256, 128, 2048, 0);
-        umma(tmem + 16 * i, ad, bd, idesc_qk, k > 0);
+        for (int k = 0; k < 8; ++k)  // 16 dims per MMA; 4 steps inside a 128-byte swizzle atom, then the next half
+          umma(tm + 16 * i, a_desc + i * (kStageBytes >> 4) + (uint32_t)((k >> 2) * kHalfBytes + (k & 3) * 32) / 16, b_desc + k * 16, idesc_qk, k > 0);
+        if (i == ntiles - 1) umma_commit(&sm->bar_s);
       }
+      __syncwarp();
     }
-    if (ok) umma_commit(&sm->bar_s);
-    else { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+    if (!ok && lane == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+    __syncwarp();
   }
-  __syncwarp();
   // ---- everyone: wait for S (bounded; leaves early if thread 0 gave up)
   if (!mbar_wait_or_abort(&sm->bar_s, 0, abort_flag)) {
     if (*abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
@@ -247,25 +248,25 @@ decode_attn_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // ---- thread 0: O^T += V^T . P for both tiles
-  if (tid == 0 && *abort_flag == 0) {
+  // ---- warp 0: O^T += V^T . P for both tiles
+  if (warp == 0 && __all_sync(0xffffffffu, *abort_flag == 0)) {
+    const uint64_t a_desc = make_desc(smem_u32(stage), kHalfBytes, 1024, 2), b_desc = make_desc(smem_u32(p_s), 128, 2048, 0);
     bool ok = true;
     for (int i = 0; i < ntiles && ok; ++i) {
-      ok = mbar_wait(&sm->bar_v[i], 0);
+      ok = (bool)__all_sync(0xffffffffu, mbar_wait(&sm->bar_v[i], 0));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t a0 = smem_u32(stage + (i == 0 ? 2 : 0) * kStageBytes);
+      if (elect_one()) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {  // 16 tokens per MMA = 2048 bytes further down both 64-dim halves
-        const uint64_t ad = make_desc(a0 + k * 2048, kHalfBytes, 1024, 2);
-        const uint64_t bd = make_desc(smem_u32(p_s + i * kPBytes) + k * 256, 128, 2048, 0);
-        umma(tmem + 32, ad, bd, idesc_pv, (i > 0 || k > 0));
+        for (int k = 0; k < 8; ++k)  // 16 tokens per MMA = 2048 bytes further down both 64-dim halves
+          umma(tm + 32, a_desc + (i == 0 ? 2 : 0) * (kStageBytes >> 4) + k * 128, b_desc + i * (kPBytes >> 4) + k * 16, idesc_pv, (i > 0 || k > 0));
+        if (i == ntiles - 1) umma_commit(&sm->bar_o);
       }
+      __syncwarp();
     }
-    if (ok) umma_commit(&sm->bar_o);
-    else { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+    if (!ok && lane == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+    __syncwarp();
   }
-  __syncwarp();
   bool have_o = *abort_flag == 0 && mbar_wait_or_abort(&sm->bar_o, 0, abort_flag);
   if (!have_o && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
   tc_fence_after();

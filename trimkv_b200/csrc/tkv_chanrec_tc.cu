@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kCtThreads, 1) chanrec_tc_kernel(ChanrecParams
   extern __shared__ __align__(1024) uint8_t base[];
   grid_dependency_wait();
   grid_launch_dependents();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int ptiles = (a.p + kCtP - 1) / kCtP, per_seg = a.batch * a.heads * ptiles;
   const int seg = blockIdx.x / per_seg, item = blockIdx.x - seg * per_seg;      // kStateOnly: a piece of a segment
   const int pt = item % ptiles, bh = item / ptiles, b = bh / a.heads, h = bh - b * a.heads;
@@ -375,17 +375,17 @@ __global__ void __launch_bounds__(kCtThreads, 1) chanrec_tc_kernel(ChanrecParams
         dst += 2 * out_row;
       }
     };
+    const uint32_t tm = warp_uniform(tmem);
     const uint32_t id_o = ct_idesc(kCtTok, 0, 0), id_a = ct_idesc(kCtTok, 1, 0), id_s = ct_idesc(kCtN, 1, 1);
     // descriptors of the first stage; another place is the address field (16-byte units) moved on
     const uint64_t d_sop = make_desc(smem_u32(sop_s), 16, 1024, 2), d_q = make_desc(smem_u32(op_s), 16, 1024, 2);
     const uint64_t d_k = make_desc(smem_u32(op_s) + kCtTile, kCtHalf, 1024, 2), d_v = make_desc(smem_u32(v_s), kCtHalf, 1024, 2);
-    auto products = [&](int i, int vst) {                  // one thread, once the chunk's operands and the state's are there
-      tc_fence_after();
+    auto products = [&](int i, int vst) {                  // the elected lane, once the chunk's operands and the state's are there
       const uint64_t q = d_q + (i & 1) * (kCtStage >> 4), k = d_k + (i & 1) * (kCtStage >> 4), v = d_v + vst * (kCtTile >> 4), at = q + (3 * kCtTile >> 4);
-      const uint32_t o = tmem + kCtO + (i & 1) * kCtTok;
+      const uint32_t o = tm + kCtO + (i & 1) * kCtTok;
 #pragma unroll
       for (int e = 0; e < 4; ++e)                          // high and low part of k R, 16 tokens each
-        umma(tmem + kCtSt, v + (e & 1) * 128, k + (e >> 1) * (kCtTile >> 4) + (e & 1) * 128, id_s, 1);
+        umma(tm + kCtSt, v + (e & 1) * 128, k + (e >> 1) * (kCtTile >> 4) + (e & 1) * 128, id_s, 1);
       if (!kStateOnly) {
 #pragma unroll
         for (int e = 0; e < 16; ++e)
@@ -438,7 +438,8 @@ __global__ void __launch_bounds__(kCtThreads, 1) chanrec_tc_kernel(ChanrecParams
       if (warp == 8) {
         alive = sync_on(&sm->sop, i);
         if (!alive) break;
-        if (lane == 0) products(i, vst);
+        tc_fence_after();
+        if (elect_one()) products(i, vst);
         __syncwarp();
       }
       if (!kStateOnly && i > 0) outputs(i - 1);

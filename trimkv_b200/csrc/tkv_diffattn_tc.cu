@@ -23,7 +23,7 @@ diff_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   grid_launch_dependents();
   const int seg = (int)(blockIdx.x / (unsigned)nblocks);
   const int blk = nblocks - 1 - (int)(blockIdx.x % (unsigned)nblocks);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
   const bool is_row = warp < 8;
   const int row = tid & (kDaTile - 1), half = (tid >> 7) & 1;
   const int hpg = p.heads / p.kv_heads;
@@ -67,7 +67,7 @@ diff_prefill_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   int k_issued = 0, v_issued = 0;
   bool ok = true;
   if (warp == 8) {
-    if ((tid & 31) == 0) ok = pair_products<Shape, true>(sm, base, tmem, ntiles, range);
+    ok = pair_products<Shape, true>(sm, base, tmem, ntiles, range);
     __syncwarp();
   } else if (warp == 9) {
     if ((tid & 31) == 0)

@@ -73,7 +73,7 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   GemmSmem* sm = reinterpret_cast<GemmSmem*>(base + kGemmStages * kGemmStageBytes);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
   const int n_tile = blockIdx.x / p.splits, split = blockIdx.x - n_tile * p.splits;
   const int ks0 = (int)((int64_t)split * p.k_steps / p.splits), ks1 = (int)((int64_t)(split + 1) * p.k_steps / p.splits);
   const int steps = ks1 - ks0;
@@ -163,24 +163,27 @@ skinny_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
       fence_async_smem();
       asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&sm->full_x[s])) : "memory");
     }
-  } else if (tid == 32) {
-    // ---- MMA issuer
-    const uint32_t idesc = make_idesc(p.is_bf16 ? 1 : 0, 0, 32);
+  } else if (warp == 1) {
+    // ---- MMA issuer (whole warp, elected lane)
+    const uint32_t idesc = make_idesc(p.is_bf16 ? 1 : 0, 0, 32), tm = warp_uniform(tmem);
+    const uint64_t w0 = make_desc(smem_u32(base), 16, 1024, 2);
     bool ok = true;
     for (int i = 0; i < steps && ok; ++i) {
       const int s = i % kGemmStages;
-      ok = mbar_wait_or_abort(&sm->full[s], (i / kGemmStages) & 1, abort_flag);
-      if (ok && kSwiglu) ok = mbar_wait_or_abort(&sm->full_x[s], (i / kGemmStages) & 1, abort_flag);
+      ok = warp_wait(&sm->full[s], (i / kGemmStages) & 1, abort_flag);
+      if (ok && kSwiglu) ok = warp_wait(&sm->full_x[s], (i / kGemmStages) & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
-      const uint32_t wa = smem_u32(base + s * kGemmStageBytes), xa = wa + kGemmWBytes;
+      if (elect_one()) {
+        const uint64_t w = w0 + (uint32_t)s * (kGemmStageBytes >> 4);
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        umma(tmem, make_desc(wa + k * 32, 16, 1024, 2), make_desc(xa + k * 32, 16, 1024, 2), idesc, (i > 0 || k > 0));
-      umma_commit(&sm->empty[s]);   // the stage may be refilled once these MMAs have read it
+        for (int k = 0; k < 4; ++k) umma(tm, w + k * 2, w + (kGemmWBytes >> 4) + k * 2, idesc, (i > 0 || k > 0));
+        umma_commit(&sm->empty[s]);   // the stage may be refilled once these MMAs have read it
+        if (i == steps - 1) umma_commit(&sm->done);
+      }
+      __syncwarp();
     }
-    if (ok && steps > 0) umma_commit(&sm->done);
-    else if (!ok && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+    if (!ok && tid == 32 && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
   }
   __syncwarp();
   // ---- epilogue: lane = weight row of the tile, 32 TMEM columns = activation rows

@@ -26,7 +26,7 @@ two_part_prefill_kernel(const __grid_constant__ CUtensorMap map_k1, const __grid
   grid_launch_dependents();
   const int seg = (int)(blockIdx.x / (unsigned)nblocks);
   const int blk = nblocks - 1 - (int)(blockIdx.x % (unsigned)nblocks);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
   const bool is_row = warp < 8;
   const int row = tid & (kDaTile - 1), t = (tid >> 7) & 1;
   const int b = seg / p.heads, head = seg - b * p.heads;
@@ -80,7 +80,7 @@ two_part_prefill_kernel(const __grid_constant__ CUtensorMap map_k1, const __grid
   int k_issued = 0, v_issued = 0;
   bool ok = true;
   if (warp == 8) {
-    if ((tid & 31) == 0) ok = pair_products<Shape, true>(sm, base, tmem, ntiles, range);
+    ok = pair_products<Shape, true>(sm, base, tmem, ntiles, range);
     __syncwarp();
   } else if (warp == 9) {
     if ((tid & 31) == 0)
@@ -145,7 +145,7 @@ two_part_one_kernel(const __grid_constant__ CUtensorMap map_k1, const __grid_con
   grid_launch_dependents();
   const int seg = (int)(blockIdx.x / (unsigned)nblocks);
   const int blk = nblocks - 1 - (int)(blockIdx.x % (unsigned)nblocks);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
   const bool is_ctrl = warp == 8;
   const int row = tid & (kDaTile - 1), half = (tid >> 7) & 1;
   const int b = seg / p.heads, head = seg - b * p.heads;
@@ -181,13 +181,11 @@ two_part_one_kernel(const __grid_constant__ CUtensorMap map_k1, const __grid_con
     for (int hh = 0; hh < K1; ++hh) tma_load_3d(k_s + st * kTileK + hh * kDaHalf, &map_k1, &sm->bar_k[st], hh * 64, head, kv0 + s * kDaTile);
 #pragma unroll
     for (int hh = 0; hh < K2; ++hh) tma_load_3d(k_s + st * kTileK + (K1 + hh) * kDaHalf, &map_k2, &sm->bar_k[st], hh * 64, 0, kv0 + s * kDaTile);
-    ++k_issued;
   };
   auto load_v = [&](int s) {
     mbar_expect_tx(&sm->bar_v, kTileV);
 #pragma unroll
     for (int hh = 0; hh < VH; ++hh) tma_load_3d(v_s + hh * kDaHalf, &map_v, &sm->bar_v, hh * 64, head, kv0 + s * kDaTile);
-    ++v_issued;
   };
   if (tid == kDaSoftmaxThreads) {
     for (int i = 0; i < 2; ++i) { mbar_init(&sm->bar_k[i], 1); mbar_init(&sm->bar_s[i], 1); }
@@ -200,6 +198,8 @@ two_part_one_kernel(const __grid_constant__ CUtensorMap map_k1, const __grid_con
     load_k(0);                                             // steps >= 1
     if (steps > 1) load_k(1);
     load_v(0);
+    k_issued = min(2, steps);
+    v_issued = 1;
   }
   __syncwarp();
   if (is_ctrl) {
@@ -224,47 +224,61 @@ two_part_one_kernel(const __grid_constant__ CUtensorMap map_k1, const __grid_con
   const uint32_t tmem = sm->tmem_base;
 
   if (is_ctrl) {
-    if (tid == kDaSoftmaxThreads) {
+    // whole warp, elected lane
+    {
+      const uint32_t tm = warp_uniform(tmem);
+      const int n_steps = warp_uniform(steps);
       const uint32_t idesc_s = pair_idesc<true>(128, 0), idesc_pv = pair_idesc<true>(VH * 64, 1);
-      const uint32_t p_addr = smem_u32(p_s), q_addr = smem_u32(q_s), v_addr = smem_u32(v_s);
+      const uint64_t q_desc = make_desc(smem_u32(q_s), 16, 1024, 2), p_desc = make_desc(smem_u32(p_s), 16, 1024, 2),
+                     k_desc = make_desc(smem_u32(k_s), 16, 1024, 2), v_desc = make_desc(smem_u32(v_s), kDaHalf, 1024, 2);
       auto issue_s = [&](int s) -> bool {
-        if (!mbar_wait_or_abort(&sm->bar_k[s & 1], (s >> 1) & 1, abort_flag)) return false;
+        if (!warp_wait(&sm->bar_k[s & 1], (s >> 1) & 1, abort_flag)) return false;
         tc_fence_after();
-        const uint32_t k_addr = smem_u32(k_s + (s & 1) * kTileK);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < KH * 4; ++k) {
-          const uint32_t off = (k >> 2) * kDaHalf + (k & 3) * 32;
-          umma(tmem + 128 * (s & 1), make_desc(q_addr + off, 16, 1024, 2), make_desc(k_addr + off, 16, 1024, 2), idesc_s, k > 0);
+          for (int k = 0; k < KH * 4; ++k) {
+            const uint32_t off = (k >> 2) * (kDaHalf >> 4) + (k & 3) * 2;
+            umma(tm + 128 * (s & 1), q_desc + off, k_desc + (s & 1) * (kTileK >> 4) + off, idesc_s, k > 0);
+          }
+          umma_commit(&sm->bar_s[s & 1]);
         }
-        umma_commit(&sm->bar_s[s & 1]);
+        __syncwarp();
         return true;
       };
       bool ok = issue_s(0);
-      for (int s = 0; s < steps && ok; ++s) {
+      for (int s = 0; s < n_steps && ok; ++s) {
         // the S buffer and the K stage of step s + 1 were last used by step s - 1, whose P has been waited for
-        if (s + 1 < steps) ok = issue_s(s + 1);
-        if (ok && s + 2 < steps) {                         // K two steps ahead goes where K of this step is
-          ok = mbar_wait_or_abort(&sm->bar_s[s & 1], (s >> 1) & 1, abort_flag);
-          if (ok) load_k(s + 2);
+        if (s + 1 < n_steps) ok = issue_s(s + 1);
+        if (ok && s + 2 < n_steps) {                       // K two steps ahead goes where K of this step is
+          ok = warp_wait(&sm->bar_s[s & 1], (s >> 1) & 1, abort_flag);
+          if (ok) {
+            if (elect_one()) load_k(s + 2);
+            __syncwarp();
+            ++k_issued;
+          }
         }
         if (ok && s > 0) {                                 // V of this step goes where V of the last one was
-          ok = mbar_wait_or_abort(&sm->bar_o, (s - 1) & 1, abort_flag);
-          if (ok) load_v(s);
+          ok = warp_wait(&sm->bar_o, (s - 1) & 1, abort_flag);
+          if (ok) {
+            if (elect_one()) load_v(s);
+            __syncwarp();
+            ++v_issued;
+          }
         }
-        if (ok) ok = mbar_wait_or_abort(&sm->bar_p, s & 1, abort_flag);
-        if (ok) ok = mbar_wait_or_abort(&sm->bar_v, s & 1, abort_flag);
+        if (ok) ok = warp_wait(&sm->bar_p, s & 1, abort_flag);
+        if (ok) ok = warp_wait(&sm->bar_v, s & 1, abort_flag);
         if (ok) {
           tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const uint64_t ad = make_desc(p_addr + (k >> 2) * kDaHalf + (k & 3) * 32, 16, 1024, 2);
-            const uint64_t bd = make_desc(v_addr + k * 2048, kDaHalf, 1024, 2);
-            umma(tmem + 256, ad, bd, idesc_pv, (s > 0 || k > 0));
+            for (int k = 0; k < 8; ++k)
+              umma(tm + 256, p_desc + (k >> 2) * (kDaHalf >> 4) + (k & 3) * 2, v_desc + k * 128, idesc_pv, (s > 0 || k > 0));
+            umma_commit(&sm->bar_o);
           }
-          umma_commit(&sm->bar_o);
+          __syncwarp();
         }
       }
-      if (!ok && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+      if (!ok && tid == kDaSoftmaxThreads && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
     }
     __syncwarp();
   } else {

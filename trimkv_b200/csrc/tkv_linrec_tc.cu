@@ -86,7 +86,7 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   extern __shared__ __align__(1024) uint8_t base[];
   grid_dependency_wait();
   grid_launch_dependents();
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   const int ptiles = (a.p + kLtP - 1) / kLtP, per_seg = a.batch * a.heads * ptiles;
   const int seg = blockIdx.x / per_seg, item = blockIdx.x - seg * per_seg;
   const int pt = item % ptiles, bh = item / ptiles, b = bh / a.heads, h = bh - b * a.heads, g = h / (a.heads / a.groups);
@@ -120,12 +120,10 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       if (!kStateOnly) tma_load_3d(q_s + hh * kLtHalf, &map_q, &sm->bar_qk, hh * 64, g, row);
       tma_load_3d(k_s + hh * kLtHalf, &map_k, &sm->bar_qk, hh * 64, g, row);
     }
-    ++qk_issued;
   };
   auto load_v = [&](int i) {
     mbar_expect_tx(&sm->bar_v[i & 1], kLtHalf);
     tma_load_3d(v_s + (i & 1) * kLtHalf, &map_v, &sm->bar_v[i & 1], pbase, h, tok0 + t_first + i * kLtC);
-    ++v_issued;
   };
   if (tid == kLtRows) {
     mbar_init(&sm->bar_qk, 1);
@@ -136,6 +134,7 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     load_qk(0);
     load_v(0);
+    qk_issued = v_issued = 1;
   }
   __syncwarp();
   if (warp == 8) {
@@ -150,60 +149,77 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   float* const final_state = a.state + ((int64_t)a.slots[b] * a.heads + h) * np;
 
   if (warp == 8) {
-    // ------------------------------------------------------------------------------------ TMA + MMA issue (one lane)
-    if (lane == 0) {
+    // ------------------------------------------------------------------------------------ TMA + MMA issue (whole warp, elected lane)
+    {
+      const uint32_t tm = warp_uniform(tmem);
       const uint32_t id_s = lt_idesc(128, 0, 0), id_o1 = lt_idesc(2 * kLtP, 0, 1), id_o2 = lt_idesc(kLtP, 0, 1), id_st = lt_idesc(2 * kLtP, 1, 1);
-      const uint32_t qa = smem_u32(q_s), ka = smem_u32(k_s);
       // K-major operand: step k covers 16 columns; MN-major operand of 128 rows: step k covers 16 rows.
-      auto kmaj = [&](uint32_t at, int k) { return make_desc(at + (k >> 2) * kLtHalf + (k & 3) * 32, 16, 1024, 2); };
-      auto mnmaj = [&](uint32_t at, int k) { return make_desc(at + k * 2048, kLtHalf, 1024, 2); };
+      auto kmaj = [&](uint64_t at, int k) { return at + (uint32_t)(((k >> 2) * kLtHalf + (k & 3) * 32) >> 4); };
+      auto mnmaj = [&](uint64_t at, int k) { return at + k * 128; };
+      const uint64_t q_k = make_desc(smem_u32(q_s), 16, 1024, 2), k_k = make_desc(smem_u32(k_s), 16, 1024, 2), p_k = make_desc(smem_u32(p_s), 16, 1024, 2);
+      const uint64_t k_mn = make_desc(smem_u32(k_s), kLtHalf, 1024, 2), v_mn = make_desc(smem_u32(v_s), kLtHalf, 1024, 2),
+                     wv_mn = make_desc(smem_u32(wv_s), kLtHalf, 1024, 2), sp_mn = make_desc(smem_u32(sp_s), kLtHalf, 1024, 2);
       bool ok = true;
       for (int i = 0; i < nchunks && ok; ++i) {
         const int ph = i & 1;
-        ok = mbar_wait_or_abort(&sm->bar_qk, ph, abort_flag);
-        if (ok && i == nchunks - 1 && last_rows < kLtC) ok = mbar_wait_or_abort(&sm->bar_clr, 0, abort_flag);
+        ok = warp_wait(&sm->bar_qk, ph, abort_flag);
+        if (ok && i == nchunks - 1 && last_rows < kLtC) ok = warp_wait(&sm->bar_clr, 0, abort_flag);
         if (!ok) break;
         tc_fence_after();
         if (!kStateOnly) {
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) umma(tmem + kLtS, kmaj(qa, k), kmaj(ka, k), id_s, k > 0);
-          umma_commit(&sm->bar_s);
+            for (int k = 0; k < 8; ++k) umma(tm + kLtS, kmaj(q_k, k), kmaj(k_k, k), id_s, k > 0);
+            umma_commit(&sm->bar_s);
+          }
+          __syncwarp();
         }
-        ok = mbar_wait_or_abort(&sm->bar_sp, ph, abort_flag);      // the state is scaled, its operand written, chunk i - 1 finished
+        ok = warp_wait(&sm->bar_sp, ph, abort_flag);       // the state is scaled, its operand written, chunk i - 1 finished
         if (!ok) break;
         tc_fence_after();
-        if (i + 1 < nchunks) load_v(i + 1);
-        if (!kStateOnly) {
-          const uint32_t sp = smem_u32(sp_s);
+        if (elect_one()) {
+          if (!kStateOnly) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) umma(tmem + kLtO1, kmaj(qa, k), mnmaj(sp, k), id_o1, k > 0);
-          umma_commit(&sm->bar_o1);
+            for (int k = 0; k < 8; ++k) umma(tm + kLtO1, kmaj(q_k, k), mnmaj(sp_mn, k), id_o1, k > 0);
+            umma_commit(&sm->bar_o1);
+          }
+          if (i + 1 < nchunks) load_v(i + 1);
         }
-        ok = mbar_wait_or_abort(&sm->bar_wv, ph, abort_flag);
+        __syncwarp();
+        v_issued += i + 1 < nchunks;
+        ok = warp_wait(&sm->bar_wv, ph, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t wv = smem_u32(wv_s);
+        if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) umma(tmem + kLtST, mnmaj(ka, k), mnmaj(wv, k), id_st, 1);
-        umma_commit(&sm->bar_st);
+          for (int k = 0; k < 8; ++k) umma(tm + kLtST, mnmaj(k_mn, k), mnmaj(wv_mn, k), id_st, 1);
+          umma_commit(&sm->bar_st);
+        }
+        __syncwarp();
         if (i + 1 < nchunks) {                             // Q and K are free once these products have completed
-          ok = mbar_wait_or_abort(&sm->bar_st, ph, abort_flag);
-          if (ok && !kStateOnly) ok = mbar_wait_or_abort(&sm->bar_o1, ph, abort_flag);
-          if (ok) load_qk(i + 1);
+          ok = warp_wait(&sm->bar_st, ph, abort_flag);
+          if (ok && !kStateOnly) ok = warp_wait(&sm->bar_o1, ph, abort_flag);
+          if (!ok) break;
+          if (elect_one()) load_qk(i + 1);
+          __syncwarp();
+          ++qk_issued;
         }
-        if (!kStateOnly && ok) {
-          ok = mbar_wait_or_abort(&sm->bar_p, ph, abort_flag);
+        if (!kStateOnly) {
+          ok = warp_wait(&sm->bar_p, ph, abort_flag);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t pa = smem_u32(p_s), va = smem_u32(v_s + (i & 1) * kLtHalf);   // V has arrived: wV was made of it
+          if (elect_one()) {
+            const uint64_t v = v_mn + (i & 1) * (kLtHalf >> 4);    // V has arrived: wV was made of it
 #pragma unroll
-          for (int part = 0; part < 2; ++part)
+            for (int part = 0; part < 2; ++part)
 #pragma unroll
-            for (int k = 0; k < 8; ++k) umma(tmem + kLtO2, kmaj(pa + part * 2 * kLtHalf, k), mnmaj(va, k), id_o2, part > 0 || k > 0);
-          umma_commit(&sm->bar_o2);
+              for (int k = 0; k < 8; ++k) umma(tm + kLtO2, kmaj(p_k + part * 2 * (kLtHalf >> 4), k), mnmaj(v, k), id_o2, part > 0 || k > 0);
+            umma_commit(&sm->bar_o2);
+          }
+          __syncwarp();
         }
       }
-      if (!ok && *abort_flag == 0) { *abort_flag = 1; report(status, TKV_DEV_TIMEOUT); }
+      if (!ok && lane == 0 && *abort_flag == 0) { *abort_flag = 1; report(status, TKV_DEV_TIMEOUT); }
     }
     __syncwarp();
   } else if (warp == 9) {

@@ -59,7 +59,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   MgSmem* sm = reinterpret_cast<MgSmem*>(base + S * kStage);
   int32_t* off = reinterpret_cast<int32_t*>(sm + 1);      // [experts + 1]
   int32_t* tile_end = off + p.experts + 1;                // [experts]
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5), lane = tid & 31;
   volatile int* abort_flag = &sm->abort_flag;
   if (tid == 0) {
     for (int s = 0; s < S; ++s) { mbar_init(&sm->full[s], 1); mbar_init(&sm->empty[s], 1); mbar_init(&sm->full_a[s], kMgGather); }
@@ -100,25 +100,28 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
 
   if (warp == 0) {
     // ---- weights, and consecutive rows
-    if (lane == 0) {
+    {
       int it = 0;
-      bool ok = *abort_flag == 0;
+      bool ok = (bool)__all_sync(0xffffffffu, *abort_flag == 0);
       while (ok && t.next()) {
         const int boxes = kGather ? 0 : (t.rows + kMgBoxRows - 1) / kMgBoxRows;
         const uint32_t bytes = (uint32_t)boxes * kMgBoxRows * 128 + BN * kMgK * 2;
         const int wrow = t.e * p.n + t.col * BN;
         for (int k = 0; k < ksteps; ++k, ++it) {
           const int s = it % S;
-          ok = mbar_wait_or_abort(&sm->empty[s], ((it / S) & 1) ^ 1, abort_flag);
+          ok = warp_wait(&sm->empty[s], ((it / S) & 1) ^ 1, abort_flag);
           if (!ok) break;
-          uint8_t* st = base + s * kStage;
-          mbar_expect_tx(&sm->full[s], bytes);
-          tma_load_2d(st + kMgABytes, &map_w, &sm->full[s], k * kMgK, wrow);
-          for (int i = 0; i < boxes; ++i)
-            tma_load_2d(st + i * kMgBoxRows * 128, &map_a, &sm->full[s], k * kMgK, t.row0 + i * kMgBoxRows);
+          if (elect_one()) {
+            uint8_t* st = base + s * kStage;
+            mbar_expect_tx(&sm->full[s], bytes);
+            tma_load_2d(st + kMgABytes, &map_w, &sm->full[s], k * kMgK, wrow);
+            for (int i = 0; i < boxes; ++i)
+              tma_load_2d(st + i * kMgBoxRows * 128, &map_a, &sm->full[s], k * kMgK, t.row0 + i * kMgBoxRows);
+          }
+          __syncwarp();
         }
       }
-      if (!ok && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+      if (!ok && lane == 0 && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
       mg_copies = it;
     }
     __syncwarp();
@@ -161,30 +164,33 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     if (!ok && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
   } else if (warp == 1) {
     // ---- products
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc(1, 0, BN);
+    {
+      const uint32_t idesc = make_idesc(1, 0, BN), tm = warp_uniform(tmem);
+      const uint64_t a0 = make_desc(smem_u32(base), 16, 1024, 2);
       int it = 0, n = 0;
-      bool ok = *abort_flag == 0;
+      bool ok = (bool)__all_sync(0xffffffffu, *abort_flag == 0);
       while (ok && t.next()) {
         const int buf = n & 1;
-        ok = mbar_wait_or_abort(&sm->acc_empty[buf], ((n >> 1) & 1) ^ 1, abort_flag);
+        ok = warp_wait(&sm->acc_empty[buf], ((n >> 1) & 1) ^ 1, abort_flag);
         tc_fence_after();
         for (int k = 0; k < ksteps && ok; ++k, ++it) {
           const int s = it % S;
-          ok = mbar_wait_or_abort(&sm->full[s], (it / S) & 1, abort_flag);
-          if (ok && kGather) ok = mbar_wait_or_abort(&sm->full_a[s], (it / S) & 1, abort_flag);
+          ok = warp_wait(&sm->full[s], (it / S) & 1, abort_flag);
+          if (ok && kGather) ok = warp_wait(&sm->full_a[s], (it / S) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t a = smem_u32(base + s * kStage), w = a + kMgABytes;
+          if (elect_one()) {
+            const uint64_t a = a0 + (uint32_t)s * (kStage >> 4);
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
-            umma(tmem + buf * BN, make_desc(a + q * 32, 16, 1024, 2), make_desc(w + q * 32, 16, 1024, 2), idesc, (k > 0 || q > 0));
-          umma_commit(&sm->empty[s]);
+            for (int q = 0; q < 4; ++q) umma(tm + buf * BN, a + q * 2, a + (kMgABytes >> 4) + q * 2, idesc, (k > 0 || q > 0));
+            umma_commit(&sm->empty[s]);
+            if (k == ksteps - 1) umma_commit(&sm->acc_full[buf]);
+          }
+          __syncwarp();
         }
-        if (ok) umma_commit(&sm->acc_full[buf]);
         ++n;
       }
-      if (!ok && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
+      if (!ok && lane == 0 && *abort_flag == 0) { *abort_flag = 1; report(p.status, TKV_DEV_TIMEOUT); }
     }
     __syncwarp();
   } else {

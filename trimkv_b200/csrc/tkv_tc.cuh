@@ -45,6 +45,21 @@ __device__ __forceinline__ bool mbar_wait_or_abort(uint64_t* bar, uint32_t parit
   }
   return false;
 }
+// Issue of products.  The operands of tcgen05.mma live in uniform registers.  Where a whole converged warp runs the loop and
+// elect.sync picks the lane, the compiler keeps addresses and descriptors there; in a branch on the lane number it cannot know that one
+// thread is left and moves every operand across, which takes longer than the product: 8 products of 128 x 128 x 16 are issued in
+// 166 cycles against 408, alone on the SM, and in 530 beside eight busy warps.  elect.sync picks the same lane each time, so a commit
+// follows the products of its own thread.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+// A value that all lanes hold, said so that the compiler knows it.
+template <typename T> __device__ __forceinline__ T warp_uniform(T x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, const volatile int* abort_flag) {
+  return (bool)__all_sync(0xffffffffu, mbar_wait_or_abort(bar, parity, abort_flag));
+}
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
