@@ -96,3 +96,51 @@ def test_selection_of_any_scores(n, kind):
         ops.evict_select(score, pos, None, n, nseg, 7, m, m, n, kept, count, status)
         assert ops.read_status(status) == 0 and bool((count == m).all())
         assert torch.equal(kept.long(), keep)
+
+
+# few segments: clusters of 8, 4 and 2 CTAs share a segment's columns, on both sides of the numbers of segments where that changes; rows
+# of 64 bytes a slice and fewer, of a width that is no power of two, in 32 bits; uneven lengths, segments that keep everything or nothing
+@pytest.mark.gpu
+@pytest.mark.parametrize("nseg", [1, 8, 9, 37, 38, 74, 75])
+@pytest.mark.parametrize("dim,dtype", [(128, torch.bfloat16), (64, torch.float16), (32, torch.bfloat16), (8, torch.bfloat16), (96, torch.bfloat16),
+                                       (128, torch.float32), (256, torch.float32)])
+def test_slices_agree(nseg, dim, dtype):
+    g = torch.Generator(device=DEV).manual_seed(nseg + dim)
+    n, cap = 1111, 1117
+    k, v = (torch.randn(nseg * cap, dim, generator=g, device=DEV).to(dtype) for _ in range(2))
+    beta, pos = -torch.rand(nseg * cap, generator=g, device=DEV), torch.arange(cap, dtype=torch.int32, device=DEV).repeat(nseg)
+    lens = torch.randint(0, n + 1, (nseg,), generator=g, device=DEV).int()
+    lens[0] = n
+    m = torch.randint(0, n + 1, (nseg,), generator=g, device=DEV).int().clamp(max=lens)
+    m[0] = 700
+    want = []
+    for s in range(nseg):
+        at = slice(s * cap, s * cap + int(lens[s]))
+        score = beta[at] * (n + 1 - pos[at]).float()
+        keep = score.sort(descending=True, stable=True).indices[:int(m[s])].sort().values
+        want.append([t[at][keep] for t in (k, v, beta, pos)])
+    status, ln, kept = ops.new_status(DEV), lens.clone(), torch.full((nseg, n), -1, dtype=torch.int32, device=DEV)
+    ops.evict_ex(k, v, beta, pos, ln, None, nseg, nseg, cap, n + 1, n, m, kept_idx_out=kept, kept_stride=n, status=status)
+    assert ops.read_status(status) == 0 and torch.equal(ln, m)
+    for s in range(nseg):
+        for t, w in zip((k, v, beta, pos), want[s]):
+            assert torch.equal(t[s * cap:s * cap + int(m[s])], w)
+        if m[s] < lens[s]:
+            assert torch.equal(kept[s, :int(m[s])], want[s][3]), s          # a segment's positions count its rows
+
+
+# ranges of rows in turns, where there are too many segments for clusters (75 and more) and where rows do not divide into slices
+@pytest.mark.gpu
+@pytest.mark.parametrize("nseg,dim", [(74, 64), (75, 64), (130, 64), (3, 8)])
+def test_ranges_of_rows_agree(nseg, dim):
+    g = torch.Generator(device=DEV).manual_seed(nseg)
+    n, m, cap, ctas = 900, 700, 903, 4
+    k, v = (torch.randn(nseg * cap, dim, generator=g, device=DEV).bfloat16() for _ in range(2))
+    beta, pos = -torch.rand(nseg * cap, generator=g, device=DEV), torch.arange(cap, dtype=torch.int32, device=DEV).repeat(nseg)
+    keep = (beta.view(nseg, cap)[:, :n] * (n + 1 - pos[:n]).float()).sort(dim=1, descending=True, stable=True).indices[:, :m].sort(dim=1).values
+    want = [t.view(nseg, cap, -1).gather(1, keep[:, :, None].expand(-1, -1, t.numel() // (nseg * cap))) for t in (k, v, beta, pos)]
+    status, ln = ops.new_status(DEV), torch.full((nseg,), n, dtype=torch.int32, device=DEV)
+    ops.evict_multi(k, v, beta, pos, ln, None, nseg, nseg, cap, n + 1, m, m, n, ctas, ops.evict_multi_workspace(nseg, m, ctas, torch.device(DEV)), status=status)
+    assert ops.read_status(status) == 0 and bool((ln == m).all())
+    for t, w in zip((k, v, beta, pos), want):
+        assert torch.equal(t.view(nseg, cap, -1)[:, :m], w)

@@ -135,17 +135,19 @@ __device__ __forceinline__ int build_kept_list(uint32_t* keys, int n, uint32_t t
 
 // Which (row of the tile, 16-byte column of the K|V row pair) vector number u of this thread is.  Vector i = tid +
 // u*kThreads of a tile is row i / nvec, column i % nvec; when nvec divides the block size the column is fixed per
-// thread and the row advances by a constant, which saves two integer divisions per 16 bytes moved.
+// thread and the row advances by a constant, which saves two integer divisions per 16 bytes moved.  A slice of the columns: nvec of
+// them from `first` on.
 struct TileMap {
-  int r0, col0, rstep, nvec, regular;
+  int r0, col0, rstep, nvec, regular, first;
   const char* cbase;   // address of this thread's column in row 0 of the segment (regular case)
 };
 template <int kThreads>
-__device__ __forceinline__ TileMap make_tile_map(int nvec, int row_vecs, const char* kbase, const char* vbase) {
+__device__ __forceinline__ TileMap make_tile_map(int nvec, int row_vecs, const char* kbase, const char* vbase, int first = 0) {
   TileMap t;
-  t.nvec = nvec; t.regular = (kThreads % nvec) == 0;
+  t.nvec = nvec; t.regular = (kThreads % nvec) == 0; t.first = first;
   t.r0 = threadIdx.x / nvec; t.col0 = threadIdx.x - t.r0 * nvec; t.rstep = kThreads / nvec;
-  t.cbase = t.col0 < row_vecs ? kbase + (int64_t)t.col0 * 16 : vbase + (int64_t)(t.col0 - row_vecs) * 16;
+  const int col = first + t.col0;
+  t.cbase = col < row_vecs ? kbase + (int64_t)col * 16 : vbase + (int64_t)(col - row_vecs) * 16;
   return t;
 }
 template <int kThreads>
@@ -160,7 +162,7 @@ template <int kThreads>
 __device__ __forceinline__ char* tile_ptr(const TileMap& t, int u, int r, int row, int64_t row_bytes, int row_vecs,
                                           const char* kbase, const char* vbase) {
   if (t.regular) return const_cast<char*>(t.cbase) + (int64_t)row * row_bytes;
-  const int col = (int)(threadIdx.x + u * kThreads) - r * t.nvec;
+  const int col = t.first + (int)(threadIdx.x + u * kThreads) - r * t.nvec;
   return const_cast<char*>(col < row_vecs ? kbase + (int64_t)col * 16 : vbase + (int64_t)(col - row_vecs) * 16) +
          (int64_t)row * row_bytes;
 }
@@ -242,11 +244,14 @@ struct EvictParams {
                                             // holds their number minus one (the workspace is preset to 0xFF bytes)
 };
 
-template <int kThreads>
+// One CTA per segment, or a cluster of kSlices: each of its CTAs selects for itself and moves a slice of every row's columns, so that
+// few segments reach more SMs.  No CTA reads what another one moves, but for log betas and positions, which all of them read for the
+// scores: those are moved behind a barrier of the cluster, by the first CTA and the second.
+template <int kThreads, int kSlices>
 __global__ void __launch_bounds__(kThreads, 1024 / kThreads) evict_inplace_kernel(EvictParams p) {
   extern __shared__ __align__(16) uint32_t keys[];
   __shared__ SelectScratch sc;
-  const int seg = blockIdx.x;
+  const int seg = (int)blockIdx.x / kSlices, slice = (int)blockIdx.x % kSlices;
   const int n = p.seg_len[seg];
   const int m = p.keep_cnt != nullptr ? p.keep_cnt[seg] : p.m;
   if (p.keep_cnt == nullptr ? (n < p.trigger_len || n <= m) : (m >= n || m < 0)) return;
@@ -279,12 +284,13 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) evict_inplace_kerne
       keys[i] = i >= n - p.protect_last ? score_key(INFINITY)
                                         : score_key(retention_score_as(p.beta[row0 + i], p.pos[row0 + i], p.q_idx, p.score_dtype));
   }
-  __syncthreads();
+  if (kSlices > 1) asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+  else __syncthreads();
   uint32_t thresh; int n_eq_keep;
   radix_select_mth<kThreads>(keys, n, m, &sc, &thresh, &n_eq_keep);
   const int j0 = build_kept_list<kThreads>(keys, n, thresh, n_eq_keep, &sc);
   const int32_t* kept = reinterpret_cast<const int32_t*>(keys);
-  if (p.kept_idx_out != nullptr)
+  if (p.kept_idx_out != nullptr && slice == 0)
     for (int j = threadIdx.x; j < m; j += kThreads) p.kept_idx_out[(int64_t)seg * p.m + j] = kept[j];
   if (p.plan != nullptr) {
     for (int j = j0 + threadIdx.x; j < m; j += kThreads) p.plan_kept[(int64_t)seg * p.plan_stride + j] = kept[j];
@@ -308,12 +314,13 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) evict_inplace_kerne
   }
 
   // Stable in-place compaction of rows j0..m (rows before the first evicted one stay where they are).
-  const int nvec = 2 * p.row_vecs;                       // K vectors then V vectors of one token
+  const int nvec = 2 * p.row_vecs / kSlices;             // of the K vectors, then V vectors of one token (a multiple of kSlices)
   const int tile_rows = min(kThreads, (kThreads * kEvictUnroll) / nvec);
   const int64_t row_bytes = (int64_t)p.row_vecs * 16;
   char* kbase = p.k + row0 * row_bytes;
   char* vbase = p.v + row0 * row_bytes;
-  const TileMap tm = make_tile_map<kThreads>(nvec, p.row_vecs, kbase, vbase);
+  const TileMap tm = make_tile_map<kThreads>(nvec, p.row_vecs, kbase, vbase, slice * nvec);
+  const bool has_beta = slice == 0, has_pos = slice == (kSlices > 1 ? 1 : 0);
 #pragma unroll 1
   for (int jb = j0; jb < m; jb += tile_rows) {
     const int rows = min(tile_rows, m - jb);
@@ -326,8 +333,8 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) evict_inplace_kerne
     float bt = 0.f; int32_t ps = 0;
     if (threadIdx.x < rows) {
       const int src = kept[jb + threadIdx.x];
-      bt = p.beta[row0 + src];
-      ps = p.pos[row0 + src];
+      if (has_beta) bt = p.beta[row0 + src];
+      if (has_pos) ps = p.pos[row0 + src];
     }
     __syncthreads();  // every load of this tile is performed before any of its stores
 #pragma unroll
@@ -336,11 +343,11 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) evict_inplace_kerne
       if (r < rows) st16(tile_ptr<kThreads>(tm, u, r, jb + r, row_bytes, p.row_vecs, kbase, vbase), reg[u]);
     }
     if (threadIdx.x < rows) {
-      p.beta[row0 + jb + threadIdx.x] = bt;
-      p.pos[row0 + jb + threadIdx.x] = ps;
+      if (has_beta) p.beta[row0 + jb + threadIdx.x] = bt;
+      if (has_pos) p.pos[row0 + jb + threadIdx.x] = ps;
     }
   }
-  if (threadIdx.x == 0) p.seg_len[seg] = m;
+  if (slice == 0 && threadIdx.x == 0) p.seg_len[seg] = m;
 }
 
 // ---- Several CTAs per segment -------------------------------------------------------------------------------------
@@ -646,6 +653,32 @@ static int set_smem(K kernel, size_t bytes, const char* what) {
   return TKV_OK;
 }
 
+// CTAs that share a segment's columns, each with a slice of 64 bytes of a row or more: as many as leave every CTA an SM of its own, where
+// clusters of eight only find room while they are few.  us with 1, 2, 4 and 8 slices, 16-bit rows of 128 dims, the best number of threads:
+//     8 segments of  640 ->  512  12.3   9.5   8.2   7.9     2560 -> 2048  33.0  21.5  15.8  13.6     4224 -> 4096  60.9  36.6  24.8  21.2
+//    32              640 ->  512  13.6  11.2   9.7  11.0     2560 -> 2048  34.7  23.6  21.8  24.1     4224 -> 4096  62.2  38.7  38.0  43.8
+//    64              640 ->  512  14.8  13.3  13.3  14.9     2560 -> 2048  35.8  31.6  33.8  39.4     4608 -> 4096  63.7  56.3  61.7  70.4
+//    96              640 ->  512  16.4  16.6  16.6          2560 -> 2048  44.5  48.1  49.2           4608 -> 4096  80.9  89.9  92.7
+// The several CTAs per segment of tkv_evict_multi, which take turns over ranges of rows, need 34 us for 8 x (4224 -> 4096), 60 for 32, 83 for 64.
+constexpr int kEvictSliceVecs = 4;
+inline int evict_slices(int nseg, int nvec) {
+  for (int s = 8; s > 1; s /= 2)
+    if (nseg <= (s == 8 ? 8 : 148 / s) && nvec % s == 0 && nvec / s >= kEvictSliceVecs) return s;
+  return 1;
+}
+template <int kThreads, int kSlices> static int launch_inplace(const EvictParams& p, size_t smem, cudaStream_t st) {
+  int rc = set_smem(evict_inplace_kernel<kThreads, kSlices>, smem, "tkv_evict");
+  if (rc != TKV_OK) return rc;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)p.nseg * kSlices); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kSlices; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = kSlices > 1 ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, evict_inplace_kernel<kThreads, kSlices>, p);
+  return e == cudaSuccess ? TKV_OK : fail(TKV_ERR_LAUNCH, "tkv_evict: %s", cudaGetErrorString(e));
+}
+
 // Threads of a segment's CTA.  A segment is one CTA's, and its time is the latency of rounds over its keys (two selection passes and
 // the list) and of tiles of rows (load, barrier, store): the fewer threads, the more rounds and tiles; the more threads, the dearer
 // each of the barriers, and the fewer CTAs on an SM.  So few and long segments get wide CTAs, many and short ones narrow CTAs.  us with
@@ -740,22 +773,27 @@ static int evict_impl(void* k_cache, void* v_cache, float* beta_cache, int32_t* 
     p.ctas = ctas; p.tail_max = mp.tail_max; mp.plan_tail = p.plan_tail;
     mp.k = p.k; mp.v = p.v; mp.beta = p.beta; mp.pos = p.pos; mp.seg_len = seg_len; mp.cap = cap; mp.row_vecs = p.row_vecs;
     mp.ctas = ctas; mp.plan = p.plan; mp.kept = p.plan_kept; mp.kept_stride = memory_size; mp.status = status;
+  }
+  const size_t smem = (size_t)max_len * 4;
+  const int slices = evict_slices(nseg, 2 * p.row_vecs);
+  if (slices > 1) { ctas = 1; p.plan = nullptr; }          // columns shared by a cluster: faster than rows in turns (evict_slices)
+  if (ctas > 1) {
     // flags = -1 (not raised), plan = -1 (segment keeps everything), fired count = -1 (none) until the selection says
     // otherwise
     cudaError_t e = cudaMemsetAsync(workspace, 0xFF, ((size_t)nseg * ctas + 2 * (size_t)nseg + 1) * 4, (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_evict_multi: memset: %s", cudaGetErrorString(e));
   }
-  const size_t smem = (size_t)max_len * 4;
   int rc;
   if (ctas > 1) {
-    rc = set_smem(evict_inplace_kernel<kEvictThreadsPlan>, smem, "tkv_evict_multi");
-    if (rc == TKV_OK) evict_inplace_kernel<kEvictThreadsPlan><<<nseg, kEvictThreadsPlan, smem, (cudaStream_t)stream>>>(p);
+    rc = set_smem(evict_inplace_kernel<kEvictThreadsPlan, 1>, smem, "tkv_evict_multi");
+    if (rc == TKV_OK) evict_inplace_kernel<kEvictThreadsPlan, 1><<<nseg, kEvictThreadsPlan, smem, (cudaStream_t)stream>>>(p);
   } else {
     // a keep count of each segment's own is not known here: as if all rows stayed
-    rc = with_evict_threads(EvictWork::kInPlace, nseg, max_len, (int64_t)(keep_cnt ? max_len : memory_size) * head_dim * es, [&](auto threads) {
-      int r = set_smem(evict_inplace_kernel<threads.value>, smem, "tkv_evict");
-      if (r == TKV_OK) evict_inplace_kernel<threads.value><<<nseg, threads.value, smem, (cudaStream_t)stream>>>(p);
-      return r;
+    const int64_t moved = (int64_t)(keep_cnt ? max_len : memory_size) * head_dim * es;
+    rc = with_evict_threads(EvictWork::kInPlace, nseg * slices, max_len, moved, [&](auto threads) {
+      constexpr int kT = threads.value;
+      return slices == 8 ? launch_inplace<kT, 8>(p, smem, (cudaStream_t)stream) : slices == 4 ? launch_inplace<kT, 4>(p, smem, (cudaStream_t)stream)
+             : slices == 2 ? launch_inplace<kT, 2>(p, smem, (cudaStream_t)stream) : launch_inplace<kT, 1>(p, smem, (cudaStream_t)stream);
     });
   }
   if (rc != TKV_OK) return rc;
