@@ -130,14 +130,15 @@ def tkv_attention_forward(
             return _ragged_causal(query, key, value, head_lens, scaling), None, None
         return _dense_causal(query, key, value, scaling), None, None
 
-    q3 = query[:, :, 0, :]
-    out = torch.empty(bsz, 1, hq, dim, dtype=query.dtype, device=query.device)
+    q3 = query.select(2, 0)
+    out = query.new_empty(bsz, 1, hq, dim)
     if key.dim() == 4:
         # Strided views of the capacity-strided cache: the segment stride is the capacity.
-        hkv, max_len = key.shape[1], key.shape[2]
-        if key.stride(3) != 1 or key.stride(2) != dim or key.stride(0) != hkv * key.stride(1):
+        _, hkv, max_len, _ = key.shape
+        sb, sh, ss, sd = key.stride()
+        if sd != 1 or ss != dim or sb != hkv * sh:
             raise ValueError("key is not a view of a capacity-strided cache")
-        cap, seg_start = key.stride(1) // dim, None
+        cap, seg_start = sh // dim, None
     else:
         # Packed [sum n, D] layout of the reference's flat caches: segment starts are cu_seqlens_k.
         hkv = flash_attn_kwargs.get("num_kv_heads") or head_lens.shape[0] // bsz

@@ -60,6 +60,18 @@ class _LayerViews:
             yield self[i]
 
 
+class _Layer:
+    """A layer's part of the slabs, and K, V, log beta and positions with the batch and the heads as axes.  Made once with the slabs:
+    a step for one token hands these out again instead of indexing and reshaping a dozen tensors per layer."""
+
+    __slots__ = ("k", "v", "beta", "pos", "len", "cu", "by_head")
+
+    def __init__(self, slab: Dict[str, torch.Tensor], l: int, batch: int, hkv: int, cap: int):
+        self.k, self.v, self.beta, self.pos, self.len, self.cu = (slab[kind][l] for kind in ("k", "v", "beta", "pos", "len", "cu"))
+        self.by_head = {kind: t.view(batch, hkv, cap, *t.shape[1:])
+                        for kind, t in (("k", self.k), ("v", self.v), ("beta", self.beta), ("pos", self.pos))}
+
+
 class TrimKVCache:
     def __init__(
         self,
@@ -182,14 +194,10 @@ class TrimKVCache:
             return {"k": k, "v": v, "beta": beta, "pos": pos}[kind]
         if self._slab is None:  # skipped layer that never received data (cache_utils.py:82-88)
             return torch.tensor([])
-        n, s = self._cache_len[l], self._slab
-        if self.static_views:
-            n = self._cap
-        if kind == "k" or kind == "v":
-            return s[kind][l].view(self._batch, self._hkv, self._cap, self._dim)[:, :, :n]
-        if kind == "beta" or kind == "pos":
-            return s[kind][l].view(self._batch, self._hkv, self._cap)[:, :, :n]
-        return s[kind][l]
+        layer = self._slab["layers"][l]
+        if kind == "len" or kind == "cu":
+            return getattr(layer, kind)
+        return layer.by_head[kind].narrow(2, 0, self._cap if self.static_views else self._cache_len[l])
 
     # ------------------------------------------------------------------ update (cache_utils.py:62-110)
     def update(
@@ -240,12 +248,15 @@ class TrimKVCache:
                     if torch.cuda.is_current_stream_capturing():
                         raise RuntimeError("cache capacity exhausted during CUDA graph capture")
                     self._grow(self._cache_len[layer_idx] + seq_len)
-                s = self._slab
-                ops.append(s["k"][layer_idx], s["v"][layer_idx], s["beta"][layer_idx], s["pos"][layer_idx],
-                           s["len"][layer_idx], s["cu"][layer_idx], key_states, value_states, retention_weights,
+                at = self._slab["layers"][layer_idx]
+                ops.append(at.k, at.v, at.beta, at.pos, at.len, at.cu, key_states, value_states, retention_weights,
                            cache_positions, self._cap, self._status)
                 self._cache_len[layer_idx] += seq_len
                 self.n_seen_tokens[layer_idx] += seq_len
+                n = self._cap if self.static_views else self._cache_len[layer_idx]
+                rows = at.by_head
+                return (rows["k"].narrow(2, 0, n), rows["v"].narrow(2, 0, n), rows["beta"].narrow(2, 0, n),
+                        rows["pos"].narrow(2, 0, n), self._attn_kwargs(layer_idx))
         return (self.key_cache[layer_idx], self.value_cache[layer_idx], self.retention_weights[layer_idx],
                 self.kv_positions[layer_idx], self._attn_kwargs(layer_idx))
 
@@ -262,10 +273,9 @@ class TrimKVCache:
             self._grow(self._cache_len[layer_idx] + 1)
         if layer_idx == 0:
             self._seen_tokens += 1
-        s = self._slab
+        at = self._slab["layers"][layer_idx]
         ops.decode_prep(qkvg, q_norm_w, k_norm_w, eps, cos, sin, gate_w2, gate_bias, pos, q_out,
-                        s["k"][layer_idx], s["v"][layer_idx], s["beta"][layer_idx], s["pos"][layer_idx],
-                        s["len"][layer_idx], s["cu"][layer_idx], self._cap, num_q_heads, self._hkv, self._status,
+                        at.k, at.v, at.beta, at.pos, at.len, at.cu, self._cap, num_q_heads, self._hkv, self._status,
                         in_splits, in_bias)
         self._cache_len[layer_idx] += 1
         self.n_seen_tokens[layer_idx] += 1
@@ -279,7 +289,8 @@ class TrimKVCache:
     def _attn_kwargs(self, l: int) -> Dict[str, Any]:
         if self._slab is None or self._pending[l] is not None:
             return {}
-        return {"head_lens": self._slab["len"][l], "cu_seqlens_k": self._slab["cu"][l],
+        layer = self._slab["layers"][l]
+        return {"head_lens": layer.len, "cu_seqlens_k": layer.cu,
                 "batch_size": self._batch, "num_kv_heads": self._hkv, "status": self._status,
                 "uniform_lengths": True}   # every segment of a layer has the same length in this class
 
@@ -296,6 +307,7 @@ class TrimKVCache:
             "len": torch.zeros(nl, nseg, dtype=torch.int32, device=dev),
             "cu": torch.zeros(nl, nseg + 1, dtype=torch.int32, device=dev),
         }
+        slab["layers"] = [_Layer(slab, l, self._batch, self._hkv, cap) for l in range(nl)]
         return slab
 
     def _any_pending_or_slab_device(self):
