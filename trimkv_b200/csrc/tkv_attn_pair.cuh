@@ -55,23 +55,6 @@ template <int KH_, int VH_, bool kTwoKeys_> struct PairShape {
 // Key tiles [j0, j1) of a tile of rows, counted from the CTA's first one; empty: no products, and O is not written.
 struct PairRange { int j0, j1; };
 
-// D += A . B with A in TMEM: a lane per row, two 16-bit elements of k per column.
-__device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accum) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accum), "r"(0u) : "memory");
-}
-__device__ __forceinline__ void pair_st16_nowait(uint32_t taddr, const float* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-      ::"r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-        "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-        "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-        "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15]))
-      : "memory");
-}
 // Two fp32 operations in one instruction.
 __device__ __forceinline__ float2 pair_fma2(float2 a, float2 b, float2 c) {
   float2 r;
@@ -245,7 +228,7 @@ __device__ __forceinline__ bool pair_softmax(PairSmem* sm, uint8_t* base, uint32
           tmem_ld16(o_addr + 16 * c, o);
 #pragma unroll
           for (int i = 0; i < 16; ++i) o[i] *= alpha;
-          pair_st16_nowait(o_addr + 16 * c, o);
+          tmem_st16_nowait(o_addr + 16 * c, o);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         l_sum[0] *= alpha; l_sum[1] *= alpha;
@@ -280,7 +263,7 @@ __device__ __forceinline__ bool pair_softmax(PairSmem* sm, uint8_t* base, uint32
         ls[(i >> 1) & 3] += x + y;
         w[i >> 1] = __uint_as_float(pair_pack2<kBf16>(x, y));
       }
-      pair_st16_nowait(s_addr + 16 * c, w);
+      tmem_st16_nowait(s_addr + 16 * c, w);
       if (c % 2 == 1) {                                    // half of P is there
         l_sum[c >> 1] += (ls[0] + ls[1]) + (ls[2] + ls[3]);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");

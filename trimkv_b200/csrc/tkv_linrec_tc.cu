@@ -4,7 +4,7 @@
 // One CTA walks the chunks of one (request, head, 64 columns of v, segment).  Per chunk, D in TMEM:
 //   S  [128 tok x 128 tok] = Q . K^T                     A = Q, B = K as TMA wrote them (K-major)
 //   O1 [128 tok x 2 x 64]  = Q . [S_prev high | low]     B = the state before the chunk as two bf16 parts (MN-major)
-//   O2 [128 tok x 64]      = P . V                       A = P, the weighted scores, high and low part; B = V (MN-major)
+//   O2 [128 tok x 64]      = P . V                       A = P, the weighted scores, high and low part, in TMEM over S; B = V (MN-major)
 //   ST [128 n x 2 x 64]    = e^{L_end} ST + K^T . [w V high | low]   A = K read MN-major, B = weighted values as two parts
 // A product with few columns costs what reading its 128 rows costs, so the two parts of a B operand go side by side into one
 // product of 128 columns and are added when they are read.  The state stays in TMEM as the accumulator of its own update; once per chunk its rows pass through registers to be scaled
@@ -12,8 +12,13 @@
 // rounded to 16 bits.
 //
 // Roles: warps 0-7 hold rows (TMEM lane = token, or state row; two threads per row, one per column half); warp 8 issues TMA
-// copies and MMAs (one lane); warp 9 computes the running log decays of the next chunk.  Q and K are refetched as soon as
-// the products that read them have completed, under the weighting of the scores; V has two stages.  Every wait is bounded;
+// copies and MMAs (one lane); warp 9 computes the running log decays of the next chunk.  Q, K and V have two stages.
+// What bounds it is shared memory, which the products' operands, the split parts and the outputs' scattered stores all pass through, and
+// the rows' work in turn: state, weighted values, weighted scores, outputs.  With the weights in shared memory as well, one stage of Q and
+// K, and the outputs behind their own chunk's O2, a chunk took 6500 cycles, 2000 of them waits for O2.  Now the outputs of a chunk come
+// one chunk later, behind the next one's weighted values (alone, that moved the waits elsewhere), O1 of a chunk once the outputs before
+// it have been read, and the weights go to TMEM, which makes room for the second stage.  4 x 8192 tokens of 16 heads 128 x 128: 245 -> 210
+// us; 4096 + 2731 tokens of 64 heads 128 x 64: 138 -> 117 us; 700 + 200 + 33 tokens of 48 heads: 37 -> 31 us.  Every wait is bounded;
 // on expiry the CTA records TKV_DEV_TIMEOUT, drains its copies, frees its TMEM and returns.
 #include <cuda.h>
 #include "tkv_linrec.cuh"
@@ -28,7 +33,7 @@ constexpr int kLtS = 0, kLtO1 = 128, kLtO2 = 256, kLtST = 320, kLtCols = 512;   
 
 struct LtSmem {
   float2 lv[2][kLtC];                                      // running log2 decay and value scale; by chunk parity
-  uint64_t bar_qk, bar_v[2], bar_l[2], bar_s, bar_sp, bar_o1, bar_wv, bar_st, bar_p, bar_o2, bar_clr;
+  uint64_t bar_qk[2], bar_v[2], bar_l[2], bar_s, bar_sp, bar_o1, bar_wv, bar_st, bar_p, bar_o2, bar_out, bar_clr;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -102,23 +107,23 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   const int last_rows = t_end - t_first - (nchunks - 1) * kLtC;    // live tokens of the last chunk
   const int pbase = pt * kLtP;
 
-  uint8_t* q_s = base;                                     // two 64-column halves
-  uint8_t* k_s = q_s + 2 * kLtHalf;
-  uint8_t* v_s = k_s + 2 * kLtHalf;                        // two stages
+  uint8_t* q_s = base;                                     // two stages of two 64-column halves
+  uint8_t* k_s = q_s + 4 * kLtHalf;                        // the same
+  uint8_t* v_s = k_s + 4 * kLtHalf;                        // two stages
   uint8_t* wv_s = v_s + 2 * kLtHalf;                       // high, low
   uint8_t* sp_s = wv_s + 2 * kLtHalf;                      // high, low
-  uint8_t* p_s = sp_s + 2 * kLtHalf;                       // high (two halves), low (two halves)
-  LtSmem* sm = reinterpret_cast<LtSmem*>(p_s + 4 * kLtHalf);
+  LtSmem* sm = reinterpret_cast<LtSmem*>(sp_s + 2 * kLtHalf);
   volatile int* abort_flag = &sm->abort_flag;
 
   int qk_issued = 0, v_issued = 0;
   auto load_qk = [&](int i) {
-    mbar_expect_tx(&sm->bar_qk, (kStateOnly ? 2 : 4) * kLtHalf);
-    const int row = tok0 + t_first + i * kLtC;
+    uint64_t* bar = &sm->bar_qk[i & 1];
+    mbar_expect_tx(bar, (kStateOnly ? 2 : 4) * kLtHalf);
+    const int row = tok0 + t_first + i * kLtC, at = (i & 1) * 2 * kLtHalf;
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
-      if (!kStateOnly) tma_load_3d(q_s + hh * kLtHalf, &map_q, &sm->bar_qk, hh * 64, g, row);
-      tma_load_3d(k_s + hh * kLtHalf, &map_k, &sm->bar_qk, hh * 64, g, row);
+      if (!kStateOnly) tma_load_3d(q_s + at + hh * kLtHalf, &map_q, bar, hh * 64, g, row);
+      tma_load_3d(k_s + at + hh * kLtHalf, &map_k, bar, hh * 64, g, row);
     }
   };
   auto load_v = [&](int i) {
@@ -126,10 +131,10 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     tma_load_3d(v_s + (i & 1) * kLtHalf, &map_v, &sm->bar_v[i & 1], pbase, h, tok0 + t_first + i * kLtC);
   };
   if (tid == kLtRows) {
-    mbar_init(&sm->bar_qk, 1);
-    for (int i = 0; i < 2; ++i) { mbar_init(&sm->bar_v[i], 1); mbar_init(&sm->bar_l[i], 32); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&sm->bar_qk[i], 1); mbar_init(&sm->bar_v[i], 1); mbar_init(&sm->bar_l[i], 32); }
     mbar_init(&sm->bar_s, 1); mbar_init(&sm->bar_o1, 1); mbar_init(&sm->bar_st, 1); mbar_init(&sm->bar_o2, 1);
-    mbar_init(&sm->bar_sp, kLtRows); mbar_init(&sm->bar_wv, kLtRows); mbar_init(&sm->bar_p, kLtRows); mbar_init(&sm->bar_clr, kLtRows);
+    mbar_init(&sm->bar_sp, kLtRows); mbar_init(&sm->bar_wv, kLtRows); mbar_init(&sm->bar_p, kLtRows);
+    mbar_init(&sm->bar_out, kLtRows); mbar_init(&sm->bar_clr, kLtRows);
     sm->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     load_qk(0);
@@ -156,53 +161,62 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       // K-major operand: step k covers 16 columns; MN-major operand of 128 rows: step k covers 16 rows.
       auto kmaj = [&](uint64_t at, int k) { return at + (uint32_t)(((k >> 2) * kLtHalf + (k & 3) * 32) >> 4); };
       auto mnmaj = [&](uint64_t at, int k) { return at + k * 128; };
-      const uint64_t q_k = make_desc(smem_u32(q_s), 16, 1024, 2), k_k = make_desc(smem_u32(k_s), 16, 1024, 2), p_k = make_desc(smem_u32(p_s), 16, 1024, 2);
+      const uint64_t q_k = make_desc(smem_u32(q_s), 16, 1024, 2), k_k = make_desc(smem_u32(k_s), 16, 1024, 2);
       const uint64_t k_mn = make_desc(smem_u32(k_s), kLtHalf, 1024, 2), v_mn = make_desc(smem_u32(v_s), kLtHalf, 1024, 2),
                      wv_mn = make_desc(smem_u32(wv_s), kLtHalf, 1024, 2), sp_mn = make_desc(smem_u32(sp_s), kLtHalf, 1024, 2);
       bool ok = true;
       for (int i = 0; i < nchunks && ok; ++i) {
         const int ph = i & 1;
-        ok = warp_wait(&sm->bar_qk, ph, abort_flag);
+        const uint32_t stage = ph * (2 * kLtHalf >> 4);
+        ok = warp_wait(&sm->bar_qk[ph], (i >> 1) & 1, abort_flag);
+        if (ok && !kStateOnly && i > 0) ok = warp_wait(&sm->bar_o2, ph ^ 1, abort_flag);   // S is written over the weights it read
         if (ok && i == nchunks - 1 && last_rows < kLtC) ok = warp_wait(&sm->bar_clr, 0, abort_flag);
         if (!ok) break;
         tc_fence_after();
         if (!kStateOnly) {
           if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) umma(tm + kLtS, kmaj(q_k, k), kmaj(k_k, k), id_s, k > 0);
+            for (int k = 0; k < 8; ++k) umma(tm + kLtS, kmaj(q_k + stage, k), kmaj(k_k + stage, k), id_s, k > 0);
             umma_commit(&sm->bar_s);
           }
           __syncwarp();
         }
+        if (i + 1 < nchunks) {                             // the other stage of Q and K: their products have completed
+          if (i > 0) ok = warp_wait(&sm->bar_st, ph ^ 1, abort_flag) && (kStateOnly || warp_wait(&sm->bar_o1, ph ^ 1, abort_flag));
+          if (!ok) break;
+          if (elect_one()) load_qk(i + 1);
+          __syncwarp();
+          ++qk_issued;
+        }
         ok = warp_wait(&sm->bar_sp, ph, abort_flag);       // the state is scaled, its operand written, chunk i - 1 finished
         if (!ok) break;
         tc_fence_after();
-        if (elect_one()) {
-          if (!kStateOnly) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k) umma(tm + kLtO1, kmaj(q_k, k), mnmaj(sp_mn, k), id_o1, k > 0);
-            umma_commit(&sm->bar_o1);
-          }
-          if (i + 1 < nchunks) load_v(i + 1);
+        if (kStateOnly && i + 1 < nchunks) {               // the values before are weighted
+          if (elect_one()) load_v(i + 1);
+          __syncwarp();
+          ++v_issued;
         }
-        __syncwarp();
-        v_issued += i + 1 < nchunks;
         ok = warp_wait(&sm->bar_wv, ph, abort_flag);
         if (!ok) break;
         tc_fence_after();
         if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) umma(tm + kLtST, mnmaj(k_mn, k), mnmaj(wv_mn, k), id_st, 1);
+          for (int k = 0; k < 8; ++k) umma(tm + kLtST, mnmaj(k_mn + stage, k), mnmaj(wv_mn, k), id_st, 1);
           umma_commit(&sm->bar_st);
         }
         __syncwarp();
-        if (i + 1 < nchunks) {                             // Q and K are free once these products have completed
-          ok = warp_wait(&sm->bar_st, ph, abort_flag);
-          if (ok && !kStateOnly) ok = warp_wait(&sm->bar_o1, ph, abort_flag);
+        if (!kStateOnly) {                                 // the outputs before have been read, with O1, O2 and their values
+          if (i > 0) ok = warp_wait(&sm->bar_out, ph ^ 1, abort_flag);
           if (!ok) break;
-          if (elect_one()) load_qk(i + 1);
+          tc_fence_after();
+          if (elect_one()) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) umma(tm + kLtO1, kmaj(q_k + stage, k), mnmaj(sp_mn, k), id_o1, k > 0);
+            umma_commit(&sm->bar_o1);
+            if (i + 1 < nchunks) load_v(i + 1);
+          }
           __syncwarp();
-          ++qk_issued;
+          v_issued += i + 1 < nchunks;
         }
         if (!kStateOnly) {
           ok = warp_wait(&sm->bar_p, ph, abort_flag);
@@ -213,7 +227,8 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
             for (int part = 0; part < 2; ++part)
 #pragma unroll
-              for (int k = 0; k < 8; ++k) umma(tm + kLtO2, kmaj(p_k + part * 2 * (kLtHalf >> 4), k), mnmaj(v, k), id_o2, part > 0 || k > 0);
+              for (int k = 0; k < 8; ++k)
+                umma_ts(tm + kLtO2, tm + kLtS + (k >> 2) * 64 + part * 32 + (k & 3) * 8, mnmaj(v, k), id_o2, part > 0 || k > 0);
             umma_commit(&sm->bar_o2);
           }
           __syncwarp();
@@ -285,6 +300,38 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       lt_st32(st_at + kLtP, s);
     }
     const float skip = a.skip != nullptr ? a.skip[h] : 0.f;
+    // Outputs of chunk i, whose row decays by er up to its token; O1 has been waited for.
+    auto outputs = [&](int i, float er) {
+      if (!sync_on(&sm->bar_o2, i & 1)) return false;
+      tc_fence_after();
+      const uint8_t* v_t = v_s + (i & 1) * kLtHalf;
+      uint32_t o1[32], o2[32], o3[32];
+      lt_ld32_nowait(lanes + kLtO1 + half * 32, o1);
+      lt_ld32_nowait(lanes + kLtO1 + kLtP + half * 32, o3);
+      lt_ld32_nowait(lanes + kLtO2 + half * 32, o2);
+      lt_wait_ld();
+      const int t = t_first + i * kLtC + row;
+      __nv_bfloat16* dst = (__nv_bfloat16*)a.out + ((int64_t)(tok0 + t) * a.heads + h) * a.p + pbase + half * 32;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const uint4 x = ld16(v_t + lt_swz(row, half * 4 + c));
+        const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int at = c * 8 + 2 * e;
+          const float u = fmaf(er, __uint_as_float(o1[at]) + __uint_as_float(o3[at]), __uint_as_float(o2[at])) + skip * __uint_as_float(xs[e] << 16);
+          const float v = fmaf(er, __uint_as_float(o1[at + 1]) + __uint_as_float(o3[at + 1]), __uint_as_float(o2[at + 1])) + skip * __uint_as_float(xs[e] & 0xffff0000u);
+          const __nv_bfloat162 pr = __floats2bfloat162_rn(u, v);
+          w[e] = *reinterpret_cast<const uint32_t*>(&pr);
+        }
+        if (t < t_end && pbase + half * 32 + c * 8 < a.p) st16(dst + c * 8, make_uint4(w[0], w[1], w[2], w[3]));
+      }
+      tc_fence_before();
+      lt_arrive(&sm->bar_out);
+      return true;
+    };
+    float er_before = 0.f;
     bool alive = true;
     for (int i = 0; i < nchunks; ++i) {
       const int ph = i & 1;
@@ -292,11 +339,11 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       uint8_t* v_t = v_s + (i & 1) * kLtHalf;
       // ---- tokens beyond the request's end belong to another request: their keys and values read as zeros
       if (i == nchunks - 1 && last_rows < kLtC) {
-        alive = sync_on(&sm->bar_qk, ph) && sync_on(&sm->bar_v[i & 1], i >> 1);
+        alive = sync_on(&sm->bar_qk[ph], i >> 1) && sync_on(&sm->bar_v[i & 1], i >> 1);
         if (!alive) break;
         if (row >= last_rows) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) st16(k_s + half * kLtHalf + row * 128 + c * 16, make_uint4(0, 0, 0, 0));
+          for (int c = 0; c < 8; ++c) st16(k_s + (2 * ph + half) * kLtHalf + row * 128 + c * 16, make_uint4(0, 0, 0, 0));
 #pragma unroll
           for (int c = 0; c < 4; ++c) st16(v_t + row * 128 + half * 64 + c * 16, make_uint4(0, 0, 0, 0));
         }
@@ -305,7 +352,7 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       }
       // ---- the state before this chunk: operand of the read-out, then scaled for its update
       alive = sync_on(&sm->bar_l[i & 1], i >> 1);
-      if (alive && i > 0) alive = sync_on(&sm->bar_st, i - 1);
+      if (alive && i > 0) alive = sync_on(&sm->bar_st, i - 1) && (kStateOnly || sync_on(&sm->bar_o1, i - 1));
       if (!alive) break;
       tc_fence_after();
       const float lend = lv[kLtC - 1].x;
@@ -359,78 +406,49 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       fence_async_smem();
       lt_arrive(&sm->bar_wv);
       if (kStateOnly) continue;
+      // ---- outputs of the chunk before
+      if (i > 0) alive = outputs(i - 1, er_before);
+      if (!alive) break;
+      er_before = exp2_weight(l_row);
       // ---- weighted scores: this thread's 64 columns of its row
       alive = sync_on(&sm->bar_s, ph);
       if (!alive) break;
       tc_fence_after();
+      // P of the thread's columns goes over them in TMEM: 32 columns of high parts, 32 of low ones.
       const int j0 = half * 64, r0 = row & ~31;            // rows r0 .. r0 + 31 of this warp
-      uint8_t* p_hi = p_s + half * kLtHalf;
-      uint8_t* p_lo = p_hi + 2 * kLtHalf;
+      uint32_t sv[64];
+      if (j0 <= r0 + 31) {
+        lt_ld32_nowait(lanes + kLtS + j0, sv);
+        lt_ld32_nowait(lanes + kLtS + j0 + 32, sv + 32);
+        lt_wait_ld();
+      }
 #pragma unroll
       for (int c2 = 0; c2 < 2; ++c2) {
         const int jb = j0 + c2 * 32;
+        float hi[16], lo[16];
         if (jb > r0 + 31) {                                // all of it in the future (warp-uniform)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const uint32_t at = lt_swz(row, c2 * 4 + c);
-            st16(p_hi + at, make_uint4(0, 0, 0, 0));
-            st16(p_lo + at, make_uint4(0, 0, 0, 0));
-          }
-          continue;
-        }
-        uint32_t sv[32];
-        lt_ld32_nowait(lanes + kLtS + jb, sv);
-        lt_wait_ld();
+          for (int e = 0; e < 16; ++e) hi[e] = lo[e] = 0.f;
+        } else {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t hi[4], lo[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int j = jb + c * 8 + 2 * e;
+          for (int e = 0; e < 16; ++e) {
+            const int j = jb + 2 * e;
             const float4 w = *reinterpret_cast<const float4*>(&lv[j]);     // two tokens: log decay, scale
-            const float x = j <= row ? __uint_as_float(sv[c * 8 + 2 * e]) * exp2_weight(l_row - w.x) * w.y : 0.f;
-            const float y = j + 1 <= row ? __uint_as_float(sv[c * 8 + 2 * e + 1]) * exp2_weight(l_row - w.z) * w.w : 0.f;
-            lt_split(x, y, &hi[e], &lo[e]);
+            const float x = j <= row ? __uint_as_float(sv[c2 * 32 + 2 * e]) * exp2_weight(l_row - w.x) * w.y : 0.f;
+            const float y = j + 1 <= row ? __uint_as_float(sv[c2 * 32 + 2 * e + 1]) * exp2_weight(l_row - w.z) * w.w : 0.f;
+            uint32_t h, l;
+            lt_split(x, y, &h, &l);
+            hi[e] = __uint_as_float(h); lo[e] = __uint_as_float(l);
           }
-          const uint32_t at = lt_swz(row, c2 * 4 + c);
-          st16(p_hi + at, make_uint4(hi[0], hi[1], hi[2], hi[3]));
-          st16(p_lo + at, make_uint4(lo[0], lo[1], lo[2], lo[3]));
         }
+        tmem_st16_nowait(lanes + kLtS + j0 + 16 * c2, hi);
+        tmem_st16_nowait(lanes + kLtS + j0 + 32 + 16 * c2, lo);
       }
-      fence_async_smem();
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       tc_fence_before();
       lt_arrive(&sm->bar_p);
-      // ---- output
-      alive = sync_on(&sm->bar_o1, ph) && sync_on(&sm->bar_o2, ph);
-      if (!alive) break;
-      tc_fence_after();
-      {
-        uint32_t o1[32], o2[32], o3[32];
-        lt_ld32_nowait(lanes + kLtO1 + half * 32, o1);
-        lt_ld32_nowait(lanes + kLtO1 + kLtP + half * 32, o3);
-        lt_ld32_nowait(lanes + kLtO2 + half * 32, o2);
-        lt_wait_ld();
-        const float er = exp2_weight(l_row);
-        const int t = t_first + i * kLtC + row;
-        __nv_bfloat16* dst = (__nv_bfloat16*)a.out + ((int64_t)(tok0 + t) * a.heads + h) * a.p + pbase + half * 32;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const uint4 x = ld16(v_t + lt_swz(row, half * 4 + c));
-          const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
-          uint32_t w[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int at = c * 8 + 2 * e;
-            const float u = fmaf(er, __uint_as_float(o1[at]) + __uint_as_float(o3[at]), __uint_as_float(o2[at])) + skip * __uint_as_float(xs[e] << 16);
-            const float v = fmaf(er, __uint_as_float(o1[at + 1]) + __uint_as_float(o3[at + 1]), __uint_as_float(o2[at + 1])) + skip * __uint_as_float(xs[e] & 0xffff0000u);
-            const __nv_bfloat162 pr = __floats2bfloat162_rn(u, v);
-            w[e] = *reinterpret_cast<const uint32_t*>(&pr);
-          }
-          if (t < t_end && pbase + half * 32 + c * 8 < a.p) st16(dst + c * 8, make_uint4(w[0], w[1], w[2], w[3]));
-        }
-      }
-      tc_fence_before();
     }
+    if (alive && !kStateOnly) alive = sync_on(&sm->bar_o1, nchunks - 1) && outputs(nchunks - 1, er_before);
     if (alive) alive = sync_on(&sm->bar_st, nchunks - 1);
     if (alive) {
       tc_fence_after();
@@ -455,7 +473,7 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   __syncthreads();
   // An aborting CTA drains the copies it started before its shared memory is released.
   if (tid == kLtRows && *abort_flag != 0) {
-    if (qk_issued > 0) mbar_wait(&sm->bar_qk, (qk_issued - 1) & 1);
+    for (int i = max(0, qk_issued - 2); i < qk_issued; ++i) mbar_wait(&sm->bar_qk[i & 1], (i >> 1) & 1);
     for (int i = max(0, v_issued - 2); i < v_issued; ++i) mbar_wait(&sm->bar_v[i & 1], (i >> 1) & 1);
   }
   __syncthreads();
