@@ -10,6 +10,7 @@
 //   linrec_scan_kernel     : any number of tokens, one after the other, state in shared memory.
 // A request whose start position is 0 starts from the zero state whatever its slot held before.  The state is fp32 and
 // is read and written once per step; its 8 n p bytes per head are what a decode step costs.
+#include <algorithm>
 #include "tkv_linrec.cuh"
 #include "tkv_state_step.cuh"
 
@@ -280,6 +281,125 @@ __global__ void __launch_bounds__(kStepThreads, 4) ssd_step_kernel(const T* proj
   for (int i = threadIdx.x; i < vdim; i += kStepThreads) dst[i] = from_f32<T>(fmaf(sk, x[i], o[i]));
 }
 
+// Several heads of a group per CTA, for many heads.  A head's CTA of its own computes the convolution of B and C again and spends most of
+// its instructions (1200 a warp, 32 state elements a thread) outside the state's update: it was bound by issue and latency, a quarter of
+// DRAM's rate under ncu.  Here B and C are made once for `per` heads, the next head's state is requested before the current one is
+// updated, and read-outs are summed once at the end.  Sums are taken in the order of ssd_step_kernel: the results are the same.
+// 256 threads; columns in vectors of 4, vdim / 4 a divisor of 256, at most kGroupRows rows of the state per thread.
+constexpr int kGroupRows = 8;
+template <typename T>
+__global__ void __launch_bounds__(kStepThreads, 2) ssd_group_step_kernel(const T* proj, int64_t row_stride, T* ring, float* state,
+                                                                     const int32_t* slots, const int32_t* pos0, const float* conv_w,
+                                                                     const float* conv_b, const float* dt_bias, const float* a_log,
+                                                                     const float* skip, T* out, int heads, int groups, int n, int vdim,
+                                                                     int taps, int parts, int per) {
+  extern __shared__ float4 sm4[];
+  float4* red = sm4;                                       // [per][kStepThreads]
+  float *q = reinterpret_cast<float*>(red + per * kStepThreads), *k = q + n, *x = k + n, *dt = x + per * vdim, *decay = dt + per;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const int part = blockIdx.x % parts, bg = blockIdx.x / parts, b = bg / groups, g = bg - b * groups;
+  const int hpg = heads / groups, h0 = g * hpg + part * per, hc = min(per, hpg - part * per);
+  if (hc <= 0) return;
+  const int pos = pos0[b], slot = slots[b], inner = heads * vdim, channels = inner + 2 * groups * n;
+  const int cb = vdim / 4, rows = kStepThreads / cb, r = threadIdx.x / cb, c = threadIdx.x - r * cb;
+  float* S = state + ((int64_t)slot * heads + h0) * n * vdim + (int64_t)r * vdim + c * 4;
+  const int64_t head_step = (int64_t)n * vdim, row_step = (int64_t)rows * vdim;
+  float4 s[2][kGroupRows];
+  auto load = [&](int buf, int i) {
+#pragma unroll
+    for (int u = 0; u < kGroupRows; ++u)
+      s[buf][u] = pos != 0 && r + u * rows < n ? *reinterpret_cast<const float4*>(S + i * head_step + u * row_step) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  load(0, 0);
+  if (hc > 1) load(1, 1);
+  const T* cur = proj + (int64_t)b * row_stride + inner;
+  T* rg = ring + (int64_t)slot * taps * channels;
+  if ((int)threadIdx.x < hc) {
+    const int h = h0 + threadIdx.x;
+    const float d = softplus_f32(to_f32<T>(cur[channels + h]) + dt_bias[h]);
+    dt[threadIdx.x] = d;
+    decay[threadIdx.x] = expf(-expf(a_log[h]) * d);
+  }
+  const int own = hc * vdim, newest = pos % taps;
+  // Two channels per thread and pass, every load requested before the first use.
+  for (int base = threadIdx.x; base < own + 2 * n; base += 2 * kStepThreads) {
+    float acc[2];
+    T in[2];
+    int chs[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = base + u * kStepThreads;
+      if (i >= own + 2 * n) continue;
+      const int ch = i < own ? h0 * vdim + i : (i < own + n ? inner + g * n + (i - own) : inner + (groups + g) * n + (i - own - n));
+      chs[u] = ch;
+      acc[u] = conv_b[ch];
+      in[u] = cur[ch];
+      if (taps == 4) {                                     // the usual number
+        const float4 w = *reinterpret_cast<const float4*>(conv_w + (int64_t)ch * 4);
+        const float x3 = pos >= 3 ? to_f32<T>(rg[(int64_t)((newest + 1) & 3) * channels + ch]) : 0.f;
+        const float x2 = pos >= 2 ? to_f32<T>(rg[(int64_t)((newest + 2) & 3) * channels + ch]) : 0.f;
+        const float x1 = pos >= 1 ? to_f32<T>(rg[(int64_t)((newest + 3) & 3) * channels + ch]) : 0.f;
+        acc[u] = fmaf(w.w, to_f32<T>(in[u]), fmaf(w.z, x1, fmaf(w.y, x2, fmaf(w.x, x3, acc[u]))));
+      } else {
+        for (int d = taps - 1; d > 0; --d)
+          if (pos - d >= 0) acc[u] = fmaf(conv_w[(int64_t)ch * taps + taps - 1 - d], to_f32<T>(rg[(int64_t)((pos - d) % taps) * channels + ch]), acc[u]);
+        acc[u] = fmaf(conv_w[(int64_t)ch * taps + taps - 1], to_f32<T>(in[u]), acc[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = base + u * kStepThreads;
+      if (i >= own + 2 * n) continue;
+      if (i < own || part == 0) rg[(int64_t)newest * channels + chs[u]] = in[u];
+      const float y = round_as<T>(silu_act<T>(acc[u]));
+      if (i < own) x[i] = y;
+      else if (i < own + n) k[i - own] = y;
+      else q[i - own - n] = y;
+    }
+  }
+  __syncthreads();
+  float kk[kGroupRows], qq[kGroupRows];
+#pragma unroll
+  for (int u = 0; u < kGroupRows; ++u) {
+    const bool in = r + u * rows < n;
+    kk[u] = in ? k[r + u * rows] : 0.f;
+    qq[u] = in ? q[r + u * rows] : 0.f;
+  }
+  auto update = [&](int buf, int i) {
+    const float a = decay[i], d = dt[i];
+    const float4 xx = *reinterpret_cast<const float4*>(x + i * vdim + c * 4);
+    const float4 v = make_float4(d * xx.x, d * xx.y, d * xx.z, d * xx.w);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < kGroupRows; ++u)
+      if (r + u * rows < n) {
+        float4 z = s[buf][u];
+        z.x = fmaf(a, z.x, kk[u] * v.x); z.y = fmaf(a, z.y, kk[u] * v.y); z.z = fmaf(a, z.z, kk[u] * v.z); z.w = fmaf(a, z.w, kk[u] * v.w);
+        acc.x = fmaf(qq[u], z.x, acc.x); acc.y = fmaf(qq[u], z.y, acc.y); acc.z = fmaf(qq[u], z.z, acc.z); acc.w = fmaf(qq[u], z.w, acc.w);
+        *reinterpret_cast<float4*>(S + i * head_step + u * row_step) = z;
+      }
+    red[i * kStepThreads + threadIdx.x] = acc;
+  };
+  for (int i = 0; i < hc; i += 2) {
+    update(0, i);
+    if (i + 2 < hc) load(0, i + 2);
+    if (i + 1 < hc) {
+      update(1, i + 1);
+      if (i + 3 < hc) load(1, i + 3);
+    }
+  }
+  __syncthreads();
+  T* dst = out + (int64_t)b * inner + (int64_t)h0 * vdim;
+  for (int j = threadIdx.x; j < own; j += kStepThreads) {
+    const int i = j / vdim;
+    const float* part_sums = reinterpret_cast<const float*>(red + i * kStepThreads) + (j - i * vdim);
+    float o = 0.f;
+    for (int e = 0; e < rows; ++e) o += part_sums[e * vdim];
+    dst[j] = from_f32<T>(fmaf(skip[h0 + i], x[j], o));
+  }
+}
+
 // ---------------------------------------------------------------------------------------------- scan, token by token
 constexpr int kScanWarps = 8;
 
@@ -446,6 +566,21 @@ extern "C" int tkv_ssd_step(const void* proj, int64_t row_stride, void* ring, fl
     return fail(TKV_ERR_ARG, "tkv_ssd_step: bad sizes");
   if (batch == 0) return TKV_OK;
   const size_t smem = ((size_t)2 * n + 3 * vdim + kStepThreads * 4) * sizeof(float);
+  // As few CTAs per group as fill two on every SM; a head's own CTA where that leaves one head each.
+  const int hpg = heads / groups, cb = vdim / 4;
+  const int64_t pairs = (int64_t)batch * groups;
+  const int parts = pairs >= 296 ? 1 : (int)std::min<int64_t>(hpg, 296 / pairs), per = (hpg + parts - 1) / parts;
+  const size_t group_smem = (size_t)per * (kStepThreads * 16 + (vdim + 2) * 4) + (size_t)n * 8;
+  if (per > 1 && vdim % 4 == 0 && cb <= kStepThreads && kStepThreads % cb == 0 && n <= kGroupRows * (kStepThreads / cb) && n % 4 == 0 &&
+      group_smem <= 100 * 1024 && ((uintptr_t)state & 15) == 0) {
+    TKV_WITH_TYPE(dtype, T, {
+      if (!allow_smem(ssd_group_step_kernel<T>, group_smem)) return fail(TKV_ERR_UNSUPPORTED, "tkv_ssd_step: n=%d vdim=%d", n, vdim);
+      TKV_CHECK_LAUNCH(launch_pdl(ssd_group_step_kernel<T>, dim3((unsigned)(pairs * parts)), dim3(kStepThreads), group_smem, (cudaStream_t)stream,
+                                  (const T*)proj, row_stride, (T*)ring, state, slots, pos0, conv_w, conv_b, dt_bias, a_log, skip, (T*)out,
+                                  heads, groups, n, vdim, taps, parts, per), "tkv_ssd_step");
+    });
+    return check_launch("tkv_ssd_step");
+  }
   TKV_WITH_TYPE(dtype, T, {
     auto kern = vdim % 4 == 0 ? ssd_step_kernel<T, 4> : ssd_step_kernel<T, 1>;
     if (!allow_smem(kern, smem)) return fail(TKV_ERR_UNSUPPORTED, "tkv_ssd_step: n=%d vdim=%d", n, vdim);
