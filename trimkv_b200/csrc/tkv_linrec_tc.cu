@@ -7,18 +7,21 @@
 //   O2 [128 tok x 64]      = P . V                       A = P, the weighted scores, high and low part, in TMEM over S; B = V (MN-major)
 //   ST [128 n x 2 x 64]    = e^{L_end} ST + K^T . [w V high | low]   A = K read MN-major, B = weighted values as two parts
 // A product with few columns costs what reading its 128 rows costs, so the two parts of a B operand go side by side into one
-// product of 128 columns and are added when they are read.  The state stays in TMEM as the accumulator of its own update; once per chunk its rows pass through registers to be scaled
-// and to be written as the operand of O1.  fp32 factors of a product enter as two bf16 parts, so nothing that recurs is
+// product of 128 columns and are added when they are read.  The state stays in TMEM as the accumulator of its own update; once per chunk its rows
+// pass through registers to be scaled and to be written as the operand of O1.  fp32 factors of a product enter as two bf16 parts, so nothing that recurs is
 // rounded to 16 bits.
 //
 // Roles: warps 0-7 hold rows (TMEM lane = token, or state row; two threads per row, one per column half); warp 8 issues TMA
 // copies and MMAs (one lane); warp 9 computes the running log decays of the next chunk.  Q, K and V have two stages.
-// What bounds it is shared memory, which the products' operands, the split parts and the outputs' scattered stores all pass through, and
-// the rows' work in turn: state, weighted values, weighted scores, outputs.  With the weights in shared memory as well, one stage of Q and
-// K, and the outputs behind their own chunk's O2, a chunk took 6500 cycles, 2000 of them waits for O2.  Now the outputs of a chunk come
+// What bounds it is shared memory, which the products' operands and the split parts all pass through, and the rows' work in turn: state,
+// weighted values, weighted scores, outputs.  With the weights in shared memory as well, one stage of Q and K, and the outputs behind
+// their own chunk's O2, a chunk took 6500 cycles, 2000 of them waits for O2.  Now the outputs of a chunk come
 // one chunk later, behind the next one's weighted values (alone, that moved the waits elsewhere), O1 of a chunk once the outputs before
-// it have been read, and the weights go to TMEM, which makes room for the second stage.  4 x 8192 tokens of 16 heads 128 x 128: 245 -> 210
-// us; 4096 + 2731 tokens of 64 heads 128 x 64: 138 -> 117 us; 700 + 200 + 33 tokens of 48 heads: 37 -> 31 us.  Every wait is bounded;
+// it have been read, and the weights go to TMEM, which makes room for the second stage: 4 x 8192 tokens of 16 heads 128 x 128 245 -> 210
+// us, 4096 + 2731 tokens of 64 heads 128 x 64 138 -> 117 us.  The outputs' 1650 cycles were 16-byte stores to rows 4 KB apart; a whole
+// chunk's now take the place of its values and leave as one copy of a tile, before the values of the next chunk but one come there: 210 ->
+// 181 us, 117 -> 103 us; 700 + 200 + 33 tokens of 48 heads 31 -> 28 us (37 at first).  Rows of a chunk that the request has only a part
+// of are stored one by one: the tile would reach into the next request.  Every wait is bounded;
 // on expiry the CTA records TKV_DEV_TIMEOUT, drains its copies, frees its TMEM and returns.
 #include <cuda.h>
 #include "tkv_linrec.cuh"
@@ -87,7 +90,7 @@ __device__ __forceinline__ void lt_split(float a, float b, uint32_t* hi, uint32_
 template <bool kStateOnly>
 __global__ void __launch_bounds__(kLtThreads, 1)
 linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                 LinrecParams a, LinrecSegs sg, int32_t* status) {
+                 const __grid_constant__ CUtensorMap map_o, LinrecParams a, LinrecSegs sg, int32_t* status) {
   extern __shared__ __align__(1024) uint8_t base[];
   grid_dependency_wait();
   grid_launch_dependents();
@@ -213,6 +216,10 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
             for (int k = 0; k < 8; ++k) umma(tm + kLtO1, kmaj(q_k + stage, k), mnmaj(sp_mn, k), id_o1, k > 0);
             umma_commit(&sm->bar_o1);
+            if (i > 0) {                                   // the outputs of a whole chunk stand where its values stood
+              tma_store_3d(&map_o, v_s + ((i - 1) & 1) * kLtHalf, pbase, h, tok0 + t_first + (i - 1) * kLtC);
+              tma_store_read();
+            }
             if (i + 1 < nchunks) load_v(i + 1);
           }
           __syncwarp();
@@ -234,6 +241,13 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           __syncwarp();
         }
       }
+      if (!kStateOnly && ok && last_rows == kLtC) {
+        ok = warp_wait(&sm->bar_out, (nchunks - 1) & 1, abort_flag);
+        if (ok && elect_one()) tma_store_3d(&map_o, v_s + ((nchunks - 1) & 1) * kLtHalf, pbase, h, tok0 + t_first + (nchunks - 1) * kLtC);
+        __syncwarp();
+      }
+      if (!kStateOnly && elect_one()) tma_store_done();
+      __syncwarp();
       if (!ok && lane == 0 && *abort_flag == 0) { *abort_flag = 1; report(status, TKV_DEV_TIMEOUT); }
     }
     __syncwarp();
@@ -304,7 +318,8 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     auto outputs = [&](int i, float er) {
       if (!sync_on(&sm->bar_o2, i & 1)) return false;
       tc_fence_after();
-      const uint8_t* v_t = v_s + (i & 1) * kLtHalf;
+      uint8_t* v_t = v_s + (i & 1) * kLtHalf;
+      const bool whole = i < nchunks - 1 || last_rows == kLtC;   // a part of a chunk ends where another request begins
       uint32_t o1[32], o2[32], o3[32];
       lt_ld32_nowait(lanes + kLtO1 + half * 32, o1);
       lt_ld32_nowait(lanes + kLtO1 + kLtP + half * 32, o3);
@@ -325,8 +340,10 @@ linrec_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           const __nv_bfloat162 pr = __floats2bfloat162_rn(u, v);
           w[e] = *reinterpret_cast<const uint32_t*>(&pr);
         }
-        if (t < t_end && pbase + half * 32 + c * 8 < a.p) st16(dst + c * 8, make_uint4(w[0], w[1], w[2], w[3]));
+        if (whole) st16(v_t + lt_swz(row, half * 4 + c), make_uint4(w[0], w[1], w[2], w[3]));
+        else if (t < t_end && pbase + half * 32 + c * 8 < a.p) st16(dst + c * 8, make_uint4(w[0], w[1], w[2], w[3]));
       }
+      fence_async_smem();
       tc_fence_before();
       lt_arrive(&sm->bar_out);
       return true;
@@ -505,21 +522,22 @@ int launch_linrec_tc(const LinrecParams& a, const LinrecSegs& sg, int64_t tokens
     if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_linrec_chunk(tc): %s", cudaGetErrorString(e));
     configured = true;
   }
-  CUtensorMap mq, mk, mv;
+  CUtensorMap mq, mk, mv, mo;
   int rc = make_map_3d_bf16(&mq, a.q, a.n, a.groups, tokens, a.q_stride, 64, kLtC);
   if (rc == TKV_OK) rc = make_map_3d_bf16(&mk, a.k, a.n, a.groups, tokens, a.k_stride, 64, kLtC);
   if (rc == TKV_OK) rc = make_map_3d_bf16(&mv, a.v, a.p, a.heads, tokens, a.v_stride, 64, kLtC);
+  if (rc == TKV_OK) rc = make_map_3d_bf16(&mo, a.out, a.p, a.heads, tokens, (int64_t)a.heads * a.p, 64, kLtC);
   if (rc != TKV_OK) return rc;
   const int64_t grid = (int64_t)a.batch * a.heads * ((a.p + kLtP - 1) / kLtP) * sg.count;
   if (grid > INT32_MAX) return fail(TKV_ERR_UNSUPPORTED, "tkv_linrec_chunk: %lld blocks", (long long)grid);
   cudaError_t e = cudaSuccess;
   if (sg.count > 1) {
-    e = launch_pdl(linrec_tc_kernel<true>, dim3((unsigned)grid), dim3(kLtThreads), (size_t)kLtSmemBytes, st, mq, mk, mv, a, sg, status);
+    e = launch_pdl(linrec_tc_kernel<true>, dim3((unsigned)grid), dim3(kLtThreads), (size_t)kLtSmemBytes, st, mq, mk, mv, mo, a, sg, status);
     if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_linrec_chunk(tc): %s", cudaGetErrorString(e));
     rc = launch_linrec_chain(a, sg, st);
     if (rc != TKV_OK) return rc;
   }
-  e = launch_pdl(linrec_tc_kernel<false>, dim3((unsigned)grid), dim3(kLtThreads), (size_t)kLtSmemBytes, st, mq, mk, mv, a, sg, status);
+  e = launch_pdl(linrec_tc_kernel<false>, dim3((unsigned)grid), dim3(kLtThreads), (size_t)kLtSmemBytes, st, mq, mk, mv, mo, a, sg, status);
   if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_linrec_chunk(tc): %s", cudaGetErrorString(e));
   return check_launch("tkv_linrec_chunk(tc)");
 }
