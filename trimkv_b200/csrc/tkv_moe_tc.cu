@@ -1,7 +1,7 @@
 // Grouped product of a mixture of experts on tcgen05 + TMEM, for prompts and for decoding:
 //   out[r, :] = act(a[src[r], :] . w[e]^T)   for the rows r of expert e.
 //
-// One persistent CTA per SM walks tiles of 128 rows x BN columns, expert by expert.  Per 64 columns of k the weight rows are one
+// One persistent CTA per SM walks tiles of M rows x BN columns, expert by expert.  Per 64 columns of k the weight rows are one
 // TMA box; the rows of A are TMA boxes of 32 where they are consecutive, and are gathered by four warps with cp.async where they
 // are not (TMA's own gather moves four rows per instruction and was the limit).  Rows a tile does not have are not fetched, so
 // few rows per expert cost little more than the weights.  A ring of stages feeds the MMAs; two TMEM accumulators let the
@@ -16,10 +16,12 @@ namespace tkv {
 
 constexpr int kMgGather = 128, kMgLag = 2;                // gathering threads; stages they run ahead of what they hand over
 constexpr int kMgThreads = 192;                           // warp 0: copies, warp 1: products, warps 2-5: epilogue (6-9: gathering)
-constexpr int kMgM = 128, kMgK = 64, kMgBoxRows = 32;
-constexpr int kMgABytes = kMgM * kMgK * 2;
-template <int BN> struct MgRing {
-  static constexpr int kStages = BN == 256 ? 4 : BN == 128 ? 6 : 8, kStageBytes = kMgABytes + BN * kMgK * 2;
+constexpr int kMgK = 64, kMgBoxRows = 32;
+// Tiles of M rows (64: the products still run over 128, whose other rows nobody reads), stages of SUBS x 64 columns of k.
+template <int M, int BN, int SUBS> struct MgRing {
+  static constexpr int kABox = M * kMgK * 2, kWBox = BN * kMgK * 2, kWAt = SUBS * kABox, kStageBytes = SUBS * (kABox + kWBox);
+  static constexpr int kFit = 196608 / kStageBytes, kStages = kFit < 8 ? kFit : 8;
+  static_assert(kStages >= 3 && (M == 128 || kWAt + kWBox >= 128 * kMgK * 2), "");
 };
 
 struct MgSmem {
@@ -28,12 +30,12 @@ struct MgSmem {
   uint32_t tmem_base;
   int abort_flag;
 };
-template <int BN> constexpr int mg_smem_bytes(int experts) {
-  return MgRing<BN>::kStages * MgRing<BN>::kStageBytes + (int)sizeof(MgSmem) + (2 * experts + 1) * 4;
+template <int M, int BN, int SUBS> constexpr int mg_smem_bytes(int experts) {
+  return MgRing<M, BN, SUBS>::kStages * MgRing<M, BN, SUBS>::kStageBytes + (int)sizeof(MgSmem) + (2 * experts + 1) * 4;
 }
 
 // Walks this CTA's tiles in order; every role keeps its own.
-struct MgTiles {
+template <int kMgM> struct MgTiles {
   const int32_t* off; const int32_t* tile_end;            // shared memory: [experts + 1], [experts]
   int experts, ncols, e, tile, step;
   int row0, rows, col;                                    // of the current tile
@@ -50,11 +52,12 @@ struct MgTiles {
   }
 };
 
-template <int BN, bool kGather>
+template <int kMgM, int BN, int SUBS, bool kGather>
 __global__ void __launch_bounds__(kMgThreads + (kGather ? kMgGather : 0), 1)
 moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, GroupedGemm p) {
   extern __shared__ __align__(1024) uint8_t base[];
-  constexpr int S = MgRing<BN>::kStages, kStage = MgRing<BN>::kStageBytes;
+  using Ring = MgRing<kMgM, BN, SUBS>;
+  constexpr int S = Ring::kStages, kStage = Ring::kStageBytes;
   constexpr int kTmemCols = 2 * BN;
   MgSmem* sm = reinterpret_cast<MgSmem*>(base + S * kStage);
   int32_t* off = reinterpret_cast<int32_t*>(sm + 1);      // [experts + 1]
@@ -94,9 +97,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sm->tmem_base;
-  const int ksteps = (p.k + kMgK - 1) / kMgK, ncols = (p.n + BN - 1) / BN;
+  const int pieces = (p.k + kMgK - 1) / kMgK, ksteps = (pieces + SUBS - 1) / SUBS, ncols = (p.n + BN - 1) / BN;
   int mg_copies = 0;                                      // stages whose TMA copies thread 0 has started
-  MgTiles t = {off, tile_end, p.experts, ncols, 0, (int)blockIdx.x - (int)gridDim.x, (int)gridDim.x, 0, 0, 0};
+  MgTiles<kMgM> t = {off, tile_end, p.experts, ncols, 0, (int)blockIdx.x - (int)gridDim.x, (int)gridDim.x, 0, 0, 0};
 
   if (warp == 0) {
     // ---- weights, and consecutive rows
@@ -105,7 +108,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       bool ok = (bool)__all_sync(0xffffffffu, *abort_flag == 0);
       while (ok && t.next()) {
         const int boxes = kGather ? 0 : (t.rows + kMgBoxRows - 1) / kMgBoxRows;
-        const uint32_t bytes = (uint32_t)boxes * kMgBoxRows * 128 + BN * kMgK * 2;
+        const uint32_t bytes = (uint32_t)boxes * kMgBoxRows * 128 + Ring::kWBox;      // of 64 columns
         const int wrow = t.e * p.n + t.col * BN;
         for (int k = 0; k < ksteps; ++k, ++it) {
           const int s = it % S;
@@ -113,10 +116,12 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           if (!ok) break;
           if (elect_one()) {
             uint8_t* st = base + s * kStage;
-            mbar_expect_tx(&sm->full[s], bytes);
-            tma_load_2d(st + kMgABytes, &map_w, &sm->full[s], k * kMgK, wrow);
-            for (int i = 0; i < boxes; ++i)
-              tma_load_2d(st + i * kMgBoxRows * 128, &map_a, &sm->full[s], k * kMgK, t.row0 + i * kMgBoxRows);
+            const int subs = min(SUBS, pieces - k * SUBS);
+            mbar_expect_tx(&sm->full[s], bytes * subs);
+            for (int j = 0; j < subs; ++j) tma_load_2d(st + Ring::kWAt + j * Ring::kWBox, &map_w, &sm->full[s], (k * SUBS + j) * kMgK, wrow);
+            for (int j = 0; j < subs; ++j)
+              for (int i = 0; i < boxes; ++i)
+                tma_load_2d(st + j * Ring::kABox + i * kMgBoxRows * 128, &map_a, &sm->full[s], (k * SUBS + j) * kMgK, t.row0 + i * kMgBoxRows);
           }
           __syncwarp();
         }
@@ -136,9 +141,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     int it = 0;
     bool ok = *abort_flag == 0;
     while (ok && t.next()) {
-      const __nv_bfloat16* row[8];
+      const __nv_bfloat16* row[kMgM / 16];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < kMgM / 16; ++i) {
         const int r = r0 + 16 * i;
         row[i] = r < t.rows ? (const __nv_bfloat16*)p.a + (int64_t)p.src[t.row0 + r] * p.a_stride + piece * 8 : nullptr;
       }
@@ -147,11 +152,14 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
         ok = mbar_wait_or_abort(&sm->empty[s], ((it / S) & 1) ^ 1, abort_flag);
         if (!ok) break;
         const uint32_t dst = smem_u32(base + s * kStage) + (uint32_t)r0 * 128 + swz;
-        const int bytes = k * kMgK + piece * 8 < p.k ? 16 : 0;       // the rest of the last piece of k reads as zeros
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          if (row[i] != nullptr)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + i * 16 * 128), "l"(bytes ? row[i] + k * kMgK : row[i] - piece * 8), "r"(bytes) : "memory");
+        for (int j = 0; j < SUBS; ++j) {
+          const int at = (k * SUBS + j) * kMgK, bytes = at + piece * 8 < p.k ? 16 : 0;   // the rest of the last piece of k reads as zeros
+#pragma unroll
+          for (int i = 0; i < kMgM / 16; ++i)
+            if (row[i] != nullptr)
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + j * Ring::kABox + i * 16 * 128), "l"(bytes ? row[i] + at : row[i] - piece * 8), "r"(bytes) : "memory");
+        }
         asm volatile("cp.async.commit_group;" ::: "memory");
         if (it >= kMgLag) {
           asm volatile("cp.async.wait_group %0;" ::"n"(kMgLag) : "memory");
@@ -180,9 +188,13 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
-            const uint64_t a = a0 + (uint32_t)s * (kStage >> 4);
+            const uint64_t a = a0 + (uint32_t)s * (kStage >> 4), w = a + (Ring::kWAt >> 4);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) umma(tm + buf * BN, a + q * 2, a + (kMgABytes >> 4) + q * 2, idesc, (k > 0 || q > 0));
+            for (int j = 0; j < SUBS; ++j)
+              if (j == 0 || k * SUBS + j < pieces)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                  umma(tm + buf * BN, a + j * (Ring::kABox >> 4) + q * 2, w + j * (Ring::kWBox >> 4) + q * 2, idesc, (k > 0 || j > 0 || q > 0));
             umma_commit(&sm->empty[s]);
             if (k == ksteps - 1) umma_commit(&sm->acc_full[buf]);
           }
@@ -241,38 +253,44 @@ bool moe_tc_shape(const GroupedGemm& p, int dtype) {
          p.experts <= 1024 && (int64_t)p.experts * p.n + 256 <= INT32_MAX && p.a_rows > 0;
 }
 
-template <int BN, bool kGather>
+template <int M, int BN, int SUBS, bool kGather>
 static int launch_mg(const GroupedGemm& p, int64_t tiles, cudaStream_t st) {
   CUtensorMap ma, mw;
   int rc = make_map_rows(&ma, p.a, p.k, p.a_rows, p.a_stride, kMgK, kMgBoxRows);
   if (rc == TKV_OK) rc = make_map_2d(&mw, p.w, p.k, (int64_t)p.experts * p.n, kMgK, BN, TKV_BF16);
   if (rc != TKV_OK) return rc;
-  const int bytes = mg_smem_bytes<BN>(p.experts);
+  const int bytes = mg_smem_bytes<M, BN, SUBS>(p.experts);
   static int allowed = 0;
   if (bytes > allowed) {
     if (bytes > 232448) return fail(TKV_ERR_UNSUPPORTED, "tkv_moe_gemm: experts=%d", p.experts);
-    cudaError_t e = cudaFuncSetAttribute(moe_tc_kernel<BN, kGather>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaError_t e = cudaFuncSetAttribute(moe_tc_kernel<M, BN, SUBS, kGather>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_moe_gemm: %s", cudaGetErrorString(e));
     allowed = bytes;
   }
-  cudaError_t e = launch_pdl(moe_tc_kernel<BN, kGather>, dim3((unsigned)(tiles < 148 ? tiles : 148)), dim3(kMgThreads + (kGather ? kMgGather : 0)),
-                             (size_t)bytes, st, ma, mw, p);
+  cudaError_t e = launch_pdl(moe_tc_kernel<M, BN, SUBS, kGather>, dim3((unsigned)(tiles < 148 ? tiles : 148)),
+                             dim3(kMgThreads + (kGather ? kMgGather : 0)), (size_t)bytes, st, ma, mw, p);
   if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "tkv_moe_gemm: %s", cudaGetErrorString(e));
   return check_launch("tkv_moe_gemm");
 }
-template <int BN>
+template <int M, int BN, int SUBS>
 static int launch_mg(const GroupedGemm& p, int64_t tiles, cudaStream_t st) {
-  return p.src != nullptr ? launch_mg<BN, true>(p, tiles, st) : launch_mg<BN, false>(p, tiles, st);
+  return p.src != nullptr ? launch_mg<M, BN, SUBS, true>(p, tiles, st) : launch_mg<M, BN, SUBS, false>(p, tiles, st);
 }
 
 int launch_moe_tc(const GroupedGemm& p, cudaStream_t st) {
   // the widest column tile that still gives every SM a few tiles (row tiles: about one per expert beyond whole ones)
-  const int64_t row_tiles = p.max_rows / kMgM + (p.experts < p.max_rows ? p.experts : p.max_rows);
-  auto tiles = [&](int bn) { return row_tiles * ((p.n + bn - 1) / bn); };
-  if (tiles(256) > INT32_MAX / 2) return fail(TKV_ERR_UNSUPPORTED, "tkv_moe_gemm: %lld tiles", (long long)tiles(256));
-  if (tiles(256) >= 148 * 6) return launch_mg<256>(p, tiles(256), st);
-  if (tiles(128) >= 148 * 2) return launch_mg<128>(p, tiles(128), st);
-  return launch_mg<64>(p, tiles(64), st);
+  auto tiles = [&](int m, int bn) { return (p.max_rows / m + (p.experts < p.max_rows ? p.experts : p.max_rows)) * ((p.n + bn - 1) / bn); };
+  if (tiles(64, 64) > INT32_MAX / 2) return fail(TKV_ERR_UNSUPPORTED, "tkv_moe_gemm: %lld tiles", (long long)tiles(64, 64));
+  if (tiles(128, 256) >= 148 * 6) return launch_mg<128, 256, 1>(p, tiles(128, 256), st);
+  if (tiles(128, 128) >= 148 * 2) {
+    // Few rows per expert: what counts is the weights' stream.  Tiles of 64 rows leave room for stages of 128 columns, 256 bytes of every
+    // weight row at a time and 128 KB in flight instead of 96.  us of both products, 2048 x 1536, 32 experts, 6 a token, stages of 64
+    // columns and now: 8 tokens 45 + 33 and 41 + 33, 16 tokens 47 + 41 and 41 + 39, 128 tokens 49 + 41 and 45 + 39; 4096 x 3072, 8 tokens
+    // 104 + 90 and 96 + 86.  Beyond 32 rows an expert, more and more experts would have their weights read for two tiles.
+    if (p.max_rows <= (int64_t)32 * p.experts) return launch_mg<64, 128, 2>(p, tiles(64, 128), st);
+    return launch_mg<128, 128, 1>(p, tiles(128, 128), st);
+  }
+  return launch_mg<128, 64, 1>(p, tiles(128, 64), st);
 }
 
 }  // namespace tkv
