@@ -105,6 +105,14 @@ __device__ __forceinline__ float sigmoid_f32(float x) { return 1.0f / (1.0f + ex
 __device__ __forceinline__ float silu_f32(float x) { return x / (1.0f + expf(-x)); }
 __device__ __forceinline__ float softplus_f32(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
+// a b + c of two values by one instruction, rounded as fmaf rounds.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\tfma.rn.f32x2 r, a, b, c;\n\t"
+      "mov.b64 {%0, %1}, r;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
 // SiLU and GELU of values that are then used in the model type: full precision for fp32 models, the hardware's exponential
 // and division (errors far below a 16-bit rounding) for 16-bit ones.
 template <typename T> __device__ __forceinline__ float silu_act(float x) {

@@ -93,15 +93,24 @@ __global__ void __launch_bounds__(kConvThreads, sizeof(T) == 2 && V > 1 && kTaps
   if (kTaps > 0) {
     constexpr int kT = kTaps > 0 ? kTaps : 1;
     float wt[kT][V], win[kT][V];                       // win[k]: input k places before the newest
+    if constexpr (kT == 4 && V > 1) {                  // the host has seen to the alignment of w and bias
 #pragma unroll
-    for (int k = 0; k < kT; ++k)
+      for (int e = 0; e < V; ++e) {
+        const float4 x = reinterpret_cast<const float4*>(w)[ch + e];
+        wt[3][e] = x.x; wt[2][e] = x.y; wt[1][e] = x.z; wt[0][e] = x.w;
+      }
+    } else {
 #pragma unroll
-      for (int e = 0; e < V; ++e) wt[k][e] = w[(int64_t)(ch + e) * kT + kT - 1 - k];
+      for (int k = 0; k < kT; ++k)
+#pragma unroll
+        for (int e = 0; e < V; ++e) wt[k][e] = w[(int64_t)(ch + e) * kT + kT - 1 - k];
+    }
 #pragma unroll
     for (int k = 1; k < kT; ++k) input(i0 - k, win[k - 1]);
-    // Latency would bound a token after the other: kConvAhead rows are requested at a time.  6827 tokens of 6144 channels: 48 us
-    // one at a time, 40 us so.  In fp32, with the copy into the ring, 118 and 110 us (163 registers; 144 us when the two words of a vector
-    // both went past L1).
+    // Latency would bound a token after the other: kConvAhead rows are requested at a time.  Then the instructions do: the taps of two
+    // channels go into one fused multiply-add, and a channel's weights into one load (32 scalar ones were as many as the loads and stores
+    // of a strip).  6827 tokens of 6144 channels, with the copy into the ring: 65 -> 53 us, 900 tokens of 4608 19.8 -> 17.2, fp32 106 -> 93.
+    // Five or six CTAs an SM with four rows ahead spill: 56 and 63 us; strips of 64 tokens 57 us.
     for (int ib = i0; ib < i1; ib += kConvAhead) {
       RawVec<T, V> ahead[kConvAhead];
 #pragma unroll
@@ -117,11 +126,12 @@ __global__ void __launch_bounds__(kConvThreads, sizeof(T) == 2 && V > 1 && kTaps
         ahead[u].floats(win[0]);
         float acc[V];
 #pragma unroll
-        for (int e = 0; e < V; ++e) {
-          acc[e] = bs[e];
+        for (int e = 0; e < V; e += 2) {
+          float2 x = make_float2(bs[e], bs[(e + 1) % V]);
 #pragma unroll
-          for (int k = kT - 1; k >= 0; --k) acc[e] = fmaf(wt[k][e], win[k][e], acc[e]);
-          acc[e] = silu_act<T>(acc[e]);
+          for (int k = kT - 1; k >= 0; --k) x = fma2(make_float2(wt[k][e], wt[k][(e + 1) % V]), make_float2(win[k][e], win[k][(e + 1) % V]), x);
+          acc[e] = silu_act<T>(x.x);
+          if (V > 1) acc[(e + 1) % V] = silu_act<T>(x.y);
         }
         store_vec<V>(out + (int64_t)(t0 + ib + u) * channels + ch, acc);
       }
@@ -505,7 +515,7 @@ extern "C" int tkv_conv_silu(const void* proj, int64_t row_stride, void* ring, c
   const int64_t strips = ((int64_t)max_tokens + kConvStrip - 1) / kConvStrip;
   if (batch > 65535 || strips > 65535) return fail(TKV_ERR_UNSUPPORTED, "tkv_conv_silu: batch=%d max_tokens=%d (at most 65535 requests of 2097120 tokens)", batch, max_tokens);
   const int64_t es = elem_size(dtype);
-  const bool vec = channels % 8 == 0 && (row_stride * es) % 16 == 0 && aligned16(proj) && aligned16(out) && aligned16(ring);
+  const bool vec = channels % 8 == 0 && (row_stride * es) % 16 == 0 && aligned16(proj) && aligned16(out) && aligned16(ring) && aligned16(conv_w);
   const int per = kConvThreads * (vec ? 8 : 1);
   const dim3 grid((channels + per - 1) / per, (unsigned)strips, batch);
   TKV_WITH_TYPE(dtype, T, {
