@@ -366,6 +366,20 @@ int make_map_3d_bf16(CUtensorMap* map, const void* base, int64_t inner, int64_t 
   return TKV_OK;
 }
 
+// Rows of a bf16 matrix in pieces of 64 columns (cols a multiple of 64): boxes of box_rows rows x box_pieces pieces, a piece after the other.
+int make_map_pieces(CUtensorMap* map, const void* base, int64_t cols, int64_t rows, int box_rows, int box_pieces) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return fail(TKV_ERR_LAUNCH, "cuTensorMapEncodeTiled is not available");
+  const cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)};
+  const cuuint64_t strides[2] = {(cuuint64_t)cols * 2, 128};
+  const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, (cuuint32_t)box_pieces};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(TKV_ERR_LAUNCH, "cuTensorMapEncodeTiled failed with %d", (int)r);
+  return TKV_OK;
+}
+
 int attn_tc_chunk_tokens() { return kTcChunk; }
 
 template <int kDtype, int kG, bool kMulti = false>

@@ -1,8 +1,8 @@
 // Grouped product of a mixture of experts on tcgen05 + TMEM, for prompts and for decoding:
 //   out[r, :] = act(a[src[r], :] . w[e]^T)   for the rows r of expert e.
 //
-// One persistent CTA per SM walks tiles of M rows x BN columns, expert by expert.  Per 64 columns of k the weight rows are one
-// TMA box; the rows of A are TMA boxes of 32 where they are consecutive, and are gathered by four warps with cp.async where they
+// One persistent CTA per SM walks tiles of M rows x BN columns, expert by expert.  The weight rows of a stage, 64 or 128 columns of k,
+// are one TMA box; the rows of A are TMA boxes of 32 where they are consecutive, and are gathered by four warps with cp.async where they
 // are not (TMA's own gather moves four rows per instruction and was the limit).  Rows a tile does not have are not fetched, so
 // few rows per expert cost little more than the weights.  A ring of stages feeds the MMAs; two TMEM accumulators let the
 // epilogue of a tile (activation, rounding, stores) overlap the next tile.
@@ -108,7 +108,6 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
       bool ok = (bool)__all_sync(0xffffffffu, *abort_flag == 0);
       while (ok && t.next()) {
         const int boxes = kGather ? 0 : (t.rows + kMgBoxRows - 1) / kMgBoxRows;
-        const uint32_t bytes = (uint32_t)boxes * kMgBoxRows * 128 + Ring::kWBox;      // of 64 columns
         const int wrow = t.e * p.n + t.col * BN;
         for (int k = 0; k < ksteps; ++k, ++it) {
           const int s = it % S;
@@ -117,8 +116,9 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
           if (elect_one()) {
             uint8_t* st = base + s * kStage;
             const int subs = min(SUBS, pieces - k * SUBS);
-            mbar_expect_tx(&sm->full[s], bytes * subs);
-            for (int j = 0; j < subs; ++j) tma_load_2d(st + Ring::kWAt + j * Ring::kWBox, &map_w, &sm->full[s], (k * SUBS + j) * kMgK, wrow);
+            mbar_expect_tx(&sm->full[s], boxes * subs * kMgBoxRows * 128 + SUBS * Ring::kWBox);
+            if (SUBS > 1) tma_load_3d(st + Ring::kWAt, &map_w, &sm->full[s], 0, wrow, k * SUBS);    // beyond the last piece: zeros
+            else tma_load_2d(st + Ring::kWAt, &map_w, &sm->full[s], k * kMgK, wrow);
             for (int j = 0; j < subs; ++j)
               for (int i = 0; i < boxes; ++i)
                 tma_load_2d(st + j * Ring::kABox + i * kMgBoxRows * 128, &map_a, &sm->full[s], (k * SUBS + j) * kMgK, t.row0 + i * kMgBoxRows);
@@ -257,7 +257,9 @@ template <int M, int BN, int SUBS, bool kGather>
 static int launch_mg(const GroupedGemm& p, int64_t tiles, cudaStream_t st) {
   CUtensorMap ma, mw;
   int rc = make_map_rows(&ma, p.a, p.k, p.a_rows, p.a_stride, kMgK, kMgBoxRows);
-  if (rc == TKV_OK) rc = make_map_2d(&mw, p.w, p.k, (int64_t)p.experts * p.n, kMgK, BN, TKV_BF16);
+  if (rc == TKV_OK)
+    rc = SUBS > 1 ? make_map_pieces(&mw, p.w, p.k, (int64_t)p.experts * p.n, BN, SUBS)
+                  : make_map_2d(&mw, p.w, p.k, (int64_t)p.experts * p.n, kMgK, BN, TKV_BF16);
   if (rc != TKV_OK) return rc;
   const int bytes = mg_smem_bytes<M, BN, SUBS>(p.experts);
   static int allowed = 0;
@@ -280,14 +282,15 @@ static int launch_mg(const GroupedGemm& p, int64_t tiles, cudaStream_t st) {
 int launch_moe_tc(const GroupedGemm& p, cudaStream_t st) {
   // the widest column tile that still gives every SM a few tiles (row tiles: about one per expert beyond whole ones)
   auto tiles = [&](int m, int bn) { return (p.max_rows / m + (p.experts < p.max_rows ? p.experts : p.max_rows)) * ((p.n + bn - 1) / bn); };
-  if (tiles(64, 64) > INT32_MAX / 2) return fail(TKV_ERR_UNSUPPORTED, "tkv_moe_gemm: %lld tiles", (long long)tiles(64, 64));
+  if (tiles(128, 256) > INT32_MAX / 2) return fail(TKV_ERR_UNSUPPORTED, "tkv_moe_gemm: %lld tiles", (long long)tiles(128, 256));
   if (tiles(128, 256) >= 148 * 6) return launch_mg<128, 256, 1>(p, tiles(128, 256), st);
   if (tiles(128, 128) >= 148 * 2) {
     // Few rows per expert: what counts is the weights' stream.  Tiles of 64 rows leave room for stages of 128 columns, 256 bytes of every
-    // weight row at a time and 128 KB in flight instead of 96.  us of both products, 2048 x 1536, 32 experts, 6 a token, stages of 64
-    // columns and now: 8 tokens 45 + 33 and 41 + 33, 16 tokens 47 + 41 and 41 + 39, 128 tokens 49 + 41 and 45 + 39; 4096 x 3072, 8 tokens
-    // 104 + 90 and 96 + 86.  Beyond 32 rows an expert, more and more experts would have their weights read for two tiles.
-    if (p.max_rows <= (int64_t)32 * p.experts) return launch_mg<64, 128, 2>(p, tiles(64, 128), st);
+    // weight row at a time by one copy (k of whole pieces of 64) and 128 KB in flight instead of 96.  us of both products, 2048 x 1536,
+    // 32 experts, 6 a token, stages of 64 columns and now: 8 tokens 45 + 33 and 39 + 33, 16 tokens 47 + 41 and 41 + 39, 128 tokens 49 + 41
+    // and 43 + 39; 4096 x 3072, 8 tokens 104 + 90 and 95 + 84.  (As two copies of 64 columns: 41 + 33, 41 + 39, 45 + 39, 96 + 86.)  Beyond
+    // 32 rows an expert, more and more experts would have their weights read for two tiles.
+    if (p.max_rows <= (int64_t)32 * p.experts && p.k % kMgK == 0) return launch_mg<64, 128, 2>(p, tiles(64, 128), st);
     return launch_mg<128, 128, 1>(p, tiles(128, 128), st);
   }
   return launch_mg<128, 64, 1>(p, tiles(128, 64), st);
