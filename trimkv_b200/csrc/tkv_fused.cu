@@ -213,8 +213,8 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(char* residual, const 
       if (i < nvec) wkeep[j] = ld16(reinterpret_cast<const char*>(weight) + (int64_t)i * 16);
     }
   }
+  grid_launch_dependents();  // a product that follows asks for its weights while the kernel before this one ends
   grid_dependency_wait();
-  grid_launch_dependents();  // a following weight-streaming GEMM may start fetching weights; it waits before reading `out`
   // Pass 1: update the residual stream and accumulate the sum of squares.
   for (int i = threadIdx.x, j = 0; i < nvec; i += 256, ++j) {
     uint4 r = ld16(residual + off + (int64_t)i * 16);
@@ -277,8 +277,8 @@ __global__ void __launch_bounds__(256) silu_mul_kernel(const char* gu, char* out
   using T = T16<kDtype>;
   const int nvec = inter / 8;
   const int64_t total = (int64_t)rows * nvec;
+  grid_launch_dependents();  // a product that follows asks for its weights while the kernel before this one ends
   grid_dependency_wait();
-  grid_launch_dependents();  // as in add_rmsnorm_kernel
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
     const int64_t r = i / nvec, c = i - r * nvec;
     auto f = [](float gg, float uu) {
