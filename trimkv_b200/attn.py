@@ -50,7 +50,7 @@ def _workspace(device, nbytes: int) -> torch.Tensor:
 #   256        1.79                                     0.23                    0.64             2.29
 #  1024        7.58                                     0.79                    0.90             7.91
 # (Taken when the query-resident kernel had one tile of 128 rows per CTA; with two, where rows are many, 64 segments of 1024
-# rows take 187 us instead of 233.)  The split-KV kernels re-read the K/V chunk once per 16 / 32 rows but spread a segment over
+# rows take 166 us instead of 233.)  The split-KV kernels re-read the K/V chunk once per 16 / 32 rows but spread a segment over
 # many CTAs; the query-resident kernel reads K/V once per 128 or 256 rows with one CTA per (segment, block of rows).  So: the
 # query-resident kernel whenever it gets enough CTAs to fill the GPU, up to 1024 rows where all heads have one length
 # (the library's causal kernel catches up around there and is ahead on whole prompts) and without limit where the

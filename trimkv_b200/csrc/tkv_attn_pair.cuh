@@ -8,9 +8,13 @@
 // What bounds it is the exponential unit (16 results per SM and cycle: 1024 cycles for a tile, the same as its two products
 // of 128 dims) and, in a chain product - softmax - product, the length of the chain: two independent chains share the units.
 // One tile with two threads per row, S of the next key tile computed ahead and P through shared memory took 3800 cycles a tile:
-// every step crossed four barriers of 256 arrivals and waited for P . V of the step before.  Now 2500 cycles.  512 queries of 8 x 16
-// heads against 4608 keys 233 -> 187 us; differential with its preparation, 8192 tokens, 16 heads, window 4096, 652 -> 464 us; two-part,
-// 2 x 4096 tokens, 32 heads, 591 -> 441 us.  Sums are taken in the order of those kernels: the results are the same bit for bit.
+// every step crossed four barriers of 256 arrivals and waited for P . V of the step before; in two tiles it takes 2500.  512 queries of
+// 8 x 16 heads against 4608 keys 233 -> 187 us; differential with its preparation, 8192 tokens, 16 heads, window 4096, 652 -> 464 us;
+// two-part, 2 x 4096 tokens, 32 heads, 591 -> 441 us.  With products issued by an elected lane of a whole warp (17 to 21 cycles each
+// instead of 51 in a branch of one lane) 187 -> 166 us, and a differential and a latent layer of the last two 635 -> 606 and 1012 -> 989 us with
+// their library products.  The power of the chip bounds it now: 4150 -> 3240 cycles for a block of keys
+// by fewer arrivals brought the SM clock from 1.80 to 1.62 GHz and the same 166 us.  Sums are taken in the order of those kernels: the
+// results are the same bit for bit.
 //
 // P . V of a step reads the TMEM columns that S of the next one writes.  PTX promises an order of two products only where they have
 // one accumulator and shape, so S is issued when P . V is complete; behind S of a step O may therefore be rescaled.  O is rescaled
@@ -291,8 +295,9 @@ __device__ __forceinline__ bool pair_meet(PairSmem* sm, int phase) {
 }
 
 // Whether CTAs of two tiles of rows take less time than CTAs of one: a CTA per SM at a time, 2.6 us per key tile for a pair against
-// 1.64 us for a tile with the chain of its own (64 segments of 192 rows, 33 key tiles: 96 us as 64 pairs, 62 us as 128 tiles; 64
-// segments of 2048 rows: 373 us as 512 pairs, 430 us as 1024 tiles).  Two-part keys of 192 dims: 3.7 and 2.6 us (2 x 4096 tokens, 32
+// 1.64 us for a tile with the chain of its own when measured (64 segments of 192 rows, 33 key tiles: 96 us as 64 pairs, 62 us as 128
+// tiles; 64 segments of 2048 rows: 373 us as 512 pairs, 430 us as 1024 tiles).  Products issued by an elected lane made both shorter, 60 us
+// as those 128 tiles and 332 us as those 512 pairs, and the line was left where it is.  Two-part keys of 192 dims: 3.7 and 2.6 us (2 x 4096 tokens, 32
 // heads: 441 and 591 us; 1500 tokens, 16 heads: 48 and 52 us); of 128 dims the ratio is lower, and 6000 tokens of 8 heads, 192 pairs or
 // 376 tiles, would take 118 us instead of 148.  CTAs count as equally long, which those of a prompt without a past are not: 16 segments of
 // 1536 rows take 41 us as 96 pairs, 37 us as 192 tiles.  One tile only is never a pair.
