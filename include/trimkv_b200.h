@@ -446,13 +446,6 @@ int tkv_skinny_gemm(const void* x, const void* w, float* partial, int m, int n, 
 int tkv_skinny_gemm_swiglu(const void* gate_up, const void* w, float* partial, int m, int n, int k, int dtype,
                            int32_t* status, tkv_stream_t stream);
 
-/*
- * y[m, n] = x[m, k] . w[n, k]^T + bias[n] (NULL: none) in bf16 (sums in fp32) for m <= 32 rows, n a multiple of 8, k of 64, row-major operands 16-byte
- * aligned: the weights' stream divided over clusters of CTAs along k.
- */
-int tkv_few_rows(const void* x, const void* w, const void* bias, void* y, int m, int n, int k, int32_t* status,
-                 tkv_stream_t stream);
-
 /* ---- decoders with recurrent layers, windowed attention and experts -------------------------------------------
  * Common conventions.  Tokens of a step are packed: request b owns rows cu_tokens[b] .. cu_tokens[b + 1) of every
  * per-token array (cu_tokens NULL, where allowed: one token per request).  What a request keeps between steps lives in

@@ -50,7 +50,6 @@ SIGNATURES = {
     "tkv_decode_prep": (I, [P, L, P, P, F, P, P, P, P, I, P, P, P, P, P, P, P, P, L, I, I, I, I, I, I, P, P, P]),
     "tkv_add_rmsnorm": (I, [P, P, P, P, I, I, F, I, I, P, P]),
     "tkv_silu_mul": (I, [P, P, I, I, I, I, P, P]),
-    "tkv_few_rows": (I, [P, P, P, P, I, I, I, P, P]),
     "tkv_skinny_gemm_splits": (I, [I, I, I]),
     "tkv_skinny_gemm": (I, [P, P, P, I, I, I, I, P, P]),
     "tkv_skinny_gemm_swiglu": (I, [P, P, P, I, I, I, I, P, P]),

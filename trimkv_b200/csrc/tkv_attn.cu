@@ -274,7 +274,7 @@ __device__ __forceinline__ float merge_partials(const AttnParams& p, int seg, in
 template <int kDtype, int kD>
 __global__ void __launch_bounds__(kD) decode_attn_combine_kernel(AttnParams p) {
   const int seg = blockIdx.x, g = blockIdx.y, d = threadIdx.x;
-  grid_launch_dependents();  // a product that follows asks for its weights while the kernel before this one ends
+  grid_launch_dependents();  // what follows may be scheduled while the kernel before this one ends; it waits for this one (0.3 to 0.6 us a call)
   grid_dependency_wait();  // launched with programmatic serialization behind the split kernel
   float early[kMergeEarly];
   load_partials_early<kD>(p, seg, g, d, early);

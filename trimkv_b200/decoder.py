@@ -117,9 +117,6 @@ class FusedDecodeStep:
         ops.skinny_gemm(x, w, buf, self.cache._status)
         return buf, splits
 
-    def _linear(self, x, w, bias):
-        return ops.linear(x, w, bias, self.cache._status)
-
     def __call__(self, ids: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
         """ids [B,1] int64, pos [1] int64 (device) -> logits [B, vocab]."""
         import torch.nn.functional as F
@@ -138,7 +135,7 @@ class FusedDecodeStep:
             ops.add_rmsnorm(x, delta, layer.input_layernorm.weight, h, self.eps, d_splits, d_bias if d_splits else None)
             qkvg, s1 = self._gemm(h, w_qkvg, "qkvg")
             if s1 == 0:
-                qkvg = self._linear(h, w_qkvg, b_qkvg)
+                qkvg = F.linear(h, w_qkvg, b_qkvg)
             qn, kn = getattr(at, "q_norm", None), getattr(at, "k_norm", None)
             k, v, kw = cache.decode_prep(l, qkvg, qn.weight if qn is not None else None,
                                          kn.weight if kn is not None else None, self.eps, cos, sin,
@@ -147,11 +144,11 @@ class FusedDecodeStep:
             o, _, _ = tkv_attention_forward(at, q_out, k, v, None, scaling=at.scaling, flash_attn_kwargs=kw)
             a, s2 = self._gemm(o.view(bsz, -1), at.o_proj.weight, "o")
             if s2 == 0:
-                a = self._linear(o.view(bsz, -1), at.o_proj.weight, at.o_proj.bias)
+                a = F.linear(o.view(bsz, -1), at.o_proj.weight, at.o_proj.bias)
             ops.add_rmsnorm(x, a, layer.post_attention_layernorm.weight, h, self.eps, s2, at.o_proj.bias if s2 else None)
             gu, s3 = self._gemm(h, w_gu, "gu")
             if s3 == 0:
-                gu = self._linear(h, w_gu, b_gu)
+                gu = F.linear(h, w_gu, b_gu)
             d_bias = layer.mlp.down_proj.bias
             w_down = layer.mlp.down_proj.weight
             d_splits = ops.skinny_gemm_splits(bsz, w_down.shape[0], w_down.shape[1]) if (self.fused_down and s3 == 0) else 0
@@ -166,9 +163,9 @@ class FusedDecodeStep:
             ops.silu_mul(gu, act, s3, b_gu if s3 else None)
             delta, d_splits = self._gemm(act, w_down, "down")
             if d_splits == 0:
-                delta = self._linear(act, w_down, d_bias)
+                delta = F.linear(act, w_down, d_bias)
         ops.add_rmsnorm(x, delta, m.norm.weight, h, self.eps, d_splits, d_bias if d_splits else None)
-        return self._linear(h, self.model.lm_head.weight, None)
+        return F.linear(h, self.model.lm_head.weight)
 
 
 class GraphedForwardStep:

@@ -345,30 +345,6 @@ def skinny_gemm_splits(m: int, n: int, k: int) -> int:
     return int(lib().tkv_skinny_gemm_splits(m, n, k))
 
 
-def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, status=None) -> torch.Tensor:
-    """``x @ w.T + bias`` of a decoding step: the kernel for few rows where it is the faster one, else the library's product.  The line
-    (us of both sides: csrc/tkv_few_rows.cu) lies where n leaves no CTAs along k, and where there is too little of k to divide: 2048 x 512
-    with 32 rows 4.4 us by the library against 5.1, 2048 x 1024 5.5 against 5.5.
-
-    For the decoders whose layers are Hugging Face's.  The hybrid ones keep the library's order of the sums: where a router chooses by the
-    result, another order now and then chooses another expert, and a state that keeps wide values in 16 bits is another one by a whole
-    step of such a value (a Dafovik step of 7 requests: 295 us by the library, 231 so, but elements of the state 0.37 away)."""
-    n, k = w.shape
-    m = x.shape[0] if x.dim() == 2 and x.shape[1] == k else 0
-    if (m > 32 or m == 0 or n > 5120 or k < 1024 or k % 64 or n % 8 or x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16
-            or not x.is_cuda or w.device != x.device or x.get_device() != torch.cuda.current_device()
-            or not (x.is_contiguous() and w.is_contiguous()) or x.data_ptr() % 16 or w.data_ptr() % 16
-            or (bias is not None and (bias.dtype != x.dtype or bias.device != x.device or bias.shape != (n,) or bias.stride(0) != 1
-                                      or bias.data_ptr() % 16))
-            or torch.is_autocast_enabled("cuda")
-            or (torch.is_grad_enabled() and (x.requires_grad or w.requires_grad or (bias is not None and bias.requires_grad)))):
-        return torch.nn.functional.linear(x, w, bias)
-    y = torch.empty(m, n, dtype=x.dtype, device=x.device)
-    check(lib().tkv_few_rows(x.data_ptr(), w.data_ptr(), _ptr(bias), y.data_ptr(), m, n, k, _ptr(status), _stream(x)), "tkv_few_rows")
-    _count(1)
-    return y
-
-
 def skinny_gemm(x, w, partial, status=None) -> int:
     """``partial [splits, M, N]`` fp32 with ``sum(partial, 0) == x [M, K] @ w [N, K].T``; returns ``splits``."""
     m, k = x.shape
