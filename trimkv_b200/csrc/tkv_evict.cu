@@ -644,9 +644,12 @@ static int launch_rebuild(const int32_t* seg_len, int32_t* cu, int nseg, int gro
   return check_launch("tkv_rebuild_cu_seqlens");
 }
 
+// Raises a kernel's dynamic shared memory limit where a launch needs it: what it gets unasked is 48 KB less what the kernel declares itself,
+// SelectScratch for the selections.
 template <typename K>
 static int set_smem(K kernel, size_t bytes, const char* what) {
-  if (bytes > 48 * 1024) {
+  static_assert(sizeof(SelectScratch) <= 16 * 1024, "declared shared memory");
+  if (bytes > 32 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return fail(TKV_ERR_LAUNCH, "%s: shared memory %zu: %s", what, bytes, cudaGetErrorString(e));
   }

@@ -86,9 +86,10 @@ template <int V> struct StateStep {
   }
 };
 
-// Raises a kernel's dynamic shared memory limit (once per kernel and size); false if the size is out of reach.
+// Raises a kernel's dynamic shared memory limit where a launch may need it (48 KB less what the kernel declares itself, a few KB, comes
+// unasked); false if the size is out of reach.
 template <typename K> inline bool allow_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return true;
+  if (bytes <= 32 * 1024) return true;
   if (bytes > 220 * 1024) return false;
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
 }
