@@ -1,4 +1,5 @@
-"""The convolution's weights as vectors (csrc/tkv_linrec.cu): weights that start between two vectors give the same bits."""
+"""The convolution's weights as vectors (csrc/tkv_linrec.cu): weights that start between two vectors give the same bits, by a channel or
+(16-bit inputs of many tokens) eight channels per thread."""
 import pytest
 import torch
 
@@ -9,7 +10,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("channels,lens", [(8, [1, 33]), (1032, [31, 64, 5]), (1028, [40])])
+@pytest.mark.parametrize("channels,lens", [(8, [1, 33]), (1032, [31, 64, 5]), (1028, [40]), (2056, [3000, 1801])])
 def test_aligned_and_shifted_weights_agree(channels, lens, dtype):
     g = torch.Generator(device="cuda").manual_seed(channels)
     x = torch.randn(sum(lens), channels, generator=g, device="cuda").to(dtype)

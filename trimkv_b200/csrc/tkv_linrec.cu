@@ -93,11 +93,11 @@ __global__ void __launch_bounds__(kConvThreads, sizeof(T) == 2 && V > 1 && kTaps
   if (kTaps > 0) {
     constexpr int kT = kTaps > 0 ? kTaps : 1;
     float wt[kT][V], win[kT][V];                       // win[k]: input k places before the newest
-    if constexpr (kT == 4 && V > 1) {                  // the host has seen to the alignment of w and bias
+    if (kT == 4 && V > 1 && (reinterpret_cast<uintptr_t>(w) & 15) == 0) {
 #pragma unroll
       for (int e = 0; e < V; ++e) {
         const float4 x = reinterpret_cast<const float4*>(w)[ch + e];
-        wt[3][e] = x.x; wt[2][e] = x.y; wt[1][e] = x.z; wt[0][e] = x.w;
+        wt[3 % kT][e] = x.x; wt[2 % kT][e] = x.y; wt[1 % kT][e] = x.z; wt[0][e] = x.w;
       }
     } else {
 #pragma unroll
@@ -515,7 +515,10 @@ extern "C" int tkv_conv_silu(const void* proj, int64_t row_stride, void* ring, c
   const int64_t strips = ((int64_t)max_tokens + kConvStrip - 1) / kConvStrip;
   if (batch > 65535 || strips > 65535) return fail(TKV_ERR_UNSUPPORTED, "tkv_conv_silu: batch=%d max_tokens=%d (at most 65535 requests of 2097120 tokens)", batch, max_tokens);
   const int64_t es = elem_size(dtype);
-  const bool vec = channels % 8 == 0 && (row_stride * es) % 16 == 0 && aligned16(proj) && aligned16(out) && aligned16(ring) && aligned16(conv_w);
+  // Weights that start between two vectors: a channel per thread, but for 16-bit inputs of many tokens, whose rows are the larger part (4 taps,
+  // 6827 tokens of 6144 channels: 77 us with a channel per thread, 63 with eight; 900 of 4608: 12.7 and 13.0; 33: 7.5 and 11.9).
+  const bool vec_rows = channels % 8 == 0 && (row_stride * es) % 16 == 0 && aligned16(proj) && aligned16(out) && aligned16(ring);
+  const bool vec = vec_rows && (aligned16(conv_w) || (taps == 4 && es == 2 && (channels / 8 + kConvThreads - 1) / kConvThreads * strips * batch >= 2 * 148));
   const int per = kConvThreads * (vec ? 8 : 1);
   const dim3 grid((channels + per - 1) / per, (unsigned)strips, batch);
   TKV_WITH_TYPE(dtype, T, {
