@@ -29,7 +29,10 @@ def _step(rows, proj, conv, state, weights, out_type, h, n, p, g, taps, start):
 @pytest.mark.gpu
 @pytest.mark.parametrize("requests,h,n,p,g,taps,start", [
     (40, 64, 128, 64, 8, 4, 9), (150, 20, 128, 64, 4, 4, 1), (99, 12, 64, 32, 2, 3, 5), (60, 33, 32, 16, 3, 4, 2), (37, 64, 128, 64, 8, 4, 0),
-    (300, 8, 20, 8, 2, 2, 7), (45, 32, 128, 128, 8, 4, 6), (60, 9, 30, 24, 3, 4, 3)])
+    (300, 8, 20, 8, 2, 2, 7), (45, 32, 128, 128, 8, 4, 6), (60, 9, 30, 24, 3, 4, 3),
+    # just beyond a group per SM, and two: thirds and halves of a group, a head per CTA, groups that stay together
+    (20, 48, 128, 64, 8, 4, 4), (49, 28, 64, 32, 4, 4, 2), (75, 14, 64, 64, 2, 4, 5), (40, 48, 64, 64, 8, 4, 5), (100, 40, 64, 32, 4, 4, 3),
+    (20, 24, 128, 64, 8, 4, 6), (20, 32, 64, 64, 8, 4, 6)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_heads_of_a_group_in_one_cta(requests, h, n, p, g, taps, start, dtype):
     gen = torch.Generator(device=DEV).manual_seed(requests)

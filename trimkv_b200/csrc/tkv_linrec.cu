@@ -582,7 +582,16 @@ extern "C" int tkv_ssd_step(const void* proj, int64_t row_stride, void* ring, fl
   // As few CTAs per group as fill two on every SM; a head's own CTA where that leaves one head each.
   const int hpg = heads / groups, cb = vdim / 4;
   const int64_t pairs = (int64_t)batch * groups;
-  const int parts = pairs >= 296 ? 1 : (int)std::min<int64_t>(hpg, 296 / pairs), per = (hpg + parts - 1) / parts;
+  int parts = pairs >= 296 ? 1 : (int)std::min<int64_t>(hpg, 296 / pairs);
+  // A CTA per group just beyond one or two on every SM leaves most of the last ones idle: smaller shares of a group then, or a head's own
+  // CTA.  us with a head, a group and a third of a group (half of one, where there are more than 296) per CTA, state rows of 64 values, n = 128:
+  //   160 groups of 3 heads   9.2  9.7 11.3    6 heads  14.8 15.4 13.9    8 heads  19.5 18.5 16.4    20 heads   58.4  57.3 47.1
+  //   192                     9.4 10.1 11.3             15.9 15.9 14.5             21.3 18.9 17.4               69.4  62.9 53.7
+  //   320                    14.8 15.4 16.9             26.5 25.5 23.2             42.0 35.9 33.2              110.0 117.4 90.5 (a third)
+  // Groups of 2, 4 and 5 heads stay together: 192 groups of 4 take 13.8, 11.9 and 13.7 us.
+  if (pairs > 148 && (pairs <= 196 || (pairs > 296 && pairs <= 400)) && (hpg == 3 || hpg >= 6))
+    parts = pairs > 296 && hpg < 10 && hpg > 3 ? 2 : 3;
+  const int per = (hpg + parts - 1) / parts;
   const size_t group_smem = (size_t)per * (kStepThreads * 16 + (vdim + 2) * 4) + (size_t)n * 8;
   if (per > 1 && vdim % 4 == 0 && cb <= kStepThreads && kStepThreads % cb == 0 && n <= kGroupRows * (kStepThreads / cb) && n % 4 == 0 &&
       group_smem <= 100 * 1024 && ((uintptr_t)state & 15) == 0) {
