@@ -144,3 +144,31 @@ def test_ranges_of_rows_agree(nseg, dim):
     assert ops.read_status(status) == 0 and bool((ln == m).all())
     for t, w in zip((k, v, beta, pos), want):
         assert torch.equal(t.view(nseg, cap, -1)[:, :m], w)
+
+
+# protected rows are left out of the search unless other rows at infinity, or without a number, take their places; protected rows up to
+# and beyond what is kept
+@pytest.mark.gpu
+@pytest.mark.parametrize("nseg,n", [(3, 1111), (75, 640), (300, 700)])
+@pytest.mark.parametrize("kind", ["equal", "wide", "infinite", "no_number", "lowest"])
+def test_protected_rows(nseg, n, kind):
+    g = torch.Generator(device=DEV).manual_seed(n)
+    beta = {"equal": lambda: torch.full((nseg, n), -1.5, device=DEV),
+            "wide": lambda: torch.randn(nseg, n, generator=g, device=DEV),
+            "infinite": lambda: torch.where(torch.rand(nseg, n, generator=g, device=DEV) < 0.5, float("inf"), -1.0),
+            "no_number": lambda: torch.where(torch.rand(nseg, n, generator=g, device=DEV) < 0.3, float("nan"), -1.0),
+            "lowest": lambda: torch.where(torch.rand(nseg, n, generator=g, device=DEV) < 0.3, float("-inf"), torch.finfo(torch.float32).min)}[kind]()
+    m, dim = n * 3 // 5, 64
+    for w in (1, 64, n // 5, m - 1, m, n - 1):
+        k, v = (torch.randn(nseg * n, dim, generator=g, device=DEV).bfloat16() for _ in range(2))
+        score = beta.double().clone()
+        score[:, n - w:] = float("inf")
+        score = torch.where(score.isnan(), 1e301, score.clamp(max=1e300))                     # no number: above infinity
+        keep = score.sort(dim=1, descending=True, stable=True).indices[:, :m].sort(dim=1).values
+        want = [t.view(nseg, n, dim).gather(1, keep[:, :, None].expand(-1, -1, dim)) for t in (k, v)]
+        status, ln = ops.new_status(DEV), torch.full((nseg,), n, dtype=torch.int32, device=DEV)
+        pos = torch.full((nseg * n,), 6, dtype=torch.int32, device=DEV)                       # the score is log beta itself
+        ops.evict_ex(k, v, beta.clone().view(-1), pos, ln, None, nseg, nseg, n, 7, n, None, w, m, m, status=status)
+        assert ops.read_status(status) == 0 and bool((ln == m).all())
+        for t, x in zip((k, v), want):
+            assert torch.equal(t.view(nseg, n, dim)[:, :m], x), w

@@ -287,7 +287,14 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) evict_inplace_kerne
   if (kSlices > 1) asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
   else __syncthreads();
   uint32_t thresh; int n_eq_keep;
-  radix_select_mth<kThreads>(keys, n, m, &sc, &thresh, &n_eq_keep);
+  // Protected rows are searched only if that many others score infinity that some of them go: infinity beside finite scores would make
+  // the first digit one of sign and exponent, in which the keys of the others hardly differ (512 x (640 -> 512), rows of one score, 64
+  // protected: 23.1 us with them in the search, 16.1 without).
+  for (int tail = p.protect_last < m ? p.protect_last : 0;; tail = 0) {
+    radix_select_mth<kThreads>(keys, n - tail, m - tail, &sc, &thresh, &n_eq_keep);
+    if (tail == 0 || thresh + (n_eq_keep == 0 ? 1u : 0u) < score_key(INFINITY)) break;
+    __syncthreads();
+  }
   const int j0 = build_kept_list<kThreads>(keys, n, thresh, n_eq_keep, &sc);
   const int32_t* kept = reinterpret_cast<const int32_t*>(keys);
   if (p.kept_idx_out != nullptr && slice == 0)
