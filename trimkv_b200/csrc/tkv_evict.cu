@@ -702,13 +702,16 @@ template <int kThreads, int kSlices> static int launch_inplace(const EvictParams
 //             2048            1152 -> 1024       20.5  27.4  45.6     4224 -> 4096   52.2  58.6  76.8      8192 -> 1024  102.1  83.7  97.8
 // `moved`: bytes of K of a segment's kept rows.  Where they outweigh the keys and 512 threads would leave one CTA on some SMs and two on
 // others, up to about 1.75 a SM, CTAs of a whole SM in two rounds share the memory better (224 segments above).
-enum class EvictWork { kInPlace, kSelect };
+// Where the scores take the norms of K, all of K is read first: four narrow CTAs on every SM in one round, instead of two wide ones in two,
+// do that faster for short segments (256 and 512 threads):
+//   in place with norms, 300 segments of  640 -> 512  111 118     1024 -> 900  199 196      512:  640 -> 512  138 152      768 -> 640  175 182
+enum class EvictWork { kInPlace, kInPlaceNorms, kSelect };
 template <typename F> static int with_evict_threads(EvictWork work, int nseg, int n, int64_t moved, F launch) {
   int threads = kEvictThreadsWide;
-  if (work == EvictWork::kInPlace) {
+  if (work != EvictWork::kSelect) {
     if (nseg <= 148) threads = n >= 2048 ? kEvictThreadsPlan : kEvictThreadsWide;
     else if (nseg <= 2 * 148) threads = nseg > 192 && nseg <= 259 && n >= 2048 && moved > 200 * (int64_t)n ? kEvictThreadsPlan : kEvictThreadsWide;
-    else threads = n > 512 ? kEvictThreadsWide : kEvictThreads;
+    else threads = n > (work == EvictWork::kInPlaceNorms && nseg <= 4 * 148 ? 896 : 512) ? kEvictThreadsWide : kEvictThreads;
   } else {
     if (nseg <= 148) threads = n >= 4096 ? kEvictThreadsPlan : n > 256 ? kEvictThreadsWide : kEvictThreads;
     else if (nseg <= 2 * 148) threads = n >= 16384 ? kEvictThreadsPlan : n > 1024 ? kEvictThreadsWide : kEvictThreads;
@@ -800,7 +803,8 @@ static int evict_impl(void* k_cache, void* v_cache, float* beta_cache, int32_t* 
   } else {
     // a keep count of each segment's own is not known here: as if all rows stayed
     const int64_t moved = (int64_t)(keep_cnt ? max_len : memory_size) * head_dim * es;
-    rc = with_evict_threads(EvictWork::kInPlace, nseg * slices, max_len, moved, [&](auto threads) {
+    const EvictWork work = scores == nullptr && strategy != 0 ? EvictWork::kInPlaceNorms : EvictWork::kInPlace;
+    rc = with_evict_threads(work, nseg * slices, max_len, moved, [&](auto threads) {
       constexpr int kT = threads.value;
       return slices == 8 ? launch_inplace<kT, 8>(p, smem, (cudaStream_t)stream) : slices == 4 ? launch_inplace<kT, 4>(p, smem, (cudaStream_t)stream)
              : slices == 2 ? launch_inplace<kT, 2>(p, smem, (cudaStream_t)stream) : launch_inplace<kT, 1>(p, smem, (cudaStream_t)stream);
