@@ -171,7 +171,8 @@ int tkv_evict_ex(void* k_cache, void* v_cache, float* beta_cache, int32_t* pos_c
  * (src/trimkv/cache_utils.py:140-198).  Requires max_len - memory_size rows of K+V to fit in shared memory
  * (<= 200 KB) and ctas_per_segment <= 32.  workspace: device scratch of tkv_evict_multi_workspace_bytes() bytes,
  * contents irrelevant before and after the call; one workspace serves one stream at a time.
- * ctas_per_segment == 1 is tkv_evict_ex without keep counts.
+ * ctas_per_segment == 1 is tkv_evict_ex without keep counts.  Up to 74 segments whose rows have 64 bytes or more take clusters of CTAs that
+ * share the columns of a segment instead, here as in tkv_evict: the arguments are checked all the same, the workspace stays untouched.
  */
 int64_t tkv_evict_multi_workspace_bytes(int nseg, int memory_size, int ctas_per_segment);
 int tkv_evict_multi(void* k_cache, void* v_cache, float* beta_cache, int32_t* pos_cache,

@@ -134,6 +134,13 @@ MULTI_CASES = [
     (2, 16512, 128, 16384, 16512, "full", torch.bfloat16, _bf16_logbeta, 32),
     (100, 384, 128, 256, 320, "ragged", torch.bfloat16, _bf16_logbeta, 8),      # more evicting segments than rows of the move grid
     (700, 160, 64, 128, 129, "ragged", torch.float16, _coarse_logbeta, 2),      # 2 x 296 blocks walk up to 700 segments
+    # too many segments for clusters that share the columns (at most 74): the rows in ranges again
+    (80, 133, 64, 100, 101, "ragged", torch.bfloat16, _coarse_logbeta, 8),
+    (75, 130, 128, 129, 130, "full", torch.bfloat16, _bf16_logbeta, 2),
+    (75, 2176, 128, 2048, 2176, "full", torch.bfloat16, _bf16_logbeta, 16),
+    (77, 700, 64, 600, 601, "ragged", torch.float16, _coarse_logbeta, 7),
+    (90, 1064, 64, 1024, 1064, "full", torch.bfloat16, _tail_heavy_logbeta, 4),
+    (75, 4224, 32, 4096, 4224, "full", torch.bfloat16, _bf16_logbeta, 32),
 ]
 
 

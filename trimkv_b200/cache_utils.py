@@ -462,9 +462,10 @@ class TrimKVCache:
             self._cache_len[l] = memory_size
 
     def _evict(self, k, v, beta, pos, ln, cu, group, nseg, q_idx, n, w, memory_size, trigger, kept, knorm):
-        """One eviction launch over ``nseg`` segments of length ``n``.  With few segments (one layer of a small batch)
-        the rows of each segment are shared by several CTAs so that more of the GPU moves them; measured on B200 this
-        pays up to about 64 segments, beyond that one CTA per segment is as fast or faster."""
+        """One eviction over ``nseg`` segments of length ``n``.  Few segments (one layer of a small batch) are offered to several CTAs
+        each, so that more of the GPU moves rows: the native call takes clusters that share the columns of a segment, or, for rows under
+        64 bytes, CTAs that share its rows and hand over through the workspace.  From about 64 segments on one CTA, or what clusters the
+        plain call takes, is as fast or faster."""
         ctas = min(32, 1024 // nseg) if 0 < nseg <= 64 else 1
         row_pair = 2 * k.shape[-1] * k.element_size() + 8
         if ctas >= 2 and 0 < n - memory_size and (n - memory_size) * row_pair <= 200 * 1024:

@@ -400,7 +400,8 @@ def evict_multi_workspace(nseg: int, memory_size: int, ctas_per_segment: int, de
 def evict_multi(k_cache, v_cache, beta_cache, pos_cache, seg_len, cu_seqlens, group: int, nseg: int, cap: int,
                 q_idx: int, memory_size: int, trigger_len: int, max_len: int, ctas_per_segment: int, workspace,
                 protect_last: int = 0, knorm: bool = False, kept_idx_out=None, status=None) -> None:
-    """:func:`evict` with ``ctas_per_segment`` CTAs sharing each evicting segment (identical result)."""
+    """:func:`evict` with up to ``ctas_per_segment`` CTAs sharing the rows of each evicting segment (identical result); where the segments
+    are few enough for clusters that share their columns, those are taken instead."""
     d = k_cache.shape[-1]
     rc = lib().tkv_evict_multi(
         k_cache.data_ptr(), v_cache.data_ptr(), beta_cache.data_ptr(), pos_cache.data_ptr(),
@@ -409,7 +410,8 @@ def evict_multi(k_cache, v_cache, beta_cache, pos_cache, seg_len, cu_seqlens, gr
         _ptr(workspace), 0 if workspace is None else workspace.numel() * workspace.element_size(),
         _ptr(kept_idx_out), _ptr(status), _stream(k_cache))
     check(rc, "tkv_evict_multi")
-    n = 1 if ctas_per_segment <= 1 else 2
+    # few segments with rows of 64 bytes and more take clusters that share the columns, one launch (evict_slices in csrc/tkv_evict.cu)
+    n = 1 if ctas_per_segment <= 1 or (nseg <= 74 and d * k_cache.element_size() >= 64) else 2
     _count(n if cu_seqlens is None else n + 1)
 
 
