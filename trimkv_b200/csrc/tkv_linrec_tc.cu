@@ -12,7 +12,7 @@
 // rounded to 16 bits.
 //
 // Roles: warps 0-7 hold rows (TMEM lane = token, or state row; two threads per row, one per column half); warp 8 issues TMA
-// copies and MMAs (one lane); warp 9 computes the running log decays of the next chunk.  Q, K and V have two stages.
+// copies and MMAs (the whole warp walks, one elected lane issues); warp 9 computes the running log decays of the next chunk.  Q, K and V have two stages.
 // What bounds it is shared memory, which the products' operands and the split parts all pass through, and the rows' work in turn: state,
 // weighted values, weighted scores, outputs.  With the weights in shared memory as well, one stage of Q and K, and the outputs behind
 // their own chunk's O2, a chunk took 6500 cycles, 2000 of them waits for O2.  Now the outputs of a chunk come

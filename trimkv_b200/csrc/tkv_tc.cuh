@@ -161,9 +161,10 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
 int make_map_2d(CUtensorMap* map, const void* base, int64_t cols, int64_t rows, int box_cols, int box_rows, int dtype);
 // The same over bf16 rows that are row_stride elements apart.
 int make_map_rows(CUtensorMap* map, const void* base, int64_t cols, int64_t rows, int64_t row_stride, int box_cols, int box_rows);
+// Rows of a bf16 matrix in pieces of 64 columns (cols a multiple of 64): boxes of box_rows rows x box_pieces pieces, a piece after the other.
+int make_map_pieces(CUtensorMap* map, const void* base, int64_t cols, int64_t rows, int box_rows, int box_pieces);
 // 3-D map over bf16 [outer][mid][inner] with element strides inner_len between mids and outer_stride between outers; the box
 // is one mid wide, so columns beyond inner_len read as zeros instead of the next mid's.
-int make_map_pieces(CUtensorMap* map, const void* base, int64_t cols, int64_t rows, int box_rows, int box_pieces);
 int make_map_3d_bf16(CUtensorMap* map, const void* base, int64_t inner, int64_t mid, int64_t outer, int64_t outer_stride, int box_inner,
                      int box_outer);
 
